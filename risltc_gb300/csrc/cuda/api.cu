@@ -824,6 +824,7 @@ risltc::RisParams ris_params(const risltc_ctx_t* ctx, const Scratch& sc, const r
 	r.accum = accum;
 	r.reservoirs = reservoirs;
 	r.error = ctx->d_error;
+	r.neg_zero = -0.0f;
 	return r;
 }
 

@@ -12,11 +12,11 @@
 //      with a counting sort over the warp, so that the lanes of one step
 //      mostly evaluate polygons with the same number of vertices;
 //   3. evaluates the items with each pixel's LTC frame read from shared
-//      memory, in a form without branches (correctly rounded square roots
-//      from sqrt_tuckerman); an item whose polygon is partially clipped in
-//      either space, or outside that form's range, is deferred to a list
-//      that the warp evaluates 32 at a time, so the clipping path runs with
-//      full warps.
+//      memory, both LTC spaces at once in the lanes of paired FP32
+//      instructions and without branches; an item whose polygon is partially
+//      clipped in either space, or outside that form's range, is deferred to
+//      a list that the warp evaluates 32 at a time, so the clipping path runs
+//      with full warps.
 // A frame's super-chunk is a unit; after up to four units (a window) the
 // last deferred items of the window are evaluated and
 //   4. each lane replays its pixel's reservoir updates in candidate order
@@ -29,13 +29,14 @@
 #pragma once
 #include <algorithm>
 #include <atomic>
+#include "pair_exact.cuh"
 #include "ris_kernels.cuh"
 
 namespace risltc {
 
 // Blocks per SM the candidate kernel is compiled for (register budget):
-// measured best 5 in exact numerics (96 registers; 19.2 against 19.9 ms per
-// 4-frame 1080p launch with 4) and 4 in fast numerics, whose paired form
+// measured best 5 in exact numerics (96 registers; 11.27 ms per 4-frame 1080p
+// launch against 11.65 with 4 and 18.05 with 6) and 4 in fast numerics, which
 // spills at 96 registers.
 #ifndef RISLTC_BINNED_MIN_BLOCKS_EXACT
 #define RISLTC_BINNED_MIN_BLOCKS_EXACT 5
@@ -170,10 +171,9 @@ RL_DEV float clipped_integral(const mat43& t, const float4* record, uint32_t n, 
 // above the horizon (the common case); a polygon entirely below contributes
 // nothing, and a partially clipped one goes through clip_polygon instead.
 // The code stays small and the vertex count of a sorted group is uniform
-// across the warp.  With allow_clip false, returns false as soon as a space
-// clips the polygon partially; the caller defers the item.
+// across the warp.
 template <class P, bool kChecked>
-RL_DEV bool binned_candidate(const float4* f, const float4* record, bool allow_clip, float& p_hat) {
+RL_DEV bool binned_candidate(const float4* f, const float4* record, float& p_hat) {
 	// kChecked: the branch-free forms (normalize_checked,
 	// integrate_edge_checked, sqrt_checked); false when any of them does not
 	// apply (a squared length outside the square root's range, an edge of 90
@@ -217,7 +217,6 @@ RL_DEV bool binned_candidate(const float4* f, const float4* record, bool allow_c
 			r = 0.0f;
 			a = true;
 		} else {
-			if (!allow_clip) return false;
 			r = clipped_integral<P, kChecked>(t, record, n, negate_y, mask, ok);
 			if (kChecked && !ok) return false;
 			a = r < 0.0f;
@@ -248,84 +247,15 @@ RL_DEV bool binned_candidate(const float4* f, const float4* record, bool allow_c
 
 // ---------------------------------------------------------------------------
 // The same candidate with both spaces in the two lanes of Blackwell's paired
-// FP32 instructions (FADD2 / FMUL2 / FFMA2 on float2; lane .x the shading
-// space, lane .y the cosine space).  Both spaces walk the same vertices, so
-// every transform, dot product, scale and edge-integral step of the two
-// spaces is one paired instruction.  Each lane performs the scalar version's
-// operations on the same operands in the same order, and a paired IEEE add
-// or multiply rounds each lane exactly as the scalar one does: the values are
-// bit-identical.  Exact numerics keeps every multiply and add separate; fast
-// numerics contracts them into paired fused multiply-adds.
-#ifndef RISLTC_CANDIDATE_PAIRS
-#define RISLTC_CANDIDATE_PAIRS 0
-#endif
-// Unroll factor of the paired vertex loop.
-#ifndef RISLTC_PAIR_UNROLL
-#define RISLTC_PAIR_UNROLL 1
-#endif
-constexpr int kPairUnroll = RISLTC_PAIR_UNROLL;
-
-// The paired operations.  Fast numerics uses the paired instructions
-// (FADD2 / FMUL2 / FFMA2), which the code generator may contract into fused
-// multiply-adds.  Exact numerics must not be contracted, and the code
-// generator contracts a paired multiply followed by a paired add into FFMA2
-// even with --fmad=false and explicit rounding modifiers (measured: every
-// exact-numerics frame then differed from the oracle).  So by default exact
-// numerics computes each lane with its own correctly rounded scalar
-// operation (__fadd_rn / __fmul_rn, never contracted); the loop still
-// carries both spaces' independent dependency chains side by side.
-// RISLTC_PAIR_OPS selects the form for exact numerics: 0 scalar per lane,
-// 1 paired PTX add/mul, 2 paired fused multiply-adds with exact one and
-// zero operands (RN(a * b + -0) = RN(a * b), RN(a * 1 + b) = RN(a + b)).
-#ifndef RISLTC_PAIR_OPS
-#define RISLTC_PAIR_OPS 0
-#endif
-#if RISLTC_PAIR_OPS == 1
-RL_DEV float2 add2(float2 a, float2 b) {
-	float2 d;
-	asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
-	    "add.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
-	    : "=f"(d.x), "=f"(d.y)
-	    : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-	return d;
-}
-RL_DEV float2 mul2(float2 a, float2 b) {
-	float2 d;
-	asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
-	    "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
-	    : "=f"(d.x), "=f"(d.y)
-	    : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-	return d;
-}
-#elif RISLTC_PAIR_OPS == 2
-RL_DEV float2 add2(float2 a, float2 b) { return __ffma2_rn(a, make_float2(1.0f, 1.0f), b); }
-RL_DEV float2 mul2(float2 a, float2 b) { return __ffma2_rn(a, b, make_float2(-0.0f, -0.0f)); }
-#else
-RL_DEV float2 add2(float2 a, float2 b) { return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)); }
-RL_DEV float2 mul2(float2 a, float2 b) { return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)); }
-#endif
-// Fast numerics: the paired instructions, contraction allowed.
-struct PairFast {
-	static RL_DEV float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-	static RL_DEV float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-	static RL_DEV float2 mad(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-};
-struct PairExact {
-	static RL_DEV float2 add(float2 a, float2 b) { return add2(a, b); }
-	static RL_DEV float2 mul(float2 a, float2 b) { return mul2(a, b); }
-	static RL_DEV float2 mad(float2 a, float2 b, float2 c) { return add2(mul2(a, b), c); }
-};
-template <class P> struct PairOps {
-	using type = PairExact;
-};
-template <> struct PairOps<FastNumerics> {
-	using type = PairFast;
-};
-RL_DEV float2 pair(float a) { return make_float2(a, a); }
-// a * b + c (contracted in fast numerics), a + b and a * b in both lanes.
-template <class P> RL_DEV float2 mad2(float2 a, float2 b, float2 c) { return PairOps<P>::type::mad(a, b, c); }
-template <class P> RL_DEV float2 padd(float2 a, float2 b) { return PairOps<P>::type::add(a, b); }
-template <class P> RL_DEV float2 pmul(float2 a, float2 b) { return PairOps<P>::type::mul(a, b); }
+// FP32 instructions (lane .x the shading space, lane .y the cosine space).
+// Both spaces walk the same vertices, so every transform, dot product, scale
+// and edge-integral step of the two spaces is one paired instruction.
+// Exact numerics takes its operations from pair_exact.cuh: each lane performs
+// the scalar version's operations on the same operands in the same order, so
+// the values are bit-identical.  Fast numerics allows contraction.
+template <class P> RL_DEV float2 mad2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+template <class P> RL_DEV float2 padd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+template <class P> RL_DEV float2 pmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 
 struct f3x2 {
 	float2 x, y, z;
@@ -350,15 +280,6 @@ template <class P> RL_DEV f3x2 normalize2(const f3x2& a) {
 	const float2 s = make_float2(P::rsqrt(d.x), P::rsqrt(d.y));
 	return {pmul<P>(a.x, s), pmul<P>(a.y, s), pmul<P>(a.z, s)};
 }
-// normalize2 with the branch-free square root of normalize_checked (exact
-// numerics; ok cleared outside its range).
-template <class P> RL_DEV f3x2 normalize2_checked(const f3x2& a, bool& ok) { return normalize2<P>(a); }
-template <> RL_DEV f3x2 normalize2_checked<ExactNumerics>(const f3x2& a, bool& ok) {
-	const float2 d = dot2<ExactNumerics>(a, a);
-	ok = ok && tuckerman_range(d.x) && tuckerman_range(d.y);
-	const float2 s = make_float2(rcp_markstein(sqrt_tuckerman(d.x)), rcp_markstein(sqrt_tuckerman(d.y)));
-	return {pmul<ExactNumerics>(a.x, s), pmul<ExactNumerics>(a.y, s), pmul<ExactNumerics>(a.z, s)};
-}
 // integrate_edge on both lanes.
 template <class P> RL_DEV float2 integrate_edge2(const f3x2& v1, const f3x2& v2) {
 	const float2 x = dot2<P>(v1, v2);
@@ -372,9 +293,8 @@ template <class P> RL_DEV float2 integrate_edge2(const f3x2& v1, const f3x2& v2)
 	return pmul<P>(cz, ts);
 }
 
-template <class P, bool kChecked = false>
+template <class P>
 RL_DEV bool binned_candidate_pair(const float4* f, const float4* record, bool allow_clip, float& p_hat) {
-	bool ok = true;
 	const float4 head = __ldg(record), pl = __ldg(record + 1);
 	const uint32_t n = __float_as_uint(head.w);
 	const float plane[4] = {pl.x, pl.y, pl.z, pl.w};
@@ -399,14 +319,14 @@ RL_DEV bool binned_candidate_pair(const float4* f, const float4* record, bool al
 	f3x2 v = mul_point2<P>(t, q0);
 	if (flip) v.y.x = -v.y.x;
 	uint32_t above_s = v.z.x > 0.0f ? 1u : 0u, above_c = v.z.y > 0.0f ? 1u : 0u;  // bit j: vertex j above
-	const f3x2 first = kChecked ? normalize2_checked<P>(v, ok) : normalize2<P>(v);
+	const f3x2 first = normalize2<P>(v);
 	v = mul_point2<P>(t, q1);
 	if (flip) v.y.x = -v.y.x;
 	above_s |= (v.z.x > 0.0f ? 1u : 0u) << 1;
 	above_c |= (v.z.y > 0.0f ? 1u : 0u) << 1;
-	f3x2 prev = first, cur = kChecked ? normalize2_checked<P>(v, ok) : normalize2<P>(v);
+	f3x2 prev = first, cur = normalize2<P>(v);
 	float2 r = pair(0.0f);
-#pragma unroll kPairUnroll
+#pragma unroll 1
 	for (uint32_t j = 1; j != n; ++j) {
 		f3x2 next = first;
 		if (j + 1 != n) {
@@ -415,14 +335,13 @@ RL_DEV bool binned_candidate_pair(const float4* f, const float4* record, bool al
 			q = __ldg(record + 2 + min(j + 2, (uint32_t) kMaxLightVertices - 1));
 			above_s |= (v.z.x > 0.0f ? 1u : 0u) << (j + 1);
 			above_c |= (v.z.y > 0.0f ? 1u : 0u) << (j + 1);
-			next = kChecked ? normalize2_checked<P>(v, ok) : normalize2<P>(v);
+			next = normalize2<P>(v);
 		}
 		r = padd<P>(r, integrate_edge2<P>(prev, cur));
 		prev = cur;
 		cur = next;
 	}
 	r = padd<P>(r, integrate_edge2<P>(prev, first));
-	if (kChecked && !ok) return false;
 	const uint32_t all = (1u << n) - 1u;
 	const bool partial_s = above_s != all && above_s != 0, partial_c = above_c != all && above_c != 0;
 	if ((partial_s || partial_c) && !allow_clip) return false;
@@ -460,28 +379,105 @@ RL_DEV bool binned_candidate_pair(const float4* f, const float4* record, bool al
 	return true;
 }
 
-// The candidate evaluation the binned kernel uses: the paired form in fast
-// numerics (measured 12% faster there: 0.325 against 0.290 Gsamples/s on
-// the 1080p 16K-light frame), the sequential scalar form in exact numerics,
-// where the paired structure with one scalar operation per lane measured
-// slower (29.4 against 24.7 ms per 4-frame launch of the candidate kernel).
-// RISLTC_CANDIDATE_PAIRS=1 selects the paired form for exact numerics too.
+// The first pass of exact numerics: one candidate with no branch in its
+// vertex loop.  False (the caller defers the item to binned_candidate, which
+// clips) when a space clips the polygon partially, a squared length lies
+// outside the square root's range or an edge spans 90 degrees or more.
+//
+// Every normalised vertex is kept negated: the reciprocal of -s gives
+// Markstein's correction without a sign change, and dot products and cross
+// products of two negated vertices equal those of the vertices.  The edge
+// integral's quotient is negated in the same way, so the sum is the negated
+// sum, whose magnitude is what is kept.
+//
+// Against the scalar form that ran the two spaces one after the other: the
+// candidate kernel takes 11.27 instead of 13.89 ms per 4-frame 1080p launch
+// with 16,384 lights, 2.77 instead of 3.22 ms per frame with 1,024.
+RL_DEV bool candidate_first_pass(const float4* f, const float4* record, float neg_zero, float& p_hat) {
+	const PairExact o{pair(neg_zero)};
+	const float4 head = __ldg(record), pl = __ldg(record + 1);
+	float4 q = __ldg(record + 2);
+	const uint32_t n = __float_as_uint(head.w);
+	const float plane[4] = {pl.x, pl.y, pl.z, pl.w};
+	const float4 f0 = f[0];
+	const bool flip = plane_dot(mk3(f0.x, f0.y, f0.z), plane) < 0.0f;
+	f3x2 t[4];
+	{
+		// A side flip negates shading space's y: the row is negated here
+		// (negation is exact and rounding symmetric).
+		const mat43 ms = load_matrix(f + 2), mc = load_matrix(f + (flip ? 8 : 5));
+		const uint32_t sign = flip ? 0x80000000u : 0u;
+#pragma unroll
+		for (int c = 0; c != 4; ++c) {
+			t[c].x = make_float2(ms.c[c].x, mc.c[c].x);
+			t[c].y = make_float2(__uint_as_float(__float_as_uint(ms.c[c].y) ^ sign), mc.c[c].y);
+			t[c].z = make_float2(ms.c[c].z, mc.c[c].z);
+		}
+	}
+	// What decides whether the branch-free forms apply: the least and the
+	// greatest squared length (as unsigned words: NaN and negative values lie
+	// above every number), the least cosine of an edge, and per space the
+	// least and the greatest z (as signed words, ordered like the floats
+	// where both are positive; -0 counts as below, +0 as not above).
+	uint32_t d_min = 0xffffffffu, d_max = 0;
+	int32_t x_min = 0x7fffffff, zs_min = 0x7fffffff, zs_max = INT32_MIN, zc_min = 0x7fffffff, zc_max = INT32_MIN;
+	auto vertex = [&](float4 q) -> f3x2 {  // transformed, normalised and negated
+		const float2 px = pair(q.x), py = pair(q.y), pz = pair(q.z);
+		f3x2 v;
+		v.x = o.add(o.add(o.add(o.mul(t[0].x, px), o.mul(t[1].x, py)), o.mul(t[2].x, pz)), t[3].x);
+		v.y = o.add(o.add(o.add(o.mul(t[0].y, px), o.mul(t[1].y, py)), o.mul(t[2].y, pz)), t[3].y);
+		v.z = o.add(o.add(o.add(o.mul(t[0].z, px), o.mul(t[1].z, py)), o.mul(t[2].z, pz)), t[3].z);
+		zs_min = min(zs_min, __float_as_int(v.z.x));
+		zs_max = max(zs_max, __float_as_int(v.z.x));
+		zc_min = min(zc_min, __float_as_int(v.z.y));
+		zc_max = max(zc_max, __float_as_int(v.z.y));
+		const float2 d = o.add(o.add(o.mul(v.x, v.x), o.mul(v.y, v.y)), o.mul(v.z, v.z));
+		d_min = __vimin3_u32(d_min, __float_as_uint(d.x), __float_as_uint(d.y));
+		d_max = __vimax3_u32(d_max, __float_as_uint(d.x), __float_as_uint(d.y));
+		const float2 nr = rsqrt_negated(o, d);
+		return {o.mul(v.x, nr), o.mul(v.y, nr), o.mul(v.z, nr)};
+	};
+	auto edge = [&](const f3x2& a, const f3x2& b) -> float2 {  // integrate_edge, negated
+		const float2 x = o.add(o.add(o.mul(a.x, b.x), o.mul(a.y, b.y)), o.mul(a.z, b.z));
+		x_min = __vimin3_s32(x_min, __float_as_int(x.x), __float_as_int(x.y));
+		return o.mul(o.sub(o.mul(a.x, b.y), o.mul(a.y, b.x)), edge_fit_negated(o, x));
+	};
+	f3x2 prev = vertex(q);
+	const f3x2 first = prev;
+	q = __ldg(record + 3);
+	float2 r = pair(0.0f);
+#pragma unroll 1
+	for (uint32_t j = 1; j != n; ++j) {
+		const f3x2 cur = vertex(q);
+		q = __ldg(record + 2 + min(j + 1, (uint32_t) kMaxLightVertices - 1));
+		r = o.add(r, edge(prev, cur));
+		prev = cur;
+	}
+	r = o.add(r, edge(prev, first));
+	const bool below_s = zs_max <= 0, below_c = zc_max <= 0;
+	if (!(d_min >= kRootMin && d_max <= kRootMax && x_min > 0 && (zs_min > 0 || below_s) && (zc_min > 0 || below_c)))
+		return false;
+	const f3 radiance = mk3(head.x, head.y, head.z);
+	const float4 f1 = f[1];
+	const f3 diffuse = below_s ? splat(0.0f) : mul(scale(mk3(f1.x, f1.y, f1.z), fabsf(r.x)), radiance);
+	const f3 ggx = below_c ? splat(0.0f) : mul(splat(fabsf(r.y) * f0.w), radiance);
+	const f3 color = add(add(splat(0.0f), diffuse), ggx);
+	bool ok = true;
+	p_hat = sqrt_checked<ExactNumerics>(dot(color, color), ok);
+	return ok;
+}
+
+// The candidate evaluation the binned kernel uses.  Exact numerics: the
+// paired first pass, and for deferred items (allow_clip) the scalar forms,
+// branch-free where they apply, the general ones otherwise.  Fast numerics:
+// the paired form for both.
 template <class P>
-RL_DEV bool evaluate_candidate(const float4* f, const float4* record, bool allow_clip, float& p_hat) {
-#if RISLTC_CANDIDATE_PAIRS
-	return allow_clip ? binned_candidate_pair<P, false>(f, record, true, p_hat)
-	                  : binned_candidate_pair<P, true>(f, record, false, p_hat);
-#else
-	// The first pass (allow_clip false) takes the branch-free square root;
-	// deferred items are evaluated with the general one.
-	if (!allow_clip) return binned_candidate<P, true>(f, record, false, p_hat);
-	// Deferred items: the branch-free forms where they apply (every item
-	// seen so far), the general ones otherwise.
-	return binned_candidate<P, true>(f, record, true, p_hat) || binned_candidate<P, false>(f, record, true, p_hat);
-#endif
+RL_DEV bool evaluate_candidate(const float4* f, const float4* record, float neg_zero, bool allow_clip, float& p_hat) {
+	if (!allow_clip) return candidate_first_pass(f, record, neg_zero, p_hat);
+	return binned_candidate<P, true>(f, record, p_hat) || binned_candidate<P, false>(f, record, p_hat);
 }
 template <>
-RL_DEV bool evaluate_candidate<FastNumerics>(const float4* f, const float4* record, bool allow_clip, float& p_hat) {
+RL_DEV bool evaluate_candidate<FastNumerics>(const float4* f, const float4* record, float, bool allow_clip, float& p_hat) {
 	return binned_candidate_pair<FastNumerics>(f, record, allow_clip, p_hat);
 }
 
@@ -624,7 +620,7 @@ RL_DEV void binned_tile(const RisParams& pr, WarpTile<BinnedSuper<P>::value, kPi
 							const uint32_t slot = item & 1023u;
 							const int32_t l = (int32_t) (item >> 10);
 							float ph;
-							if (evaluate_candidate<P>(tile.frame[slot / kSuper], light_record(pr.scene, l), false, ph)) {
+							if (evaluate_candidate<P>(tile.frame[slot / kSuper], light_record(pr.scene, l), pr.neg_zero, false, ph)) {
 								uphat[slot] = ph;
 							} else {
 								const uint32_t d = atomicAdd(&tile.deferred_count, 1u);
@@ -639,7 +635,7 @@ RL_DEV void binned_tile(const RisParams& pr, WarpTile<BinnedSuper<P>::value, kPi
 						const uint32_t slot = tile.deferred[d] & 1023u;
 						float ph = 0.0f;
 						evaluate_candidate<P>(tile.frame[slot / kSuper], light_record(pr.scene, (int) (tile.deferred[d] >> 10)),
-						                      true, ph);
+						                      pr.neg_zero, true, ph);
 						phat[tile.deferred_unit[d] * kUnitSlots + slot] = ph;
 						__syncwarp();
 						if (lane == 0) tile.deferred_count = pending - 32;
@@ -655,7 +651,7 @@ RL_DEV void binned_tile(const RisParams& pr, WarpTile<BinnedSuper<P>::value, kPi
 				const uint32_t slot = tile.deferred[lane] & 1023u;
 				float ph = 0.0f;
 				evaluate_candidate<P>(tile.frame[slot / kSuper], light_record(pr.scene, (int) (tile.deferred[lane] >> 10)),
-				                      true, ph);
+				                      pr.neg_zero, true, ph);
 				phat[tile.deferred_unit[lane] * kUnitSlots + slot] = ph;
 			}
 			__syncwarp();

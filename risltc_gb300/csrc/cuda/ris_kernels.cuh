@@ -76,6 +76,7 @@ struct RisParams {
 	double* accum;
 	risltc_reservoir_t* reservoirs;
 	uint32_t* error;
+	float neg_zero;  // -0: the addend of PairExact::mul, unknown to the code generator
 };
 
 // Sum of integrate_edge over the n edges of an unclipped polygon in slot
