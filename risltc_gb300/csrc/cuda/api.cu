@@ -326,7 +326,7 @@ EXTERN_C int risltc_scene_create(risltc_ctx_t* ctx, const float* lights_std140, 
 	for (size_t i = 0; i != 9 * (size_t) triangle_count; ++i)
 		if (!std::isfinite(triangles[i])) return RISLTC_ERROR_NON_FINITE;
 	cudaSetDevice(ctx->device);
-	// Lights: 160-byte records {radiance, vertex_count | plane | 8 x {xyz, 0}},
+	// Lights: 160-byte records {radiance, vertex_count | 8 x {xyz, 0} | plane},
 	// then the vertex counts as bytes.
 	const size_t stride = 12 + 4 * (size_t) max_vertex_count;
 	std::vector<float> lights((size_t) light_count * risltc::kLightWords, 0.0f);
@@ -340,14 +340,9 @@ EXTERN_C int risltc_scene_create(risltc_ctx_t* ctx, const float* lights_std140, 
 		d[1] = s[1];
 		d[2] = s[2];
 		memcpy(d + 3, &vc, 4);
-		for (int c = 0; c != 4; ++c) d[4 + c] = s[4 + c];
-		for (uint32_t v = 0; v != RISLTC_MAX_LIGHT_VERTEX_COUNT; ++v) {
-			const float* src = s + 12 + 4 * (v < vc ? v : 0);
-			d[8 + 4 * v + 0] = src[0];
-			d[8 + 4 * v + 1] = src[1];
-			d[8 + 4 * v + 2] = src[2];
-			d[8 + 4 * v + 3] = 0.0f;
-		}
+		for (int c = 0; c != 4; ++c) d[4 * risltc::kRecordPlane + c] = s[4 + c];
+		for (uint32_t v = 0; v != RISLTC_MAX_LIGHT_VERTEX_COUNT; ++v)
+			memcpy(d + 4 * (risltc::kRecordVertex + v), s + 12 + 4 * (v < vc ? v : 0), 3 * sizeof(float));
 	}
 	// LTC: 8 floats per texel {m00, -m02, m11, m20, m22, albedo, 0, 0}.
 	size_t texels = (size_t) ltc->roughness_count * ltc->inclination_count * ltc->fresnel_count;
@@ -459,7 +454,7 @@ EXTERN_C int risltc_scene_set_clusters(risltc_scene_t* scene, const uint32_t* of
 		if (offsets[c + 1] < offsets[c]) return RISLTC_ERROR_INVALID_ARGUMENT;
 	cudaSetDevice(scene->ctx->device);
 	cudaStreamSynchronize(scene->ctx->stream);
-	// The device light records {radiance, count}, plane, 8 vertex slots, as
+	// The device light records {radiance, count}, 8 vertex slots, plane, as
 	// std140 rows for risltc_cluster_summaries.
 	std::vector<float> rec((size_t) n * risltc::kLightWords);
 	cudaError_t e = cudaMemcpy(rec.data(), scene->d_lights, rec.size() * sizeof(float), cudaMemcpyDeviceToHost);
@@ -471,10 +466,10 @@ EXTERN_C int risltc_scene_set_clusters(risltc_scene_t* scene, const uint32_t* of
 		const float* r = &rec[(size_t) l * risltc::kLightWords];
 		float* row = &std140[stride * l];
 		for (int a = 0; a != 3; ++a) row[a] = r[a];
-		for (int a = 0; a != 4; ++a) row[4 + a] = r[4 + a];
+		for (int a = 0; a != 4; ++a) row[4 + a] = r[4 * risltc::kRecordPlane + a];
 		memcpy(row + 8, r + 3, sizeof(float));
 		for (uint32_t v = 0; v != maxv; ++v)
-			for (int a = 0; a != 3; ++a) row[12 + 4 * v + a] = r[8 + 4 * v + a];
+			for (int a = 0; a != 3; ++a) row[12 + 4 * v + a] = r[4 * (risltc::kRecordVertex + v) + a];
 	}
 	std::vector<float> bounds(4 * (size_t) cluster_count), power(cluster_count);
 	int st = risltc_cluster_summaries(std140.data(), n, maxv, offsets, cluster_count, bounds.data(), power.data());

@@ -35,15 +35,15 @@ RL_DEV float rsqrt_approx(float x) {
 	return y;
 }
 
-// -RN(1 / RN(sqrt(d))) in both lanes, for d in [2^-76, 2^126] (as words
-// [kRootMin, kRootMax]).  The root is g = d * rsqrt(d) corrected once: the
+// -RN(1 / RN(sqrt(d))) in both lanes, for every finite d of 2^-76 or more
+// (as words [kRootMin, kRootMax]).  The root is g = d * rsqrt(d) corrected once: the
 // remainder d - g^2 comes from one fused multiply-add and is added with half
 // the approximate reciprocal root; the reciprocal is Markstein's correction
 // of the hardware reciprocal, taken of -s so that no sign has to change.
 // Ten operations against fourteen of rcp_markstein(sqrt_tuckerman(d)), none
 // of them a comparison.  A GPU test compares both lanes with
 // __frcp_rn(__fsqrt_rn(d)) on every float of the range.
-constexpr uint32_t kRootMin = 0x19800000u, kRootMax = 0x7e800000u;
+constexpr uint32_t kRootMin = 0x19800000u, kRootMax = 0x7f7fffffu;
 RL_DEV float2 rsqrt_negated(const PairExact& o, float2 d) {
 	const float2 y = make_float2(rsqrt_approx(d.x), rsqrt_approx(d.y));
 	const float2 g = o.mul(d, y);

@@ -34,18 +34,19 @@
 
 namespace risltc {
 
-// Blocks per SM the candidate kernel is compiled for (register budget):
-// measured best 5 in exact numerics (96 registers; 11.27 ms per 4-frame 1080p
-// launch against 11.65 with 4 and 18.05 with 6) and 4 in fast numerics, which
-// spills at 96 registers.
+// Blocks per SM the candidate kernel is compiled for (register budget).
+// Exact numerics 6 (80 registers): 8.46 ms per 4-frame 1080p launch with
+// 16,384 lights against 8.89 with 5, 9.30 with 4 and 9.05 with 7.  Fast
+// numerics 5: 1.71 ms per 2-frame 720p launch with 4,096 lights against 1.80
+// with 4 and 1.81 with 6.
 #ifndef RISLTC_BINNED_MIN_BLOCKS_EXACT
-#define RISLTC_BINNED_MIN_BLOCKS_EXACT 5
+#define RISLTC_BINNED_MIN_BLOCKS_EXACT 6
 #endif
 #ifndef RISLTC_BINNED_MIN_BLOCKS_FAST
-#define RISLTC_BINNED_MIN_BLOCKS_FAST 4
+#define RISLTC_BINNED_MIN_BLOCKS_FAST 5
 #endif
 
-// A warp's p_hat values, [window unit][pixel lane][candidate], live in its
+// A warp's p_hat values, [window unit][candidate][pixel lane], live in its
 // slot of RisParams::p_hat_scratch (global memory, L2/L1): keeping them out
 // of shared memory leaves room in the SM's combined L1/shared storage for
 // the light records the candidates read.  A slot holds 4096 values: four
@@ -72,9 +73,17 @@ template <class P> struct BinnedMinBlocks {
 template <> struct BinnedMinBlocks<FastNumerics> {
 	static constexpr int value = RISLTC_BINNED_MIN_BLOCKS_FAST;
 };
-// A pixel's LTC frame in 11 16-byte words (an odd number of them, so that
-// the 16-byte reads of 8 lanes from different pixels spread over the banks).
-constexpr int kFrameQuads = 11;
+// A pixel's LTC frame in 7 16-byte words (an odd number of them, so that the
+// 16-byte reads of 8 lanes from different pixels spread over the banks):
+// word 0 {diffuse albedo, LTC albedo}, then the world-to-shading and
+// world-to-cosine matrices (mat4x3, column-major) element by element in
+// pairs {shading, cosine}.
+//
+// The side flip (shading_pass.frag.glsl:424-428) is left out: it negates the
+// y row of both matrices (shading_to_cosine couples y with nothing), which
+// changes neither z nor any dot product and negates every edge integral, so
+// the integrals' magnitudes, and with them p_hat, are the same bit for bit.
+constexpr int kFrameQuads = 7;
 constexpr int kBinnedWarps = 4;              // warps per block
 constexpr int kBins = kMaxLightVertices - 2; // vertex counts 3..8
 
@@ -84,46 +93,44 @@ template <int kSuper, int kPixels, int kChunk> struct WarpTile {
 	static_assert(kItems < 1024, "10-bit bin counters");
 	static_assert(kSuper % kChunk == 0 && kPixels * kSuper <= 1024, "super-chunk layout (10-bit slots)");
 	float4 frame[kPixels][kFrameQuads];
-	// Items as light << 10 | slot, slot = pixel lane * kSuper + candidate of
-	// the super-chunk (below 1024; lights below 2^22).
+	// Items as light << 10 | slot, slot = candidate of the super-chunk *
+	// kPixels + pixel lane (below 1024; lights below 2^22).
 	uint32_t item[kItems];
 	uint32_t deferred[kDeferred];
 	uint8_t deferred_unit[kDeferred];  // the window unit of each deferred item
 	uint32_t deferred_count;
 };
 
-// Frame layout (16-byte words): 0 {position, LTC albedo}, 1 {diffuse
-// albedo, 0}, 2-4 world to shading, 5-7 world to cosine, 8-10 its y-flipped
-// counterpart; each mat4x3's 12 floats column-major across three words.
-RL_DEV void store_matrix(float4* q, const mat43& m) {
-	q[0] = make_float4(m.c[0].x, m.c[0].y, m.c[0].z, m.c[1].x);
-	q[1] = make_float4(m.c[1].y, m.c[1].z, m.c[2].x, m.c[2].y);
-	q[2] = make_float4(m.c[2].z, m.c[3].x, m.c[3].y, m.c[3].z);
+RL_DEV void store_frame(float4* f, f3 diffuse_albedo, float ltc_albedo, const mat43& w2s, const mat43& w2c) {
+	f[0] = make_float4(diffuse_albedo.x, diffuse_albedo.y, diffuse_albedo.z, ltc_albedo);
+#pragma unroll
+	for (int c = 0; c != 4; c += 2) {
+		const f3 s0 = w2s.c[c], s1 = w2s.c[c + 1], c0 = w2c.c[c], c1 = w2c.c[c + 1];
+		float4* const q = f + 1 + 3 * (c / 2);
+		q[0] = make_float4(s0.x, c0.x, s0.y, c0.y);
+		q[1] = make_float4(s0.z, c0.z, s1.x, c1.x);
+		q[2] = make_float4(s1.y, c1.y, s1.z, c1.z);
+	}
 }
-RL_DEV mat43 load_matrix(const float4* q) {
-	const float4 a = q[0], b = q[1], c = q[2];
+// The frame's matrix of one space (0 shading, 1 cosine).
+RL_DEV mat43 load_matrix(const float4* f, int space) {
+	float e[12];
+#pragma unroll
+	for (int k = 0; k != 6; ++k) {
+		const float4 q = f[1 + k];
+		e[2 * k] = space == 0 ? q.x : q.y;
+		e[2 * k + 1] = space == 0 ? q.z : q.w;
+	}
 	mat43 m;
-	m.c[0] = mk3(a.x, a.y, a.z);
-	m.c[1] = mk3(a.w, b.x, b.y);
-	m.c[2] = mk3(b.z, b.w, c.x);
-	m.c[3] = mk3(c.y, c.z, c.w);
+#pragma unroll
+	for (int c = 0; c != 4; ++c) m.c[c] = mk3(e[3 * c], e[3 * c + 1], e[3 * c + 2]);
 	return m;
 }
-RL_DEV void store_frame(float4* f, const CandidateFrame& cf) {
-	f[0] = make_float4(cf.position.x, cf.position.y, cf.position.z, cf.ltc_albedo);
-	f[1] = make_float4(cf.diffuse_albedo.x, cf.diffuse_albedo.y, cf.diffuse_albedo.z, 0.0f);
-	store_matrix(f + 2, cf.w2s);
-	store_matrix(f + 5, cf.w2c[0]);
-	store_matrix(f + 8, cf.w2c[1]);
-}
 
-// A light vertex (slot j of the record) in local space: mat4x3 * vec4(v, 1)
-// with y negated when negate_y is set (the side flip).
-RL_DEV f3 local_vertex(const mat43& t, const float4* record, uint32_t j, bool negate_y) {
-	const float4 q = __ldg(record + 2 + j);
-	f3 v = mul_point(t, mk3(q.x, q.y, q.z));
-	v.y = negate_y ? -v.y : v.y;
-	return v;
+// A light vertex (slot j of the record) in local space: mat4x3 * vec4(v, 1).
+RL_DEV f3 local_vertex(const mat43& t, const float4* record, uint32_t j) {
+	const float4 q = __ldg(record + kRecordVertex + j);
+	return mul_point(t, mk3(q.x, q.y, q.z));
 }
 
 // The partially clipped case, streamed: the integral calculate_ltc gives
@@ -136,20 +143,20 @@ RL_DEV f3 local_vertex(const mat43& t, const float4* record, uint32_t j, bool ne
 // clips to nothing.  With kChecked, uses the branch-free normalisation and
 // edge integral and clears ok where they do not apply.
 template <class P, bool kChecked>
-RL_DEV float clipped_integral(const mat43& t, const float4* record, uint32_t n, bool negate_y, uint32_t mask, bool& ok) {
+RL_DEV float clipped_integral(const mat43& t, const float4* record, uint32_t n, uint32_t mask, bool& ok) {
 	const uint32_t k = __popc(mask);
 	const uint32_t s = clip_run_start(n, mask);
 	if (s == n) return -1.0f;
 	const uint32_t e = clip_wrap(s + k - 1, n), vc = k + 2;
-	const f3 entry = iz0<P>(local_vertex(t, record, clip_wrap(s + n - 1, n), negate_y), local_vertex(t, record, s, negate_y));
-	const f3 exit = iz0<P>(local_vertex(t, record, e, negate_y), local_vertex(t, record, clip_wrap(e + 1, n), negate_y));
+	const f3 entry = iz0<P>(local_vertex(t, record, clip_wrap(s + n - 1, n)), local_vertex(t, record, s));
+	const f3 exit = iz0<P>(local_vertex(t, record, e), local_vertex(t, record, clip_wrap(e + 1, n)));
 	const uint32_t j0 = clip_wrap(vc - clip_rotation(n, k, s), vc);  // cycle element of slot 0
 	f3 first = splat(0.0f), prev = splat(0.0f);
 	float r = 0.0f;
 #pragma unroll 1
 	for (uint32_t slot = 0; slot != vc; ++slot) {
 		const uint32_t j = clip_wrap(j0 + slot, vc);
-		const f3 v = j == 0 ? entry : (j == k + 1 ? exit : local_vertex(t, record, clip_wrap(s + j - 1, n), negate_y));
+		const f3 v = j == 0 ? entry : (j == k + 1 ? exit : local_vertex(t, record, clip_wrap(s + j - 1, n)));
 		const f3 cur = kChecked ? normalize_checked<P>(v, ok) : normalize<P>(v);
 		if (slot == 0)
 			first = cur;
@@ -163,9 +170,8 @@ RL_DEV float clipped_integral(const mat43& t, const float4* record, uint32_t n, 
 
 // One candidate (ltc_cp_candidate, then p_hat = length(color)) with the
 // frame in shared memory.  The two LTC integrals run in one loop over the
-// spaces.  Each polygon streams vertex by vertex from the light record (the
-// next vertex's load issued before the current one is used): every vertex is
-// transformed, counted if above the horizon, normalised and joined to the
+// spaces.  Each polygon streams vertex by vertex from the light record: every
+// vertex is transformed, counted if above the horizon, normalised and joined to the
 // previous one in the edge order of calculate_ltc (edges 0-1, ...,
 // (n-2)-(n-1), then (n-1)-0).  The sum is kept when the whole polygon is
 // above the horizon (the common case); a polygon entirely below contributes
@@ -179,30 +185,22 @@ RL_DEV bool binned_candidate(const float4* f, const float4* record, float& p_hat
 	// apply (a squared length outside the square root's range, an edge of 90
 	// degrees or more), and the caller takes the general forms.
 	bool ok = true;
-	const float4 head = __ldg(record), pl = __ldg(record + 1);
+	const float4 head = __ldg(record);
 	const uint32_t n = __float_as_uint(head.w);
-	const float plane[4] = {pl.x, pl.y, pl.z, pl.w};
 	const float4 f0 = f[0];
-	const bool flip = plane_dot(mk3(f0.x, f0.y, f0.z), plane) < 0.0f;
 	float integral[2];
 	bool away[2];
 #pragma unroll 1
 	for (int s = 0; s != 2; ++s) {
-		const mat43 t = load_matrix(f + (s == 0 ? 2 : (flip ? 8 : 5)));
-		const bool negate_y = s == 0 && flip;
-		float4 q = __ldg(record + 2);
-		f3 v = mul_point(t, mk3(q.x, q.y, q.z));
-		v.y = negate_y ? -v.y : v.y;
-		q = __ldg(record + 3);
+		const mat43 t = load_matrix(f, s);
+		f3 v = local_vertex(t, record, 0);
 		uint32_t mask = v.z > 0.0f ? 1u : 0u;  // bit j: vertex j above the horizon
 		const f3 first = kChecked ? normalize_checked<P>(v, ok) : normalize<P>(v);
 		f3 prev = first;
 		float r = 0.0f;
 #pragma unroll 1
 		for (uint32_t j = 1; j != n; ++j) {
-			v = mul_point(t, mk3(q.x, q.y, q.z));
-			v.y = negate_y ? -v.y : v.y;
-			q = __ldg(record + 2 + min(j + 1, (uint32_t) kMaxLightVertices - 1));
+			v = local_vertex(t, record, j);
 			mask |= (v.z > 0.0f ? 1u : 0u) << j;
 			const f3 cur = kChecked ? normalize_checked<P>(v, ok) : normalize<P>(v);
 			r += kChecked ? integrate_edge_checked<P>(prev, cur, ok) : integrate_edge<P>(prev, cur);
@@ -217,7 +215,7 @@ RL_DEV bool binned_candidate(const float4* f, const float4* record, float& p_hat
 			r = 0.0f;
 			a = true;
 		} else {
-			r = clipped_integral<P, kChecked>(t, record, n, negate_y, mask, ok);
+			r = clipped_integral<P, kChecked>(t, record, n, mask, ok);
 			if (kChecked && !ok) return false;
 			a = r < 0.0f;
 			r = a ? 0.0f : r;
@@ -232,10 +230,9 @@ RL_DEV bool binned_candidate(const float4* f, const float4* record, float& p_hat
 	}
 	const f3 radiance = mk3(head.x, head.y, head.z);
 	f3 result = splat(0.0f);
-	const float4 f1 = f[1];
-	const f3 diffuse = away[0] ? splat(0.0f) : mul(scale(mk3(f1.x, f1.y, f1.z), integral[0]), radiance);
+	const f3 diffuse = away[0] ? splat(0.0f) : mul(scale(mk3(f0.x, f0.y, f0.z), integral[0]), radiance);
 	result = add(result, diffuse);
-	const f3 ggx = away[1] ? splat(0.0f) : mul(splat(integral[1] * f[0].w), radiance);
+	const f3 ggx = away[1] ? splat(0.0f) : mul(splat(integral[1] * f0.w), radiance);
 	const f3 color = add(result, ggx);
 	if (kChecked) {
 		p_hat = sqrt_checked<P>(dot(color, color), ok);
@@ -264,6 +261,31 @@ struct f3x2 {
 struct mat43x2 {
 	f3x2 c[4];
 };
+RL_DEV mat43x2 load_pairs(const float4* f) {
+	mat43x2 m;
+#pragma unroll
+	for (int c = 0; c != 4; c += 2) {
+		const float4 a = f[1 + 3 * (c / 2)], b = f[2 + 3 * (c / 2)], d = f[3 + 3 * (c / 2)];
+		m.c[c] = {make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y)};
+		m.c[c + 1] = {make_float2(b.z, b.w), make_float2(d.x, d.y), make_float2(d.z, d.w)};
+	}
+	return m;
+}
+// Two consecutive 16-byte words of a light record in one 32-byte load: the
+// lanes of a warp read 32 unrelated records, and each such load costs L1 32
+// tag lookups whatever its width, which with 16-byte loads bound the kernel
+// (L1 73% busy; with these 58%).  (volatile: the loads stay where they are
+// written, ahead of their use.)
+struct RecordWords {
+	float4 a, b;
+};
+RL_DEV RecordWords load_words(const float4* p) {
+	RecordWords w;
+	asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+	             : "=f"(w.a.x), "=f"(w.a.y), "=f"(w.a.z), "=f"(w.a.w), "=f"(w.b.x), "=f"(w.b.y), "=f"(w.b.z), "=f"(w.b.w)
+	             : "l"(p));
+	return w;
+}
 template <class P> RL_DEV f3x2 mul_point2(const mat43x2& m, float4 q) {
 	const float2 px = pair(q.x), py = pair(q.y), pz = pair(q.z);
 	f3x2 r;
@@ -294,34 +316,21 @@ template <class P> RL_DEV float2 integrate_edge2(const f3x2& v1, const f3x2& v2)
 }
 
 template <class P>
-RL_DEV bool binned_candidate_pair(const float4* f, const float4* record, bool allow_clip, float& p_hat) {
-	const float4 head = __ldg(record), pl = __ldg(record + 1);
+RL_DEV void binned_candidate_pair(const float4* f, const float4* record, float& p_hat) {
+	const float4 head = __ldg(record);
 	const uint32_t n = __float_as_uint(head.w);
-	const float plane[4] = {pl.x, pl.y, pl.z, pl.w};
 	const float4 f0 = f[0];
-	const bool flip = plane_dot(mk3(f0.x, f0.y, f0.z), plane) < 0.0f;
-	// Lane .x: world to shading space (y negated on a flip); lane .y: world
-	// to cosine space (the y-flipped matrix on a flip).
-	const mat43 ms = load_matrix(f + 2), mc = load_matrix(f + (flip ? 8 : 5));
-	mat43x2 t;
-#pragma unroll
-	for (int c = 0; c != 4; ++c) {
-		t.c[c].x = make_float2(ms.c[c].x, mc.c[c].x);
-		t.c[c].y = make_float2(ms.c[c].y, mc.c[c].y);
-		t.c[c].z = make_float2(ms.c[c].z, mc.c[c].z);
-	}
+	const mat43x2 t = load_pairs(f);
 	// Vertices 0 and 1 first; then iteration j normalises vertex j + 1 while
 	// it integrates edge (j - 1, j), so the two dependency chains overlap.
 	// The edges are added in calculate_ltc's order: (0, 1), ..., (n - 2,
 	// n - 1), then (n - 1, 0).
-	const float4 q0 = __ldg(record + 2), q1 = __ldg(record + 3);
-	float4 q = __ldg(record + 4);
+	const float4 q0 = __ldg(record + kRecordVertex), q1 = __ldg(record + kRecordVertex + 1);
+	float4 q = __ldg(record + kRecordVertex + 2);
 	f3x2 v = mul_point2<P>(t, q0);
-	if (flip) v.y.x = -v.y.x;
 	uint32_t above_s = v.z.x > 0.0f ? 1u : 0u, above_c = v.z.y > 0.0f ? 1u : 0u;  // bit j: vertex j above
 	const f3x2 first = normalize2<P>(v);
 	v = mul_point2<P>(t, q1);
-	if (flip) v.y.x = -v.y.x;
 	above_s |= (v.z.x > 0.0f ? 1u : 0u) << 1;
 	above_c |= (v.z.y > 0.0f ? 1u : 0u) << 1;
 	f3x2 prev = first, cur = normalize2<P>(v);
@@ -331,8 +340,7 @@ RL_DEV bool binned_candidate_pair(const float4* f, const float4* record, bool al
 		f3x2 next = first;
 		if (j + 1 != n) {
 			v = mul_point2<P>(t, q);
-			if (flip) v.y.x = -v.y.x;
-			q = __ldg(record + 2 + min(j + 2, (uint32_t) kMaxLightVertices - 1));
+					q = __ldg(record + kRecordVertex + min(j + 2, (uint32_t) kMaxLightVertices - 1));
 			above_s |= (v.z.x > 0.0f ? 1u : 0u) << (j + 1);
 			above_c |= (v.z.y > 0.0f ? 1u : 0u) << (j + 1);
 			next = normalize2<P>(v);
@@ -343,8 +351,6 @@ RL_DEV bool binned_candidate_pair(const float4* f, const float4* record, bool al
 	}
 	r = padd<P>(r, integrate_edge2<P>(prev, first));
 	const uint32_t all = (1u << n) - 1u;
-	const bool partial_s = above_s != all && above_s != 0, partial_c = above_c != all && above_c != 0;
-	if ((partial_s || partial_c) && !allow_clip) return false;
 	float integral[2];
 	bool away[2];
 	const uint32_t above[2] = {above_s, above_c};
@@ -359,9 +365,8 @@ RL_DEV bool binned_candidate_pair(const float4* f, const float4* record, bool al
 			rs = 0.0f;
 			a = true;
 		} else {
-			const mat43 ts = s == 0 ? ms : mc;
 			bool unused = true;
-			rs = clipped_integral<P, false>(ts, record, n, s == 0 && flip, above[s], unused);
+			rs = clipped_integral<P, false>(load_matrix(f, s), record, n, above[s], unused);
 			a = rs < 0.0f;
 			rs = a ? 0.0f : rs;
 		}
@@ -370,96 +375,129 @@ RL_DEV bool binned_candidate_pair(const float4* f, const float4* record, bool al
 	}
 	const f3 radiance = mk3(head.x, head.y, head.z);
 	f3 result = splat(0.0f);
-	const float4 f1 = f[1];
-	const f3 diffuse = away[0] ? splat(0.0f) : mul(scale(mk3(f1.x, f1.y, f1.z), integral[0]), radiance);
+	const f3 diffuse = away[0] ? splat(0.0f) : mul(scale(mk3(f0.x, f0.y, f0.z), integral[0]), radiance);
 	result = add(result, diffuse);
-	const f3 ggx = away[1] ? splat(0.0f) : mul(splat(integral[1] * f[0].w), radiance);
+	const f3 ggx = away[1] ? splat(0.0f) : mul(splat(integral[1] * f0.w), radiance);
 	const f3 color = add(result, ggx);
 	p_hat = P::sqrt(dot(color, color));
-	return true;
 }
 
-// The first pass of exact numerics: one candidate with no branch in its
-// vertex loop.  False (the caller defers the item to binned_candidate, which
-// clips) when a space clips the polygon partially, a squared length lies
-// outside the square root's range or an edge spans 90 degrees or more.
+// The first pass's operations per numerics mode.  Both return sums and
+// quotients of one sign throughout (see candidate_first_pass).
 //
-// Every normalised vertex is kept negated: the reciprocal of -s gives
-// Markstein's correction without a sign change, and dot products and cross
+// Exact numerics keeps every normalised vertex negated: the reciprocal of -s
+// gives Markstein's correction without a sign change, and dot and cross
 // products of two negated vertices equal those of the vertices.  The edge
 // integral's quotient is negated in the same way, so the sum is the negated
 // sum, whose magnitude is what is kept.
-//
-// Against the scalar form that ran the two spaces one after the other: the
-// candidate kernel takes 11.27 instead of 13.89 ms per 4-frame 1080p launch
-// with 16,384 lights, 2.77 instead of 3.22 ms per frame with 1,024.
-RL_DEV bool candidate_first_pass(const float4* f, const float4* record, float neg_zero, float& p_hat) {
-	const PairExact o{pair(neg_zero)};
-	const float4 head = __ldg(record), pl = __ldg(record + 1);
-	float4 q = __ldg(record + 2);
-	const uint32_t n = __float_as_uint(head.w);
-	const float plane[4] = {pl.x, pl.y, pl.z, pl.w};
-	const float4 f0 = f[0];
-	const bool flip = plane_dot(mk3(f0.x, f0.y, f0.z), plane) < 0.0f;
-	f3x2 t[4];
-	{
-		// A side flip negates shading space's y: the row is negated here
-		// (negation is exact and rounding symmetric).
-		const mat43 ms = load_matrix(f + 2), mc = load_matrix(f + (flip ? 8 : 5));
-		const uint32_t sign = flip ? 0x80000000u : 0u;
-#pragma unroll
-		for (int c = 0; c != 4; ++c) {
-			t[c].x = make_float2(ms.c[c].x, mc.c[c].x);
-			t[c].y = make_float2(__uint_as_float(__float_as_uint(ms.c[c].y) ^ sign), mc.c[c].y);
-			t[c].z = make_float2(ms.c[c].z, mc.c[c].z);
-		}
+struct FirstPassExact {
+	PairExact o;
+	RL_DEV explicit FirstPassExact(float neg_zero) : o{pair(neg_zero)} {}
+	RL_DEV float2 row(float2 c0, float2 c1, float2 c2, float2 c3, float2 px, float2 py, float2 pz) const {
+		return o.add(o.add(o.add(o.mul(c0, px), o.mul(c1, py)), o.mul(c2, pz)), c3);
 	}
-	// What decides whether the branch-free forms apply: the least and the
-	// greatest squared length (as unsigned words: NaN and negative values lie
-	// above every number), the least cosine of an edge, and per space the
-	// least and the greatest z (as signed words, ordered like the floats
-	// where both are positive; -0 counts as below, +0 as not above).
-	uint32_t d_min = 0xffffffffu, d_max = 0;
-	int32_t x_min = 0x7fffffff, zs_min = 0x7fffffff, zs_max = INT32_MIN, zc_min = 0x7fffffff, zc_max = INT32_MIN;
-	auto vertex = [&](float4 q) -> f3x2 {  // transformed, normalised and negated
-		const float2 px = pair(q.x), py = pair(q.y), pz = pair(q.z);
-		f3x2 v;
-		v.x = o.add(o.add(o.add(o.mul(t[0].x, px), o.mul(t[1].x, py)), o.mul(t[2].x, pz)), t[3].x);
-		v.y = o.add(o.add(o.add(o.mul(t[0].y, px), o.mul(t[1].y, py)), o.mul(t[2].y, pz)), t[3].y);
-		v.z = o.add(o.add(o.add(o.mul(t[0].z, px), o.mul(t[1].z, py)), o.mul(t[2].z, pz)), t[3].z);
-		zs_min = min(zs_min, __float_as_int(v.z.x));
-		zs_max = max(zs_max, __float_as_int(v.z.x));
-		zc_min = min(zc_min, __float_as_int(v.z.y));
-		zc_max = max(zc_max, __float_as_int(v.z.y));
-		const float2 d = o.add(o.add(o.mul(v.x, v.x), o.mul(v.y, v.y)), o.mul(v.z, v.z));
-		d_min = __vimin3_u32(d_min, __float_as_uint(d.x), __float_as_uint(d.y));
-		d_max = __vimax3_u32(d_max, __float_as_uint(d.x), __float_as_uint(d.y));
+	RL_DEV float2 dot(const f3x2& a, const f3x2& b) const {
+		return o.add(o.add(o.mul(a.x, b.x), o.mul(a.y, b.y)), o.mul(a.z, b.z));
+	}
+	RL_DEV f3x2 normalized(const f3x2& v, float2 d) const {
 		const float2 nr = rsqrt_negated(o, d);
 		return {o.mul(v.x, nr), o.mul(v.y, nr), o.mul(v.z, nr)};
-	};
-	auto edge = [&](const f3x2& a, const f3x2& b) -> float2 {  // integrate_edge, negated
-		const float2 x = o.add(o.add(o.mul(a.x, b.x), o.mul(a.y, b.y)), o.mul(a.z, b.z));
-		x_min = __vimin3_s32(x_min, __float_as_int(x.x), __float_as_int(x.y));
-		return o.mul(o.sub(o.mul(a.x, b.y), o.mul(a.y, b.x)), edge_fit_negated(o, x));
-	};
-	f3x2 prev = vertex(q);
-	const f3x2 first = prev;
-	q = __ldg(record + 3);
-	float2 r = pair(0.0f);
-#pragma unroll 1
-	for (uint32_t j = 1; j != n; ++j) {
-		const f3x2 cur = vertex(q);
-		q = __ldg(record + 2 + min(j + 1, (uint32_t) kMaxLightVertices - 1));
-		r = o.add(r, edge(prev, cur));
-		prev = cur;
 	}
-	r = o.add(r, edge(prev, first));
+	// r + the edge integral of a, b, whose dot product is x.
+	RL_DEV float2 add_edge(float2 r, const f3x2& a, const f3x2& b, float2 x) const {
+		return o.add(r, o.mul(o.sub(o.mul(a.x, b.y), o.mul(a.y, b.x)), edge_fit_negated(o, x)));
+	}
+};
+// Fast numerics: fused multiply-adds, the hardware's reciprocal square root
+// and quotient.
+struct FirstPassFast {
+	RL_DEV explicit FirstPassFast(float) {}
+	RL_DEV float2 row(float2 c0, float2 c1, float2 c2, float2 c3, float2 px, float2 py, float2 pz) const {
+		return __fadd2_rn(__ffma2_rn(c2, pz, __ffma2_rn(c1, py, __fmul2_rn(c0, px))), c3);
+	}
+	RL_DEV float2 dot(const f3x2& a, const f3x2& b) const {
+		return __ffma2_rn(a.z, b.z, __ffma2_rn(a.y, b.y, __fmul2_rn(a.x, b.x)));
+	}
+	RL_DEV f3x2 normalized(const f3x2& v, float2 d) const {
+		const float2 s = make_float2(rsqrt_approx(d.x), rsqrt_approx(d.y));
+		return {__fmul2_rn(v.x, s), __fmul2_rn(v.y, s), __fmul2_rn(v.z, s)};
+	}
+	RL_DEV float2 add_edge(float2 r, const f3x2& a, const f3x2& b, float2 x) const {
+		const float2 num = __ffma2_rn(__ffma2_rn(pair(0.0145206f), x, pair(0.4965155f)), x, pair(0.8543985f));
+		const float2 den = __ffma2_rn(__fadd2_rn(pair(4.1616724f), x), x, pair(3.4175940f));
+		const float2 t = __fmul2_rn(num, make_float2(rcp_approx(den.x), rcp_approx(den.y)));
+		const float2 ay = make_float2(-a.y.x, -a.y.y);
+		return __ffma2_rn(__ffma2_rn(a.x, b.y, __fmul2_rn(ay, b.x)), t, r);
+	}
+};
+template <class P> struct FirstPass {
+	using type = FirstPassExact;
+};
+template <> struct FirstPass<FastNumerics> {
+	using type = FirstPassFast;
+};
+
+// The first pass: one candidate with no branch in its vertex loop but the
+// loop's.  False (the caller defers the item, which is then clipped) when a
+// space clips the polygon partially, a squared length lies outside the square
+// root's range or an edge spans 90 degrees or more.
+template <class O>
+RL_DEV bool candidate_first_pass(const float4* f, const float4* record, float neg_zero, float& p_hat) {
+	const O o(neg_zero);
+	const RecordWords head = load_words(record);  // {radiance, vertex count}, vertex 0
+	RecordWords q = load_words(record + kRecordVertex + 1);  // vertices 1 and 2
+	const uint32_t n = __float_as_uint(head.a.w);
+	float2 r = pair(0.0f);
+	// What decides whether the branch-free forms apply: the least squared
+	// length (an infinite or NaN one leaves a NaN sum), the least cosine of an
+	// edge, the least z of both spaces and the greatest of each (as signed
+	// words, ordered like the floats where both are positive; -0 counts as
+	// below, +0 as not above).
+	uint32_t d_min = 0xffffffffu;
+	int32_t x_min = 0x7fffffff, z_min = 0x7fffffff, zs_max = INT32_MIN, zc_max = INT32_MIN;
+	auto edge = [&](const f3x2& a, const f3x2& b) {
+		const float2 x = o.dot(a, b);
+		x_min = __vimin3_s32(x_min, __float_as_int(x.x), __float_as_int(x.y));
+		r = o.add_edge(r, a, b, x);
+	};
+	const mat43x2 t = load_pairs(f);
+	auto vertex = [&](float4 p) -> f3x2 {  // transformed and normalised
+		const float2 px = pair(p.x), py = pair(p.y), pz = pair(p.z);
+		const f3x2 v = {o.row(t.c[0].x, t.c[1].x, t.c[2].x, t.c[3].x, px, py, pz),
+		                o.row(t.c[0].y, t.c[1].y, t.c[2].y, t.c[3].y, px, py, pz),
+		                o.row(t.c[0].z, t.c[1].z, t.c[2].z, t.c[3].z, px, py, pz)};
+		z_min = __vimin3_s32(z_min, __float_as_int(v.z.x), __float_as_int(v.z.y));
+		zs_max = max(zs_max, __float_as_int(v.z.x));
+		zc_max = max(zc_max, __float_as_int(v.z.y));
+		const float2 d = o.dot(v, v);
+		d_min = __vimin3_u32(d_min, __float_as_uint(d.x), __float_as_uint(d.y));
+		return o.normalized(v, d);
+	};
+	const f3x2 first = vertex(head.b);
+	f3x2 a = vertex(q.a), b;
+	edge(first, a);
+#pragma unroll 1
+	for (uint32_t j = 2;; j += 2) {
+		// Vertex j is in q.b; the next two are fetched while it is used.
+		RecordWords next = q;
+		if (j + 1 < n) next = load_words(record + kRecordVertex + 1 + j);
+		b = vertex(q.b);
+		edge(a, b);
+		if (j + 1 >= n) break;
+		a = vertex(next.a);
+		edge(b, a);
+		if (j + 2 >= n) {
+			b = a;
+			break;
+		}
+		q.b = next.b;
+	}
+	edge(b, first);
 	const bool below_s = zs_max <= 0, below_c = zc_max <= 0;
-	if (!(d_min >= kRootMin && d_max <= kRootMax && x_min > 0 && (zs_min > 0 || below_s) && (zc_min > 0 || below_c)))
-		return false;
-	const f3 radiance = mk3(head.x, head.y, head.z);
-	const float4 f1 = f[1];
-	const f3 diffuse = below_s ? splat(0.0f) : mul(scale(mk3(f1.x, f1.y, f1.z), fabsf(r.x)), radiance);
+	if (!(d_min >= kRootMin && x_min > 0 && (z_min > 0 || (below_s && below_c)))) return false;
+	const f3 radiance = mk3(head.a.x, head.a.y, head.a.z);
+	const float4 f0 = f[0];
+	const f3 diffuse = below_s ? splat(0.0f) : mul(scale(mk3(f0.x, f0.y, f0.z), fabsf(r.x)), radiance);
 	const f3 ggx = below_c ? splat(0.0f) : mul(splat(fabsf(r.y) * f0.w), radiance);
 	const f3 color = add(add(splat(0.0f), diffuse), ggx);
 	bool ok = true;
@@ -467,18 +505,25 @@ RL_DEV bool candidate_first_pass(const float4* f, const float4* record, float ne
 	return ok;
 }
 
-// The candidate evaluation the binned kernel uses.  Exact numerics: the
-// paired first pass, and for deferred items (allow_clip) the scalar forms,
-// branch-free where they apply, the general ones otherwise.  Fast numerics:
-// the paired form for both.
-template <class P>
-RL_DEV bool evaluate_candidate(const float4* f, const float4* record, float neg_zero, bool allow_clip, float& p_hat) {
-	if (!allow_clip) return candidate_first_pass(f, record, neg_zero, p_hat);
-	return binned_candidate<P, true>(f, record, p_hat) || binned_candidate<P, false>(f, record, p_hat);
+// A deferred candidate, clipped where it has to be.  Exact numerics: the
+// scalar forms, branch-free where they apply, the general ones otherwise.
+// Fast numerics: the paired form.
+template <class P> RL_DEV void deferred_candidate(const float4* f, const float4* record, float& p_hat) {
+	if (!binned_candidate<P, true>(f, record, p_hat)) binned_candidate<P, false>(f, record, p_hat);
 }
-template <>
-RL_DEV bool evaluate_candidate<FastNumerics>(const float4* f, const float4* record, float, bool allow_clip, float& p_hat) {
-	return binned_candidate_pair<FastNumerics>(f, record, allow_clip, p_hat);
+template <> RL_DEV void deferred_candidate<FastNumerics>(const float4* f, const float4* record, float& p_hat) {
+	binned_candidate_pair<FastNumerics>(f, record, p_hat);
+}
+
+// The reservoir's test rnd < w / w_sum (insert_in_reservoir) for w > 0: the
+// division is needed only where rnd * w_sum lies within 2^-20 of w, or where
+// a product might leave the normal range.
+template <class P> RL_DEV bool reservoir_accepts(float rnd, float w, float w_sum) {
+	const float t = rnd * w_sum;
+	const bool normal = w > 1e-25f && w_sum < 1e30f;
+	if (normal && t < w * (1.0f - 0x1p-20f)) return true;
+	if (normal && t > w * (1.0f + 0x1p-20f)) return false;
+	return rnd < P::div(w, w_sum);
 }
 
 // One warp tile t (pixels t * kPixels .. + kPixels - 1) of one frame set:
@@ -491,223 +536,209 @@ RL_DEV void binned_tile(const RisParams& pr, WarpTile<BinnedSuper<P>::value, kPi
 	const uint32_t lane = threadIdx.x % 32;
 	const uint32_t np = pr.width * pr.height;
 	const int n_lights = pr.scene.light_count;
-	const float p = P::rcp((float) n_lights);
-	// With uniform candidates and a power-of-two light count, p is a power of
-	// two and p_hat / p equals p_hat * (1 / p) bit for bit (scaling by a
-	// power of two is exact): the replay multiplies instead of dividing.
-	const bool scale_weight = !pr.candidates && (n_lights & (n_lights - 1)) == 0;
-	const float inv_p = (float) n_lights;
 	// Lanes kPixels..31 own no pixel: they draw nothing and only evaluate
 	// items of the sorted lists.
 	const bool own = lane < (uint32_t) kPixels;
-	{
-		const uint32_t i = t * kPixels + lane;
-		const bool valid = own && i < np && !(pr.primitive && pr.primitive[i] == 0xffffffffu);
-		if (valid) {
-			const float* g = pr.gbuffer;
-			const size_t snp = np;
-			const f3 position = mk3(g[0 * snp + i], g[1 * snp + i], g[2 * snp + i]);
-			const f3 normal = mk3(g[3 * snp + i], g[4 * snp + i], g[5 * snp + i]);
-			const f3 outgoing = mk3(g[6 * snp + i], g[7 * snp + i], g[8 * snp + i]);
-			const f3 fresnel_0 = mk3(g[13 * snp + i], g[14 * snp + i], g[15 * snp + i]);
-			const float roughness = g[16 * snp + i];
-			CandidateFrame cf;
-			cf.position = position;
-			cf.diffuse_albedo = mk3(g[10 * snp + i], g[11 * snp + i], g[12 * snp + i]);
-			const float fl = dot(fresnel_0, mk3(0.2126f, 0.7152f, 0.0722f));
-			const Ltc ltc = get_ltc_coefficients<P>(pr.scene, fl, roughness, position, normal, outgoing);
-			cf.ltc_albedo = ltc.albedo;
-			cf.w2s = ltc.world_to_shading;
-			mat43 flipped = ltc.world_to_shading;
+	const uint32_t i = t * kPixels + lane;
+	const bool valid = own && i < np && !(pr.primitive && pr.primitive[i] == 0xffffffffu);
+	if (valid) {
+		const float* g = pr.gbuffer;
+		const size_t snp = np;
+		const f3 position = mk3(g[0 * snp + i], g[1 * snp + i], g[2 * snp + i]);
+		const f3 normal = mk3(g[3 * snp + i], g[4 * snp + i], g[5 * snp + i]);
+		const f3 outgoing = mk3(g[6 * snp + i], g[7 * snp + i], g[8 * snp + i]);
+		const f3 fresnel_0 = mk3(g[13 * snp + i], g[14 * snp + i], g[15 * snp + i]);
+		const float roughness = g[16 * snp + i];
+		const f3 diffuse_albedo = mk3(g[10 * snp + i], g[11 * snp + i], g[12 * snp + i]);
+		const float fl = dot(fresnel_0, mk3(0.2126f, 0.7152f, 0.0722f));
+		const Ltc ltc = get_ltc_coefficients<P>(pr.scene, fl, roughness, position, normal, outgoing);
+		store_frame(tile.frame[lane], diffuse_albedo, ltc.albedo, ltc.world_to_shading,
+		            mul(ltc.shading_to_cosine, ltc.world_to_shading));
+	}
+	if (lane == 0) tile.deferred_count = 0;
+	__syncwarp();
+	// The noise state at the start of frame f (get_noise_accessor with the
+	// frame's random offset).
+	auto frame_seed = [&](uint32_t f) -> uint32_t {
+		if (!valid) return 0u;
+		const uint32_t rn_x = pr.animate ? wang_random_number((pr.noise_seed + f) * 4u) : 0u;
+		return get_noise_accessor(i % pr.width, i / pr.width, pr.width, rn_x);
+	};
+	auto drawn_light = [&](float u) -> int {
+		const int idx = (int) (u * (float) n_lights);
+		return idx > n_lights - 1 ? n_lights - 1 : idx;
+	};
+	// The tile's work comes in units of one frame's super-chunk.  Up to
+	// kWindow units are evaluated before their reservoirs are replayed, so
+	// that deferred items of several units share the general path's rounds:
+	// unit u of the window keeps its p_hat values at phat[u * kUnitSlots +
+	// slot].
+	constexpr uint32_t kUnitSlots = (uint32_t) (kPixels * kSuper);
+	constexpr uint32_t kWindow = (uint32_t) kPHatSlot / kUnitSlots;
+	const uint32_t units_per_frame = ((uint32_t) pr.candidate_count + kSuper - 1) / kSuper;
+	const uint32_t units = pr.frame_count * units_per_frame;
+	uint32_t window = 0;  // units evaluated since the last replay
+	uint32_t draw = 0;    // the draw phase's noise state
+	for (uint32_t unit = 0; unit != units; ++unit) {
+		const uint32_t f = unit / units_per_frame, cs = (unit % units_per_frame) * kSuper;
+		if (cs == 0) draw = frame_seed(f);
+		const int super_count = min(kSuper, pr.candidate_count - (int) cs);
+		const bool window_ends = window + 1 == kWindow || unit + 1 == units;
+		float* const uphat = phat + window * kUnitSlots;
+		for (int c0 = 0; c0 < super_count; c0 += kChunk) {
+			const int chunk = min(kChunk, super_count - c0);
+			// 1. This lane's candidate lights; bin them by vertex count (six
+			//    10-bit counters).
+			int light[kChunk];
+			uint32_t bin[kChunk];
+			unsigned long long counts = 0;
 #pragma unroll
-			for (int c = 0; c != 4; ++c) flipped.c[c].y = -flipped.c[c].y;
-			cf.w2c[0] = mul(ltc.shading_to_cosine, cf.w2s);
-			cf.w2c[1] = mul(ltc.shading_to_cosine, flipped);
-			store_frame(tile.frame[lane], cf);
+			for (int k = 0; k != kChunk; ++k) {
+				light[k] = -1;
+				bin[k] = kBins;
+				if (valid && k < chunk) {
+					int idx = drawn_light(get_noise_1(draw));
+					if (pr.candidates)
+						idx = pr.candidates[((size_t) f * np + i) * pr.candidate_count + cs + c0 + k].light;
+					draw = 1664525u * draw + 1013904223u;  // the reservoir's draw
+					light[k] = idx;
+					bin[k] = light_vertex_count(pr.scene, idx) - 3u;
+					counts += 1ull << (10 * bin[k]);
+				}
+			}
+			// 2. Counting sort: exclusive scan of the counters across the
+			//    warp, then each bin's start.
+			unsigned long long prefix = counts;
+#pragma unroll
+			for (int d = 1; d < 32; d <<= 1) {
+				const unsigned long long o = __shfl_up_sync(0xffffffffu, prefix, d);
+				if ((int) lane >= d) prefix += o;
+			}
+			const unsigned long long totals = __shfl_sync(0xffffffffu, prefix, 31);
+			prefix -= counts;
+			uint32_t start[kBins + 1];
+			start[0] = 0;
+#pragma unroll
+			for (int b = 0; b != kBins; ++b) start[b + 1] = start[b] + (uint32_t) ((totals >> (10 * b)) & 1023u);
+			const uint32_t item_count = start[kBins];
+#pragma unroll
+			for (int k = 0; k != kChunk; ++k) {
+				if (bin[k] < kBins) {
+					const uint32_t b = bin[k];
+					uint32_t s = 0;
+#pragma unroll
+					for (int q = 0; q != kBins; ++q)
+						if (q == (int) b) s = start[q];
+					const uint32_t pos = s + (uint32_t) ((prefix >> (10 * b)) & 1023u);
+					prefix += 1ull << (10 * b);
+					tile.item[pos] = ((uint32_t) light[k] << 10) | ((c0 + k) * kPixels + lane);
+				}
+			}
+			__syncwarp();
+			// 3. Evaluate the sorted items, 32 at a time; defer partial clips
+			//    (with their unit).
+			for (uint32_t base = 0; base < item_count; base += 32) {
+				const uint32_t it = base + lane;
+				if (it < item_count) {
+					const uint32_t item = tile.item[it];
+					const uint32_t slot = item & 1023u;
+					float ph;
+					if (candidate_first_pass<typename FirstPass<P>::type>(
+					        tile.frame[slot % kPixels], light_record(pr.scene, (int) (item >> 10)), pr.neg_zero, ph)) {
+						uphat[slot] = ph;
+					} else {
+						const uint32_t d = atomicAdd(&tile.deferred_count, 1u);
+						tile.deferred[d] = item;
+						tile.deferred_unit[d] = (uint8_t) window;
+					}
+				}
+			}
+			__syncwarp();
+			// Deferred items 32 at a time; the rest when the window ends.
+			const uint32_t least = window_ends && c0 + kChunk >= super_count ? 1u : 32u;
+			for (uint32_t pending = tile.deferred_count; pending >= least;) {
+				const uint32_t take = min(pending, 32u);
+				pending -= take;
+				if (lane < take) {
+					const uint32_t d = pending + lane;
+					const uint32_t item = tile.deferred[d], slot = item & 1023u;
+					float ph = 0.0f;
+					deferred_candidate<P>(tile.frame[slot % kPixels], light_record(pr.scene, (int) (item >> 10)), ph);
+					phat[tile.deferred_unit[d] * kUnitSlots + slot] = ph;
+				}
+				__syncwarp();
+				if (lane == 0) tile.deferred_count = pending;
+				__syncwarp();
+			}
 		}
-		__syncwarp();
-		const uint32_t x = i % pr.width, y = i / pr.width;
-		// The noise state at the start of frame f (get_noise_accessor with
-		// the frame's random offset).
-		auto frame_seed = [&](uint32_t f) -> uint32_t {
-			if (!valid) return 0u;
-			const uint32_t rn_x = pr.animate ? wang_random_number((pr.noise_seed + f) * 4u) : 0u;
-			return get_noise_accessor(x, y, pr.width, rn_x);
-		};
-		// The tile's work comes in units of one frame's super-chunk.  Up to
-		// kWindow units are evaluated before their reservoirs are replayed, so
-		// that deferred items of several units share the general path's
-		// rounds: unit u of the window keeps its p_hat values at
-		// phat[u * kUnitSlots + slot].
-		constexpr uint32_t kUnitSlots = (uint32_t) (kPixels * kSuper);
-		constexpr uint32_t kWindow = (uint32_t) kPHatSlot / kUnitSlots;
-		const uint32_t units_per_frame = ((uint32_t) pr.candidate_count + kSuper - 1) / kSuper;
-		const uint32_t units = pr.frame_count * units_per_frame;
-		// The replay's cursor: frame rf, its next super-chunk rcs, and the
-		// frame's reservoir so far.
-		uint32_t rf = 0, rcs = 0, seed = 0;
+		++window;
+		if (!window_ends) continue;
+		// 4. Reservoir updates of the window's units in candidate order,
+		//    drawing the same noise again.  A frame whose super-chunks reach
+		//    past the window leaves its reservoir in its record.
+		const float p = P::rcp((float) n_lights);
+		// With uniform candidates and a power-of-two light count, p is a power
+		// of two and p_hat / p equals p_hat * (1 / p) bit for bit (scaling by a
+		// power of two is exact): the replay multiplies instead of dividing.
+		const bool scale_weight = !pr.candidates && (n_lights & (n_lights - 1)) == 0;
+		const float inv_p = (float) n_lights;
+		uint32_t seed = 0;
 		float w_sum = 0.0f, sample_value = 0.0f;
 		int res_index = -1;
-		uint32_t window = 0;  // units evaluated since the last replay
-		uint32_t draw = 0;    // the draw phase's noise state
-		if (lane == 0) tile.deferred_count = 0;
-		__syncwarp();
-		for (uint32_t unit = 0; unit != units; ++unit) {
-			const uint32_t f = unit / units_per_frame, cs = (unit % units_per_frame) * kSuper;
-			if (cs == 0) draw = frame_seed(f);
-			const int super_count = min(kSuper, pr.candidate_count - (int) cs);
-			float* const uphat = phat + window * kUnitSlots;
-			{
-				for (int c0 = 0; c0 < super_count; c0 += kChunk) {
-					const int chunk = min(kChunk, super_count - c0);
-					// 1. This lane's candidate lights; bin them by vertex count
-					//    (six 10-bit counters).
-					int light[kChunk];
-					uint32_t bin[kChunk];
-					unsigned long long counts = 0;
-#pragma unroll
-					for (int k = 0; k != kChunk; ++k) {
-						light[k] = -1;
-						bin[k] = kBins;
-						if (valid && k < chunk) {
-							int idx = (int) (get_noise_1(draw) * (float) n_lights);
-							idx = idx > n_lights - 1 ? n_lights - 1 : idx;
-							if (pr.candidates)
-								idx = pr.candidates[((size_t) f * np + i) * pr.candidate_count + cs + c0 + k].light;
-							get_noise_1(draw);
-							light[k] = idx;
-							bin[k] = light_vertex_count(pr.scene, idx) - 3u;
-							counts += 1ull << (10 * bin[k]);
-						}
-					}
-					// 2. Counting sort: exclusive scan of the counters across
-					//    the warp, then each bin's start.
-					unsigned long long prefix = counts;
-#pragma unroll
-					for (int d = 1; d < 32; d <<= 1) {
-						const unsigned long long o = __shfl_up_sync(0xffffffffu, prefix, d);
-						if ((int) lane >= d) prefix += o;
-					}
-					const unsigned long long totals = __shfl_sync(0xffffffffu, prefix, 31);
-					prefix -= counts;
-					uint32_t start[kBins + 1];
-					start[0] = 0;
-#pragma unroll
-					for (int b = 0; b != kBins; ++b)
-						start[b + 1] = start[b] + (uint32_t) ((totals >> (10 * b)) & 1023u);
-					const uint32_t item_count = start[kBins];
-#pragma unroll
-					for (int k = 0; k != kChunk; ++k) {
-						if (bin[k] < kBins) {
-							const uint32_t b = bin[k];
-							uint32_t s = 0;
-#pragma unroll
-							for (int q = 0; q != kBins; ++q)
-								if (q == (int) b) s = start[q];
-							const uint32_t pos = s + (uint32_t) ((prefix >> (10 * b)) & 1023u);
-							prefix += 1ull << (10 * b);
-							tile.item[pos] = ((uint32_t) light[k] << 10) | (lane * kSuper + c0 + k);
-						}
-					}
-					__syncwarp();
-					// 3. Evaluate the sorted items, 32 at a time; defer partial
-					//    clips (with their unit), and evaluate deferred items
-					//    whenever 32 are pending.
-					for (uint32_t base = 0; base < item_count; base += 32) {
-						const uint32_t it = base + lane;
-						if (it < item_count) {
-							const uint32_t item = tile.item[it];
-							const uint32_t slot = item & 1023u;
-							const int32_t l = (int32_t) (item >> 10);
-							float ph;
-							if (evaluate_candidate<P>(tile.frame[slot / kSuper], light_record(pr.scene, l), pr.neg_zero, false, ph)) {
-								uphat[slot] = ph;
-							} else {
-								const uint32_t d = atomicAdd(&tile.deferred_count, 1u);
-								tile.deferred[d] = item;
-								tile.deferred_unit[d] = (uint8_t) window;
-							}
-						}
-					}
-					__syncwarp();
-					for (uint32_t pending = tile.deferred_count; pending >= 32; pending -= 32) {
-						const uint32_t d = pending - 32 + lane;
-						const uint32_t slot = tile.deferred[d] & 1023u;
-						float ph = 0.0f;
-						evaluate_candidate<P>(tile.frame[slot / kSuper], light_record(pr.scene, (int) (tile.deferred[d] >> 10)),
-						                      pr.neg_zero, true, ph);
-						phat[tile.deferred_unit[d] * kUnitSlots + slot] = ph;
-						__syncwarp();
-						if (lane == 0) tile.deferred_count = pending - 32;
-						__syncwarp();
-					}
-				}
+		for (uint32_t u = 0; u != window; ++u) {
+			const uint32_t ru = unit + 1 - window + u;
+			const uint32_t rf = ru / units_per_frame, rcs = (ru % units_per_frame) * kSuper;
+			const size_t at = (size_t) rf * np + i;
+			if (rcs == 0) {
+				seed = frame_seed(rf);
+				w_sum = 0.0f;
+				sample_value = 0.0f;
+				res_index = -1;
+			} else if (u == 0 && valid) {
+				const ReservoirRecord r = pr.records[at];
+				res_index = r.light_index;
+				w_sum = r.w_sum;
+				sample_value = r.p_hat;
+				seed = r.seed;
 			}
-			++window;
-			if (window != kWindow && unit + 1 != units) continue;
-			// The window's remaining deferred items.
-			const uint32_t rest = tile.deferred_count;
-			if (lane < rest) {
-				const uint32_t slot = tile.deferred[lane] & 1023u;
-				float ph = 0.0f;
-				evaluate_candidate<P>(tile.frame[slot / kSuper], light_record(pr.scene, (int) (tile.deferred[lane] >> 10)),
-				                      pr.neg_zero, true, ph);
-				phat[tile.deferred_unit[lane] * kUnitSlots + slot] = ph;
-			}
-			__syncwarp();
-			if (lane == 0) tile.deferred_count = 0;
-			__syncwarp();
-			// 4. Reservoir updates of the window's units in candidate order,
-			//    drawing the same noise again; a frame's record is written
-			//    after its last super-chunk.
-			for (uint32_t u = 0; u != window; ++u) {
-				if (rcs == 0) {
-					seed = frame_seed(rf);
-					w_sum = 0.0f;
-					sample_value = 0.0f;
-					res_index = -1;
-				}
-				const int rcount = min(kSuper, pr.candidate_count - (int) rcs);
-				const float* const rphat = phat + u * kUnitSlots + lane * kSuper;
-				if (valid) {
+			const int rcount = min(kSuper, pr.candidate_count - (int) rcs);
+			const float* const rphat = phat + u * kUnitSlots + lane;
+			if (valid) {
+				int chosen = -1;           // the candidate that the reservoir took last,
+				uint32_t chosen_seed = 0;  // and the noise state that drew its light
 #pragma unroll 4
-					for (int k = 0; k < rcount; ++k) {
-						int idx = (int) (get_noise_1(seed) * (float) n_lights);
-						idx = idx > n_lights - 1 ? n_lights - 1 : idx;
-						float pk = p;
-						if (pr.candidates) {
-							const ProposalCandidate q =
-							    pr.candidates[((size_t) rf * np + i) * pr.candidate_count + rcs + k];
-							idx = q.light;
-							pk = q.pdf;
-						}
-						const float rnd = get_noise_1(seed);
-						const float p_hat = rphat[k];
-						const float w = scale_weight ? p_hat * inv_p : P::div(p_hat, pk);
-						if (pr.train_stride && rf == 0 && i % pr.train_stride == pr.train_phase)
-							pr.train_candidates[(size_t) i * pr.candidate_count + rcs + k].pdf = w;
-						w_sum += w;
-						if (w > 0.0f && rnd < P::div(w, w_sum)) {
-							res_index = idx;
-							sample_value = p_hat;
-						}
+				for (int k = 0; k < rcount; ++k) {
+					seed = 1664525u * seed + 1013904223u;  // the light's draw
+					const uint32_t light_seed = seed;
+					const float rnd = get_noise_1(seed);
+					const float p_hat = rphat[k * kPixels];
+					float pk = p;
+					if (pr.candidates) pk = pr.candidates[at * pr.candidate_count + rcs + k].pdf;
+					const float w = scale_weight ? p_hat * inv_p : P::div(p_hat, pk);
+					if (pr.train_stride && rf == 0 && i % pr.train_stride == pr.train_phase)
+						pr.train_candidates[(size_t) i * pr.candidate_count + rcs + k].pdf = w;
+					w_sum += w;
+					if (w > 0.0f && reservoir_accepts<P>(rnd, w, w_sum)) {
+						chosen = k;
+						chosen_seed = light_seed;
+						sample_value = p_hat;
 					}
 				}
-				rcs += kSuper;
-				if (rcs >= (uint32_t) pr.candidate_count) {
-					if (valid)
-						pr.records[(size_t) rf * np + i] = ReservoirRecord{res_index, w_sum, sample_value, seed};
-					else if (own && i < np)
-						pr.records[(size_t) rf * np + i] = ReservoirRecord{-1, 0.0f, 0.0f, 0u};
-					++rf;
-					rcs = 0;
-				}
+				if (chosen >= 0)
+					res_index = pr.candidates ? pr.candidates[at * pr.candidate_count + rcs + chosen].light
+					                          : drawn_light(__uint2float_rn(chosen_seed) * 2.3283064365386962890625e-10f);
 			}
-			window = 0;
-			__syncwarp();
+			if (u + 1 == window || rcs + kSuper >= (uint32_t) pr.candidate_count) {
+				if (valid)
+					pr.records[at] = ReservoirRecord{res_index, w_sum, sample_value, seed};
+				else if (own && i < np)
+					pr.records[at] = ReservoirRecord{-1, 0.0f, 0.0f, 0u};
+			}
 		}
+		window = 0;
 		__syncwarp();
 	}
+	__syncwarp();
 }
 
 template <class P, int kPixels, int kChunk>

@@ -48,7 +48,7 @@ struct RisParams {
 	uint32_t animate;
 	uint32_t frame_count;
 	ReservoirRecord* records;  // [frame][pixel] scratch
-	// Per-warp scratch of the binned candidate kernel (one slot of 32 x 32
+	// Per-warp scratch of the binned candidate kernel (a slot of kPHatSlot
 	// floats per warp of the grid); null selects the one-thread-per-pixel
 	// candidate kernel.
 	float* p_hat_scratch;
@@ -125,7 +125,7 @@ RL_DEV float ltc_integral(const mat43& m, bool flip_y, const float4* record, uin
 #pragma unroll
 	for (int j = 0; j != kMaxLightVertices; ++j) {
 		// Slots past the count hold vertex 0, so they are always valid.
-		float4 q = __ldg(record + 2 + j);
+		float4 q = __ldg(record + kRecordVertex + j);
 		t.v[j] = mul_point(m, mk3(q.x, q.y, q.z));
 		t.v[j].y = flip_y ? -t.v[j].y : t.v[j].y;
 		if (j < (int) n && t.v[j].z > 0.0f) ++above;
@@ -150,7 +150,7 @@ struct CandidateFrame {
 // evaluate_polygonal_light_shading with SAMPLE_POLYGON_LTC_CP,
 // shading_pass.frag.glsl:421-456, for one candidate light record.
 template <class P> RL_DEV f3 ltc_cp_candidate(const CandidateFrame& cf, const float4* record) {
-	float4 head = __ldg(record), pl = __ldg(record + 1);
+	float4 head = __ldg(record), pl = __ldg(record + kRecordPlane);
 	const f3 radiance = mk3(head.x, head.y, head.z);
 	const uint32_t n = __float_as_uint(head.w);
 	const float plane[4] = {pl.x, pl.y, pl.z, pl.w};

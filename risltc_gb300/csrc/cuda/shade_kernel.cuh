@@ -284,7 +284,7 @@ RL_DEV uint32_t prepare_space_record(const mat43& w2l, const float4* record, Psa
 #pragma unroll
 	for (int j = 0; j != kMaxLightVertices; ++j) {
 		if (j < (int) n) {
-			const float4 q = __ldg(record + 2 + j);
+			const float4 q = __ldg(record + kRecordVertex + j);
 			verts[j] = mul_point(w2l, mk3(q.x, q.y, q.z));
 		}
 	}

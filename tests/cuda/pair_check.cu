@@ -3,7 +3,7 @@
 //
 // risltc_test_pairs(counts, neg_zero) fills counts[5]:
 //   0 lanes of rsqrt_negated differing from -__frcp_rn(__fsqrt_rn(d)) over
-//     every float d in [2^-76, 2^126];
+//     every finite float d of 2^-76 or more;
 //   1 the number of lanes checked there;
 //   2 lanes of edge_fit_negated differing from -__fdiv_rn(a(x), b(x)) over
 //     every float x in (0, 1 + 2^-15];
