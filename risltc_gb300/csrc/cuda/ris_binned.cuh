@@ -133,30 +133,38 @@ RL_DEV f3 local_vertex(const mat43& t, const float4* record, uint32_t j) {
 	return mul_point(t, mk3(q.x, q.y, q.z));
 }
 
-// The partially clipped case, streamed: the integral calculate_ltc gives
-// over the polygon clip_polygon makes (mask: the vertices above z = 0, one
-// bit each), with the clipped vertices produced one at a time in the order of
-// clip_polygon's output slots: the cycle [entry, the run above the horizon,
-// exit] starting at its rotation, the run's vertices transformed again from
-// the light record.  The same values in the same order as clip_polygon
-// followed by calculate_ltc, without a vertex array.  -1 when the polygon
-// clips to nothing.  With kChecked, uses the branch-free normalisation and
-// edge integral and clears ok where they do not apply.
+// The integral calculate_ltc gives over the part of the polygon above the
+// horizon (mask: the vertices above z = 0, one bit each, at least one),
+// streamed: with all vertices above in the record's order, otherwise with
+// the clipped vertices produced one at a time in the order of clip_polygon's
+// output slots: the cycle [entry, the run above the horizon, exit] starting
+// at its rotation, the run's vertices transformed again from the light
+// record.  The same values in the same order as clip_polygon followed by
+// calculate_ltc, without a vertex array.  -1 when the polygon clips to
+// nothing.  With kChecked, uses the branch-free normalisation and edge
+// integral and clears ok where they do not apply.
 template <class P, bool kChecked>
 RL_DEV float clipped_integral(const mat43& t, const float4* record, uint32_t n, uint32_t mask, bool& ok) {
+	const bool whole = mask == (1u << n) - 1u;
 	const uint32_t k = __popc(mask);
-	const uint32_t s = clip_run_start(n, mask);
-	if (s == n) return -1.0f;
-	const uint32_t e = clip_wrap(s + k - 1, n), vc = k + 2;
-	const f3 entry = iz0<P>(local_vertex(t, record, clip_wrap(s + n - 1, n)), local_vertex(t, record, s));
-	const f3 exit = iz0<P>(local_vertex(t, record, e), local_vertex(t, record, clip_wrap(e + 1, n)));
-	const uint32_t j0 = clip_wrap(vc - clip_rotation(n, k, s), vc);  // cycle element of slot 0
+	uint32_t s = 0, vc = n, j0 = 0;
+	f3 entry = splat(0.0f), exit = splat(0.0f);
+	if (!whole) {
+		s = clip_run_start(n, mask);
+		if (s == n) return -1.0f;
+		const uint32_t e = clip_wrap(s + k - 1, n);
+		vc = k + 2;
+		entry = iz0<P>(local_vertex(t, record, clip_wrap(s + n - 1, n)), local_vertex(t, record, s));
+		exit = iz0<P>(local_vertex(t, record, e), local_vertex(t, record, clip_wrap(e + 1, n)));
+		j0 = clip_wrap(vc - clip_rotation(n, k, s), vc);  // cycle element of slot 0
+	}
 	f3 first = splat(0.0f), prev = splat(0.0f);
 	float r = 0.0f;
 #pragma unroll 1
 	for (uint32_t slot = 0; slot != vc; ++slot) {
 		const uint32_t j = clip_wrap(j0 + slot, vc);
-		const f3 v = j == 0 ? entry : (j == k + 1 ? exit : local_vertex(t, record, clip_wrap(s + j - 1, n)));
+		f3 v = local_vertex(t, record, whole ? slot : clip_wrap(s + (j == 0 ? 0 : j - 1), n));
+		if (!whole) v = j == 0 ? entry : (j == k + 1 ? exit : v);
 		const f3 cur = kChecked ? normalize_checked<P>(v, ok) : normalize<P>(v);
 		if (slot == 0)
 			first = cur;
@@ -169,15 +177,9 @@ RL_DEV float clipped_integral(const mat43& t, const float4* record, uint32_t n, 
 }
 
 // One candidate (ltc_cp_candidate, then p_hat = length(color)) with the
-// frame in shared memory.  The two LTC integrals run in one loop over the
-// spaces.  Each polygon streams vertex by vertex from the light record: every
-// vertex is transformed, counted if above the horizon, normalised and joined to the
-// previous one in the edge order of calculate_ltc (edges 0-1, ...,
-// (n-2)-(n-1), then (n-1)-0).  The sum is kept when the whole polygon is
-// above the horizon (the common case); a polygon entirely below contributes
-// nothing, and a partially clipped one goes through clip_polygon instead.
-// The code stays small and the vertex count of a sorted group is uniform
-// across the warp.
+// frame in shared memory, of any polygon.  In each space the vertices above
+// the horizon are counted first, so that only the polygon that is kept is
+// normalised and integrated.
 template <class P, bool kChecked>
 RL_DEV bool binned_candidate(const float4* f, const float4* record, float& p_hat) {
 	// kChecked: the branch-free forms (normalize_checked,
@@ -189,50 +191,24 @@ RL_DEV bool binned_candidate(const float4* f, const float4* record, float& p_hat
 	const uint32_t n = __float_as_uint(head.w);
 	const float4 f0 = f[0];
 	float integral[2];
-	bool away[2];
 #pragma unroll 1
 	for (int s = 0; s != 2; ++s) {
 		const mat43 t = load_matrix(f, s);
-		f3 v = local_vertex(t, record, 0);
-		uint32_t mask = v.z > 0.0f ? 1u : 0u;  // bit j: vertex j above the horizon
-		const f3 first = kChecked ? normalize_checked<P>(v, ok) : normalize<P>(v);
-		f3 prev = first;
-		float r = 0.0f;
+		uint32_t mask = 0;  // bit j: vertex j above the horizon
 #pragma unroll 1
-		for (uint32_t j = 1; j != n; ++j) {
-			v = local_vertex(t, record, j);
-			mask |= (v.z > 0.0f ? 1u : 0u) << j;
-			const f3 cur = kChecked ? normalize_checked<P>(v, ok) : normalize<P>(v);
-			r += kChecked ? integrate_edge_checked<P>(prev, cur, ok) : integrate_edge<P>(prev, cur);
-			prev = cur;
-		}
-		r += kChecked ? integrate_edge_checked<P>(prev, first, ok) : integrate_edge<P>(prev, first);
-		if (kChecked && !ok) return false;
-		bool a = false;
-		if (mask == (1u << n) - 1u) {
-			r = fabsf(r);
-		} else if (mask == 0) {
-			r = 0.0f;
-			a = true;
-		} else {
-			r = clipped_integral<P, kChecked>(t, record, n, mask, ok);
-			if (kChecked && !ok) return false;
-			a = r < 0.0f;
-			r = a ? 0.0f : r;
-		}
-		if (s == 0) {
+		for (uint32_t j = 0; j != n; ++j) mask |= (local_vertex(t, record, j).z > 0.0f ? 1u : 0u) << j;
+		const float r = mask == 0 ? -1.0f : clipped_integral<P, kChecked>(t, record, n, mask, ok);
+		if (s == 0)
 			integral[0] = r;
-			away[0] = a;
-		} else {
+		else
 			integral[1] = r;
-			away[1] = a;
-		}
 	}
+	if (kChecked && !ok) return false;
 	const f3 radiance = mk3(head.x, head.y, head.z);
 	f3 result = splat(0.0f);
-	const f3 diffuse = away[0] ? splat(0.0f) : mul(scale(mk3(f0.x, f0.y, f0.z), integral[0]), radiance);
+	const f3 diffuse = integral[0] < 0.0f ? splat(0.0f) : mul(scale(mk3(f0.x, f0.y, f0.z), integral[0]), radiance);
 	result = add(result, diffuse);
-	const f3 ggx = away[1] ? splat(0.0f) : mul(splat(integral[1] * f0.w), radiance);
+	const f3 ggx = integral[1] < 0.0f ? splat(0.0f) : mul(splat(integral[1] * f0.w), radiance);
 	const f3 color = add(result, ggx);
 	if (kChecked) {
 		p_hat = sqrt_checked<P>(dot(color, color), ok);
@@ -587,51 +563,45 @@ RL_DEV void binned_tile(const RisParams& pr, WarpTile<BinnedSuper<P>::value, kPi
 		float* const uphat = phat + window * kUnitSlots;
 		for (int c0 = 0; c0 < super_count; c0 += kChunk) {
 			const int chunk = min(kChunk, super_count - c0);
-			// 1. This lane's candidate lights; bin them by vertex count (six
-			//    10-bit counters).
+			// 1. This lane's candidate lights, counted by vertex count in six
+			//    10-bit fields of a word (field b: b + 3 vertices).
 			int light[kChunk];
-			uint32_t bin[kChunk];
+			uint32_t field[kChunk];  // the field's shift
 			unsigned long long counts = 0;
 #pragma unroll
 			for (int k = 0; k != kChunk; ++k) {
 				light[k] = -1;
-				bin[k] = kBins;
+				field[k] = 0;
 				if (valid && k < chunk) {
 					int idx = drawn_light(get_noise_1(draw));
 					if (pr.candidates)
 						idx = pr.candidates[((size_t) f * np + i) * pr.candidate_count + cs + c0 + k].light;
 					draw = 1664525u * draw + 1013904223u;  // the reservoir's draw
 					light[k] = idx;
-					bin[k] = light_vertex_count(pr.scene, idx) - 3u;
-					counts += 1ull << (10 * bin[k]);
+					field[k] = 10u * (light_vertex_count(pr.scene, idx) - 3u);
+					counts += 1ull << field[k];
 				}
 			}
-			// 2. Counting sort: exclusive scan of the counters across the
-			//    warp, then each bin's start.
-			unsigned long long prefix = counts;
+			// 2. Counting sort: a scan of the fields across the warp gives
+			//    each lane's place in every bin, and one multiplication adds
+			//    the bins' starts (field b of totals * (2^10 + ... + 2^50) is
+			//    the sum of the fields below b; no field reaches 1024).
+			unsigned long long place = counts;
 #pragma unroll
 			for (int d = 1; d < 32; d <<= 1) {
-				const unsigned long long o = __shfl_up_sync(0xffffffffu, prefix, d);
-				if ((int) lane >= d) prefix += o;
+				const unsigned long long o = __shfl_up_sync(0xffffffffu, place, d);
+				if ((int) lane >= d) place += o;
 			}
-			const unsigned long long totals = __shfl_sync(0xffffffffu, prefix, 31);
-			prefix -= counts;
-			uint32_t start[kBins + 1];
-			start[0] = 0;
-#pragma unroll
-			for (int b = 0; b != kBins; ++b) start[b + 1] = start[b] + (uint32_t) ((totals >> (10 * b)) & 1023u);
-			const uint32_t item_count = start[kBins];
+			const unsigned long long totals = __shfl_sync(0xffffffffu, place, 31);
+			const unsigned long long starts = totals * 0x0004010040100400ull;
+			const uint32_t item_count = (uint32_t) ((starts >> 50) & 1023u) + (uint32_t) ((totals >> 50) & 1023u);
+			place += starts - counts;
 #pragma unroll
 			for (int k = 0; k != kChunk; ++k) {
-				if (bin[k] < kBins) {
-					const uint32_t b = bin[k];
-					uint32_t s = 0;
-#pragma unroll
-					for (int q = 0; q != kBins; ++q)
-						if (q == (int) b) s = start[q];
-					const uint32_t pos = s + (uint32_t) ((prefix >> (10 * b)) & 1023u);
-					prefix += 1ull << (10 * b);
-					tile.item[pos] = ((uint32_t) light[k] << 10) | ((c0 + k) * kPixels + lane);
+				if (light[k] >= 0) {
+					tile.item[(uint32_t) (place >> field[k]) & 1023u] =
+					    ((uint32_t) light[k] << 10) | ((c0 + k) * kPixels + lane);
+					place += 1ull << field[k];
 				}
 			}
 			__syncwarp();
