@@ -149,7 +149,9 @@ int grid_for(const risltc_ctx_t* ctx, size_t items) {
 
 // The BVH's device layout for traversal: the root's record {bmin, reference,
 // bmax, 0} (8 floats), then one 16-float record per inner node holding both
-// children's records.  A reference is an inner node's record index (>= 0) or
+// children: the six box planes {bmin.x, bmin.y, bmin.z, bmax.x, bmax.y,
+// bmax.z} with the children's values side by side, then the two references
+// and two unused words.  A reference is an inner node's record index (>= 0) or
 // a leaf, -(1 + (first triangle << 3 | triangle count)) with 1..7 triangles;
 // a larger leaf becomes a small subtree of leaves of at most 7 triangles, all
 // with the leaf's box, so the triangles tested for a ray do not change.  Inner
@@ -191,12 +193,19 @@ std::vector<float> child_pair_nodes(const float* nodes, uint32_t node_count) {
 		stack.push_back({r, true, node, first, count});
 		return r;
 	};
-	auto put = [&](size_t at, uint32_t box_node, int32_t ref) {
-		memcpy(out.data() + at, nodes + 8 * (size_t) box_node, 8 * sizeof(float));
-		memcpy(out.data() + at + 3, &ref, sizeof(ref));
-		out[at + 7] = 0.0f;
+	const int32_t root = reference(0, false, 0, 0);
+	memcpy(out.data(), nodes, 8 * sizeof(float));
+	memcpy(out.data() + 3, &root, sizeof(root));
+	out[7] = 0.0f;
+	// Child `child` (0 or 1) of a record: box_node's box and the reference.
+	auto put = [&](size_t record_at, int child, uint32_t box_node, int32_t ref) {
+		const float* box = nodes + 8 * (size_t) box_node;
+		for (int a = 0; a != 3; ++a) {
+			out[record_at + 2 * a + child] = box[a];
+			out[record_at + 6 + 2 * a + child] = box[4 + a];
+		}
+		memcpy(out.data() + record_at + 12 + child, &ref, sizeof(ref));
 	};
-	put(0, 0, reference(0, false, 0, 0));
 	while (!stack.empty()) {
 		const Pending p = stack.back();
 		stack.pop_back();
@@ -205,14 +214,14 @@ std::vector<float> child_pair_nodes(const float* nodes, uint32_t node_count) {
 			const uint32_t half = p.count / 2;
 			const int32_t r0 = reference(p.node, true, p.first, half);
 			const int32_t r1 = reference(p.node, true, p.first + half, p.count - half);
-			put(at, p.node, r0);
-			put(at + 8, p.node, r1);
+			put(at, 0, p.node, r0);
+			put(at, 1, p.node, r1);
 		} else {
 			const uint32_t left = (uint32_t) word(p.node, 3);
 			const int32_t r0 = reference(left, false, 0, 0);
 			const int32_t r1 = reference(left + 1, false, 0, 0);
-			put(at, left, r0);
-			put(at + 8, left + 1, r1);
+			put(at, 0, left, r0);
+			put(at, 1, left + 1, r1);
 		}
 	}
 	return out;

@@ -247,21 +247,6 @@ RL_DEV mat43x2 load_pairs(const float4* f) {
 	}
 	return m;
 }
-// Two consecutive 16-byte words of a light record in one 32-byte load: the
-// lanes of a warp read 32 unrelated records, and each such load costs L1 32
-// tag lookups whatever its width, which with 16-byte loads bound the kernel
-// (L1 73% busy; with these 58%).  (volatile: the loads stay where they are
-// written, ahead of their use.)
-struct RecordWords {
-	float4 a, b;
-};
-RL_DEV RecordWords load_words(const float4* p) {
-	RecordWords w;
-	asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-	             : "=f"(w.a.x), "=f"(w.a.y), "=f"(w.a.z), "=f"(w.a.w), "=f"(w.b.x), "=f"(w.b.y), "=f"(w.b.z), "=f"(w.b.w)
-	             : "l"(p));
-	return w;
-}
 template <class P> RL_DEV f3x2 mul_point2(const mat43x2& m, float4 q) {
 	const float2 px = pair(q.x), py = pair(q.y), pz = pair(q.z);
 	f3x2 r;

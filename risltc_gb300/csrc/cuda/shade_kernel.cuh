@@ -165,15 +165,50 @@ template <class P> RL_DEV int trace_triangle(const SceneView& s, TraceRay& r) {
 	return hit ? kTraceHit : kTraceContinue;
 }
 
+RL_DEV float max3f(float a, float b, float c) {
+	float d;
+	asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+	return d;
+}
+RL_DEV float min3f(float a, float b, float c) {
+	float d;
+	asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+	return d;
+}
+
 // One inner node: both child boxes, the nearer hit child next and the other
 // pushed.  kTraceContinue, or kTraceMiss with the error recorded when the
-// stack is full.
+// stack is full.  Two 32-byte loads; the two children's slab distances are
+// the lanes of paired subtractions and multiplications, ray_box's operations
+// (trace kernel 4.54 -> 4.40 ms per 4-frame 1080p launch with 1M occluders).
+// Bound by issue (70% of the slots at 11 of 32 active lanes).  Four-child
+// nodes in the same form (128 bytes, nearest child first) took 5.09 ms.
 RL_DEV int trace_node(const SceneView& s, TraceRay& r, int32_t* stack, uint32_t* error) {
 	const float4* n = s.pairs + 2 + 4 * (size_t) r.node;
-	const float4 lo0 = __ldg(n), hi0 = __ldg(n + 1), lo1 = __ldg(n + 2), hi1 = __ldg(n + 3);
+	const RecordWords p = load_words(n), q = load_words(n + 2);
+	const int32_t ref0 = __float_as_int(q.b.x), ref1 = __float_as_int(q.b.y);
 	float e0, e1;
-	const bool h0 = ray_box(r, lo0, hi0, &e0), h1 = ray_box(r, lo1, hi1, &e1);
-	const int32_t ref0 = __float_as_int(lo0.w), ref1 = __float_as_int(lo1.w);
+	bool h0, h1;
+	if (r.minmax) {
+		const float2 lo[3] = {make_float2(p.a.x, p.a.y), make_float2(p.a.z, p.a.w), make_float2(p.b.x, p.b.y)};
+		const float2 hi[3] = {make_float2(p.b.z, p.b.w), make_float2(q.a.x, q.a.y), make_float2(q.a.z, q.a.w)};
+		const float o[3] = {r.o.x, r.o.y, r.o.z};
+		float2 near[3], far[3];
+#pragma unroll
+		for (int ax = 0; ax != 3; ++ax) {
+			const float2 no = make_float2(-o[ax], -o[ax]), inv = make_float2(r.inv[ax], r.inv[ax]);
+			const float2 t0 = __fmul2_rn(__fadd2_rn(lo[ax], no), inv), t1 = __fmul2_rn(__fadd2_rn(hi[ax], no), inv);
+			near[ax] = make_float2(fminf(t0.x, t1.x), fminf(t0.y, t1.y));
+			far[ax] = make_float2(fmaxf(t0.x, t1.x), fmaxf(t0.y, t1.y));
+		}
+		e0 = fmaxf(r.t_min, max3f(near[0].x, near[1].x, near[2].x));
+		e1 = fmaxf(r.t_min, max3f(near[0].y, near[1].y, near[2].y));
+		h0 = e0 <= fminf(r.t_max, min3f(far[0].x, far[1].x, far[2].x));
+		h1 = e1 <= fminf(r.t_max, min3f(far[0].y, far[1].y, far[2].y));
+	} else {
+		h0 = ray_box(r, make_float4(p.a.x, p.a.z, p.b.x, 0.0f), make_float4(p.b.z, q.a.x, q.a.z, 0.0f), &e0);
+		h1 = ray_box(r, make_float4(p.a.y, p.a.w, p.b.y, 0.0f), make_float4(p.b.w, q.a.y, q.a.w, 0.0f), &e1);
+	}
 	if (h0 && h1) {
 		if (r.sp >= kBvhStack) {
 			atomicOr(error, kErrorTraversalLimit);
