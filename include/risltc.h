@@ -486,7 +486,11 @@ EXTERN_C void risltc_scene_destroy(risltc_scene_t* scene);
  * on its first launch.  After one call, later calls that need no more
  * scratch (no more pixels, frames, lights, candidates or clusters) make no
  * allocation and no configuration call; a default-configuration call made
- * after one such call can be captured into a CUDA graph. */
+ * after one such call can be captured into a CUDA graph.  Calls with one
+ * uniformly drawn light, projected solid angle samples and shadow rays grow
+ * scratch of their own (210 bytes per pixel and frame); where it cannot be
+ * had, beyond 2^26 pixel-frames and while the stream is being captured they
+ * run without it, with the same results, more slowly. */
 EXTERN_C int risltc_ctx_reserve(risltc_ctx_t* ctx, uint32_t width, uint32_t height, uint32_t frame_count);
 
 /* Shades frame_count consecutive frames of the G-buffer (device pointers).
@@ -619,8 +623,9 @@ EXTERN_C int risltc_ctx_profile(risltc_ctx_t* ctx, int enable, float* phase_ms, 
 EXTERN_C int risltc_ctx_launch_count(const risltc_ctx_t* ctx, uint64_t* launches);
 
 /* The shadow rays that the last risltc_shade call on the context traced
- * through its ray queue (the default configuration with shadows on: rays
- * grouped by light, then traced by the persistent kernel); 0 when that call
+ * through its ray queue (the default configuration with shadows on, and one
+ * uniformly drawn light with projected solid angle samples: rays grouped by
+ * light, then traced by the persistent kernel); 0 when that call
  * traced none that way.  Waits for the context's stream.  No counterpart in
  * the reference, whose ray queries run inside the fragment shader; the
  * shadow-ray rate of the benchmark (rays per second) comes from it. */

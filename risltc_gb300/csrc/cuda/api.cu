@@ -67,6 +67,10 @@ struct risltc_ctx_s {
 	size_t wavefront_capacity;
 	size_t light_capacity;
 	size_t queue_capacity;  // ray queues (2 words each) in d_ray_count
+	// The scratch of uniform-light calls with queued shadow rays
+	// (uniform_scratch).
+	void* d_uniform;
+	size_t uniform_pixel_frames, uniform_lights;
 	// risltc_shade_batch: items run on these streams, forked from and joined
 	// back to the context's stream.
 	cudaStream_t batch_streams[RISLTC_BATCH_STREAMS];
@@ -82,8 +86,9 @@ struct risltc_ctx_s {
 	cudaEvent_t events[64][RISLTC_PROFILE_PHASES + 1];
 	// Kernels of this library launched through the context (risltc_ctx_launch_count).
 	uint64_t kernel_launches;
-	// Whether the last risltc_shade call queued its shadow rays (queue 0 of
-	// d_ray_count then holds their number: risltc_ctx_ray_count).
+	// Where the last risltc_shade call queued its shadow rays, whose number
+	// risltc_ctx_ray_count reports: 0 nowhere, 1 queue 0 of d_ray_count, 2 the
+	// queue of d_uniform.
 	int rays_queued;
 	int events_created;
 };
@@ -301,6 +306,7 @@ EXTERN_C void risltc_ctx_destroy(risltc_ctx_t* ctx) {
 	cudaFree(ctx->d_primitive);
 	cudaFree(ctx->d_rgb);
 	cudaFreeHost(ctx->h_pinned_rgb);
+	cudaFree(ctx->d_uniform);
 	cudaFree(ctx->d_records);
 	cudaFree(ctx->d_phat);
 	cudaFree(ctx->d_candidates);
@@ -586,6 +592,18 @@ bool uses_ray_queue(const risltc_scene_t* scene, const risltc_settings_t* s, siz
 	       pixel_frames < (1ull << 31);
 }
 
+// The reference's ground-truth estimator (one uniformly drawn light, projected
+// solid angle samples) with its shadow rays queued as above, up to 2^26
+// pixel-frames (13 GB of scratch); larger calls, and calls without scratch,
+// run shade_kernel, which gives the same results with inline rays.
+bool may_queue_uniform(const risltc_scene_t* scene, const risltc_settings_t* s, size_t pixel_frames) {
+	return s->light_sampling == light_uniform && s->sample_count_light == 1 && s->sample_count == 1 && s->shadows &&
+	       scene->view.triangle_count && pixel_frames <= (1ull << 26) &&
+	       (s->polygon_sampling_technique == sample_polygon_ltc_cp ||
+	        s->polygon_sampling_technique == sample_polygon_projected_solid_angle ||
+	        s->polygon_sampling_technique == sample_polygon_projected_solid_angle_biased);
+}
+
 // One call's share of the context's scratch.
 struct Scratch {
 	risltc::ReservoirRecord* records;
@@ -598,6 +616,8 @@ struct Scratch {
 	uint8_t* hits;
 	uint32_t* ray_count;
 	uint32_t* light_rays;
+	uint32_t* sample_cursor;  // null: the word after the candidate kernel's tile cursor
+	bool queue_uniform;       // the scratch is uniform_scratch's: may_queue_uniform's route
 };
 
 bool uses_proposal(const risltc_settings_t* s) { return s->proposal != risltc_proposal_uniform; }
@@ -803,19 +823,21 @@ risltc::RisParams ris_params(const risltc_ctx_t* ctx, const Scratch& sc, const r
 	r.primitive = gbuffer->primitive;
 	r.width = gbuffer->width;
 	r.height = gbuffer->height;
+	r.technique = (int) settings->polygon_sampling_technique;
 	r.candidate_count = (int) settings->candidate_count;
 	r.mis_heuristic = (int) settings->mis_heuristic;
 	r.sample_count = (int) settings->sample_count;
 	r.mis_visibility_estimate = settings->mis_visibility_estimate;
 	r.fast_atan = (int) settings->fast_atan;
 	r.shadows = (int) settings->shadows;
+	r.uniform_light = settings->light_sampling == light_uniform ? 1 : 0;
 	r.noise_seed = noise_seed;
 	r.animate = animate;
 	r.frame_count = frame_count;
 	r.records = sc.records;
 	r.p_hat_scratch = sc.p_hat;
 	r.tile_cursor = sc.p_hat ? reinterpret_cast<uint32_t*>(sc.p_hat + phat_slot_floats(ctx)) : nullptr;
-	r.sample_cursor = r.tile_cursor ? r.tile_cursor + 1 : nullptr;
+	r.sample_cursor = sc.sample_cursor ? sc.sample_cursor : (r.tile_cursor ? r.tile_cursor + 1 : nullptr);
 	if (ray_queue) {
 		r.samples = sc.samples;
 		r.staged = sc.staged;
@@ -921,6 +943,13 @@ int shade_one(risltc_ctx_t* ctx, cudaStream_t stream, const Scratch& sc, const r
 		if (e == cudaSuccess && train)
 			e = launch_training(ctx, stream, scene, gbuffer, sc.candidates, r.candidate_count, r.train_stride,
 			                    r.train_phase, r.train_shaded, r.records);
+	} else if (sc.queue_uniform) {
+		const risltc::RisParams r = ris_params(ctx, sc, scene, gbuffer, settings, noise_seed, animate, frame_count,
+		                                       out_rgb, accum, reservoirs, true);
+		e = risltc::launch_ris(r, stream, grid_for(ctx, pixels), grid_for(ctx, 2 * pixels * frame_count), events,
+		                       false, 0, 0);
+		// Sample, bucket scan, scatter, trace and resolve kernels.
+		if (e == cudaSuccess) ctx->kernel_launches += 5;
 	} else {
 		e = risltc::launch_shade(p, stream, grid_for(ctx, pixels), events, fast);
 		if (e == cudaSuccess) ctx->kernel_launches += 1;
@@ -942,6 +971,51 @@ int check_shade_call(const risltc_ctx_t* ctx, const risltc_scene_t* scene, const
 	return RISLTC_OK;
 }
 
+// The scratch of may_queue_uniform's route into sc, an allocation of its own:
+// such a call must not move the scratch that a captured frame of the default
+// configuration refers to.  False where the route is not to be taken: no
+// memory, or the stream is being captured into a graph (which then needs no
+// scratch that a later, larger call would move).
+bool uniform_scratch(risltc_ctx_t* ctx, size_t pixel_frames, size_t light_count, Scratch& sc) {
+	cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+	if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+		cudaGetLastError();
+		return false;
+	}
+	if (pixel_frames > ctx->uniform_pixel_frames || light_count > ctx->uniform_lights) {
+		const size_t pf = std::max(pixel_frames, ctx->uniform_pixel_frames);
+		const size_t lights = std::max(light_count, ctx->uniform_lights);
+		cudaStreamSynchronize(ctx->stream);
+		cudaFree(ctx->d_uniform);
+		ctx->d_uniform = nullptr;
+		ctx->uniform_pixel_frames = ctx->uniform_lights = 0;
+		const size_t bytes = pf * (sizeof(risltc::SampleRecord) + 4 * sizeof(risltc::ShadowRay) +
+		                           sizeof(risltc::ReservoirRecord) + 2) + 256 +
+		                     lights * risltc::kLightCounterStride * sizeof(uint32_t);
+		if (cudaMalloc(&ctx->d_uniform, bytes) != cudaSuccess) {
+			cudaGetLastError();
+			ctx->d_uniform = nullptr;
+			return false;
+		}
+		ctx->uniform_pixel_frames = pf;
+		ctx->uniform_lights = lights;
+	}
+	// 256 bytes of counters (queue length, fetch cursor, sample cursor), the
+	// per-light counters, then the per-pixel-frame arrays by falling alignment.
+	const size_t pf = ctx->uniform_pixel_frames;
+	uint32_t* const counters = static_cast<uint32_t*>(ctx->d_uniform);
+	sc.ray_count = counters;
+	sc.sample_cursor = counters + 2;
+	sc.light_rays = counters + 64;
+	sc.samples = reinterpret_cast<risltc::SampleRecord*>(sc.light_rays + ctx->uniform_lights * risltc::kLightCounterStride);
+	sc.staged = reinterpret_cast<risltc::ShadowRay*>(sc.samples + pf);
+	sc.rays = sc.staged + 2 * pf;
+	sc.records = reinterpret_cast<risltc::ReservoirRecord*>(sc.rays + 2 * pf);
+	sc.hits = reinterpret_cast<uint8_t*>(sc.records + pf);
+	sc.queue_uniform = true;
+	return true;
+}
+
 // risltc_shade after its checks: grows the scratch and launches on the
 // context's stream with the given events (may be null).
 int shade_on_context(risltc_ctx_t* ctx, const risltc_scene_t* scene, const risltc_gbuffer_t* gbuffer,
@@ -961,11 +1035,14 @@ int shade_on_context(risltc_ctx_t* ctx, const risltc_scene_t* scene, const rislt
 		    (st = reserve_wavefront(ctx, pixel_frames, scene->view.light_count)))
 			return st;
 	}
-	const Scratch sc{ctx->d_records, ctx->d_phat, ctx->d_candidates, ctx->d_logits, ctx->d_samples, ctx->d_staged,
-	                 ctx->d_rays, ctx->d_hits, ctx->d_ray_count, ctx->d_light_rays};
+	Scratch sc{ctx->d_records, ctx->d_phat, ctx->d_candidates, ctx->d_logits, ctx->d_samples, ctx->d_staged,
+	           ctx->d_rays, ctx->d_hits, ctx->d_ray_count, ctx->d_light_rays};
+	if (may_queue_uniform(scene, settings, pixel_frames))
+		uniform_scratch(ctx, pixel_frames, scene->view.light_count, sc);
 	st = shade_one(ctx, ctx->stream, sc, scene, gbuffer, settings, noise_seed, animate, frame_count, out_rgb, accum,
 	               reservoirs, events);
-	ctx->rays_queued = st == RISLTC_OK && uses_ris_pipeline(settings) && uses_ray_queue(scene, settings, pixel_frames);
+	ctx->rays_queued =
+	    st != RISLTC_OK ? 0 : (sc.queue_uniform ? 2 : (uses_ray_queue(scene, settings, pixel_frames) ? 1 : 0));
 	return st;
 }
 
@@ -1356,9 +1433,10 @@ EXTERN_C int risltc_trace_shadow(risltc_ctx_t* ctx, const risltc_scene_t* scene,
 EXTERN_C int risltc_ctx_ray_count(risltc_ctx_t* ctx, uint32_t* rays) {
 	if (!ctx || !rays) return RISLTC_ERROR_INVALID_ARGUMENT;
 	*rays = 0;
-	if (!ctx->rays_queued || !ctx->d_ray_count) return RISLTC_OK;
+	const void* queue = ctx->rays_queued == 2 ? ctx->d_uniform : ctx->d_ray_count;
+	if (!ctx->rays_queued || !queue) return RISLTC_OK;
 	cudaSetDevice(ctx->device);
-	cudaError_t e = cudaMemcpyAsync(rays, ctx->d_ray_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream);
+	cudaError_t e = cudaMemcpyAsync(rays, queue, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream);
 	if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
 	return cuda_status(e);
 }

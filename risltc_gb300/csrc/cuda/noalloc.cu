@@ -89,6 +89,7 @@ EXTERN_C int risltc_shade_noalloc(const risltc_scene_t* scene, const risltc_gbuf
 	r.primitive = gbuffer->primitive;
 	r.width = gbuffer->width;
 	r.height = gbuffer->height;
+	r.technique = (int) settings->polygon_sampling_technique;
 	r.candidate_count = (int) settings->candidate_count;
 	r.mis_heuristic = (int) settings->mis_heuristic;
 	r.sample_count = (int) settings->sample_count;

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kSampleThreads, RISLTC_SAMPLE_MIN_BLOCKS) ris_
 	const uint32_t total = b.pixel_begin[b.count];
 	for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < total; u += gridDim.x * blockDim.x) {
 		const uint32_t k = batch_item(b.pixel_begin, b.count, u);
-		sample_pixel<P>(b.item[k], u - b.pixel_begin[k], poly[threadIdx.x]);
+		sample_pixel<P, false>(b.item[k], u - b.pixel_begin[k], poly[threadIdx.x]);
 	}
 }
 

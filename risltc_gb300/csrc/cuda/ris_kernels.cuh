@@ -38,12 +38,16 @@ struct RisParams {
 	const float* gbuffer;
 	const uint32_t* primitive;
 	uint32_t width, height;
+	int technique;                 // sample_polygon_technique_t of the estimator
 	int candidate_count;
 	int mis_heuristic;
 	int sample_count;
 	float mis_visibility_estimate;
 	int fast_atan;
 	int shadows;
+	// Non-zero: no candidates; the sample kernel draws each pixel-frame's light
+	// uniformly (light_uniform) and writes its record.
+	int uniform_light;
 	uint32_t noise_seed;
 	uint32_t animate;
 	uint32_t frame_count;
@@ -252,7 +256,7 @@ template <class P> __global__ void __launch_bounds__(kShadeThreads) ris_shade_ke
 	const uint32_t np = pr.width * pr.height;
 	ShadeParams sp;  // the fields psa_mis_shade and polygon_visibility read
 	sp.scene = pr.scene;
-	sp.technique = sample_polygon_ltc_cp;
+	sp.technique = pr.technique;
 	sp.mis_heuristic = pr.mis_heuristic;
 	sp.sample_count = pr.sample_count;
 	sp.mis_visibility_estimate = pr.mis_visibility_estimate;
@@ -347,7 +351,7 @@ cudaError_t launch_shadow_trace(const RisParams& p, cudaStream_t stream, int gri
 cudaError_t launch_ris_resolve(const RisParams& p, cudaStream_t stream, int grid);
 
 // The candidate kernel (fast or exact numerics, tile shape `tile`, at most
-// grid_cap blocks), then the shading phase (always exact): ris_shade_kernel,
+// grid_cap blocks; none with p.uniform_light), then the shading phase (always exact): ris_shade_kernel,
 // or with p.samples set the sample kernel, the shadow rays' grouping by light
 // and trace, and the resolve kernel.  events (may be null) holds five events,
 // recorded before, between and after the phases (the last three together for
@@ -355,8 +359,9 @@ cudaError_t launch_ris_resolve(const RisParams& p, cudaStream_t stream, int grid
 inline cudaError_t launch_ris(const RisParams& p, cudaStream_t stream, int grid, int trace_grid, cudaEvent_t* events,
                               bool fast, int tile, int grid_cap) {
 	if (events) cudaEventRecord(events[0], stream);
-	cudaError_t e = fast ? launch_candidates_fast(p, stream, grid_cap, tile)
-	                     : launch_candidates_exact(p, stream, grid_cap, tile);
+	cudaError_t e = cudaSuccess;
+	if (!p.uniform_light)
+		e = fast ? launch_candidates_fast(p, stream, grid_cap, tile) : launch_candidates_exact(p, stream, grid_cap, tile);
 	if (e != cudaSuccess) return e;
 	if (events) cudaEventRecord(events[1], stream);
 	if (p.samples) {

@@ -17,7 +17,10 @@
 // The contributions are the same operations on the same values, added in
 // the same order, so the pixels are bit-identical to ris_shade_kernel's.
 // Used for one sample per technique (SAMPLE_COUNT == 1, the reference's
-// default) with shadows on.
+// default) with shadows on: after the candidate kernel, or (uniform_light)
+// with one uniformly drawn light per pixel-frame, the reference's ground-truth
+// estimator, for which shade_kernel with its inline rays took 17.6 ms per
+// 4-frame 640x360 call with 5,000 occluders against 1.20 here.
 // Restates upstream risltc routines (GPLv3): see NOTICE.
 #pragma once
 #include "ris_kernels.cuh"
@@ -61,14 +64,14 @@ RL_DEV void store_contributions(SampleRecord* dst, int j, f3 c0, f3 c1) {
 	}
 }
 
-// evaluate_polygonal_light_shading_peters for SAMPLE_COUNT == 1 up to the
-// visibility test.  Writes both techniques' contributions into *dst (zero
+// evaluate_polygonal_light_shading_peters or, with peters false, the PSA
+// branch of evaluate_polygonal_light_shading, for SAMPLE_COUNT == 1 up to the visibility test.  Writes both techniques' contributions into *dst (zero
 // where a technique has none) and each traced technique's shadow ray into
 // staged[j] as soon as they are known, and returns the techniques' modes.
 // l is the light whose device record is `record`; poly is the thread's
 // polygon buffer.
 template <class P>
-RL_DEV uint32_t psa_mis_emit(const ShadeParams& pr, const ShadingData& sd, Ltc ltc, const Light& l,
+RL_DEV uint32_t psa_mis_emit(const ShadeParams& pr, bool peters, const ShadingData& sd, Ltc ltc, const Light& l,
                              const float4* record, uint32_t& seed, SampleRecord* dst, ShadowRay* staged,
                              PsaPolygon& poly) {
 	const bool fa = pr.fast_atan != 0;
@@ -143,7 +146,7 @@ RL_DEV uint32_t psa_mis_emit(const ShadeParams& pr, const ShadingData& sd, Ltc l
 			f3 integrand = scale(visibility ? rb_lit : splat(0.0f), dir.z);
 			f3 r;
 			if (j == 0 && psa[1] <= 0.0f)
-				r = visibility ? scale(integrand, P::rcp(diffuse_density)) : splat(0.0f);
+				r = visibility || !peters ? scale(integrand, P::rcp(diffuse_density)) : splat(0.0f);
 			else
 				r = mis_estimate<P>(pr.mis_heuristic, integrand, own_weight, own_density, other_weight, other_density,
 				                    pr.mis_visibility_estimate);
@@ -183,11 +186,14 @@ RL_DEV void store_sample(SampleRecord* dst, const f3 (&c)[2][2], float W, uint32
 constexpr int kSampleThreads = 128;
 // The sample phase of pixel i (all frames of the call); i may be past the
 // frame (the thread then does nothing).
-template <class P> RL_DEV void sample_pixel(const RisParams& pr, uint32_t i, PsaPolygon& poly) {
+// kUniform: RisParams::uniform_light (a variant of its own: its few
+// instructions cost the other 2%).
+template <class P, bool kUniform> RL_DEV void sample_pixel(const RisParams& pr, uint32_t i, PsaPolygon& poly) {
 	const uint32_t np = pr.width * pr.height;
 	ShadeParams sp;  // the fields psa_prepare_both and psa_mis_emit read
 	sp.scene = pr.scene;
-	sp.technique = sample_polygon_ltc_cp;
+	sp.technique = kUniform ? pr.technique : (int) sample_polygon_ltc_cp;
+	const bool peters = !kUniform || pr.technique == sample_polygon_ltc_cp;
 	sp.mis_heuristic = pr.mis_heuristic;
 	sp.sample_count = 1;
 	sp.mis_visibility_estimate = pr.mis_visibility_estimate;
@@ -216,17 +222,28 @@ template <class P> RL_DEV void sample_pixel(const RisParams& pr, uint32_t i, Psa
 			uint32_t modes = 0;
 			int light = -1;
 			if (active) {
-				const ReservoirRecord r = pr.records[pf];
+				ReservoirRecord r;
+				if (kUniform) {
+					const int n = pr.scene.light_count;
+					const uint32_t rn_x = pr.animate ? wang_random_number((pr.noise_seed + f) * 4u) : 0u;
+					uint32_t seed = get_noise_accessor(i % pr.width, i / pr.width, pr.width, rn_x);
+					const int idx = (int) (get_noise_1(seed) * (float) n);
+					r = ReservoirRecord{idx > n - 1 ? n - 1 : idx, 0.0f, 0.0f, seed};
+					pr.records[pf] = r;
+				} else {
+					r = pr.records[pf];
+				}
 				light = r.light_index;
 				if (r.light_index >= 0) {
 					Light l;
 					load_light(pr.scene, r.light_index, l);
 					uint32_t seed = r.seed;
 					// Contributions and staged rays go to memory inside.
-					modes = psa_mis_emit<P>(sp, sd, ltc, l, light_record(pr.scene, r.light_index), seed,
+					modes = psa_mis_emit<P>(sp, peters, sd, ltc, l, light_record(pr.scene, r.light_index), seed,
 					                        pr.samples + pf, pr.staged + 2 * pf, poly);
 					float W = P::div(r.w_sum, (float) pr.candidate_count * r.p_hat);
 					if (r.p_hat == 0.0f) W = 0.0f;
+					if (kUniform) W = (float) pr.scene.light_count;
 					*reinterpret_cast<float2*>(reinterpret_cast<float*>(pr.samples + pf) + 12) =
 					    make_float2(W, __uint_as_float(modes));
 				} else {
@@ -242,13 +259,13 @@ template <class P> RL_DEV void sample_pixel(const RisParams& pr, uint32_t i, Psa
 }
 
 // Each warp takes 32 consecutive pixels at a time from the launch's cursor.
-template <class P>
+template <class P, bool kUniform>
 __global__ void __launch_bounds__(kSampleThreads, RISLTC_SAMPLE_MIN_BLOCKS) ris_sample_kernel(const __grid_constant__ RisParams pr) {
 	__shared__ PsaPolygon poly[kSampleThreads];
 	const uint32_t np = pr.width * pr.height;
 	const uint32_t chunks = (np + 31) / 32;
 	for (uint32_t c = next_warp_tile(pr.sample_cursor); c < chunks; c = next_warp_tile(pr.sample_cursor))
-		sample_pixel<P>(pr, c * 32 + threadIdx.x % 32, poly[threadIdx.x]);
+		sample_pixel<P, kUniform>(pr, c * 32 + threadIdx.x % 32, poly[threadIdx.x]);
 }
 
 // Exclusive prefix sum of the per-light ray counts, in place (each becomes

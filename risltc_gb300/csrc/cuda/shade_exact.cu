@@ -34,7 +34,10 @@ cudaError_t launch_proposal(const ProposalParams& p, cudaStream_t stream, int gr
 	return cudaGetLastError();
 }
 cudaError_t launch_ris_sample(const RisParams& p, cudaStream_t stream, int grid) {
-	ris_sample_kernel<ExactNumerics><<<grid, kSampleThreads, 0, stream>>>(p);
+	if (p.uniform_light)
+		ris_sample_kernel<ExactNumerics, true><<<grid, kSampleThreads, 0, stream>>>(p);
+	else
+		ris_sample_kernel<ExactNumerics, false><<<grid, kSampleThreads, 0, stream>>>(p);
 	return cudaGetLastError();
 }
 cudaError_t launch_shadow_sort(const RisParams& p, cudaStream_t stream, int grid) {
