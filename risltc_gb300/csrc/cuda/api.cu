@@ -726,9 +726,10 @@ cudaError_t launch_training(risltc_ctx_t* ctx, cudaStream_t stream, const risltc
 	return e;
 }
 
-// The model's logits for every pixel of the G-buffer into logits.
+// The model's logits for every pixel of the G-buffer into logits (BF16), or
+// into logits_f32 where that is not null.
 cudaError_t launch_logits(risltc_ctx_t* ctx, cudaStream_t stream, const risltc_model_t* m,
-                          const risltc_gbuffer_t* gbuffer, __nv_bfloat16* logits) {
+                          const risltc_gbuffer_t* gbuffer, __nv_bfloat16* logits, float* logits_f32 = nullptr) {
 	risltc::MlpParams q;
 	memset(&q, 0, sizeof(q));
 	q.gbuffer = gbuffer->planes;
@@ -741,14 +742,18 @@ cudaError_t launch_logits(risltc_ctx_t* ctx, cudaStream_t stream, const risltc_m
 	for (int a = 0; a != 3; ++a) q.center[a] = m->center[a];
 	q.inv_half_extent = m->inv_half_extent;
 	q.logits = logits;
+	q.logits_f32 = logits_f32;
 	q.error = ctx->d_error;
 	q.skip_issue = (ctx->inject & RISLTC_FAULT_TENSOR_WAIT) ? 1u : 0u;
 	ctx->inject &= ~(uint32_t) RISLTC_FAULT_TENSOR_WAIT;
 	static std::atomic<uint64_t> configured{0};
 	const uint64_t bit = 1ull << (ctx->device & 63);
 	if (!(configured.load() & bit)) {
-		cudaError_t e = cudaFuncSetAttribute(risltc::mlp_logits_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                                     (int) risltc::mlp_tc_smem_bytes(risltc::kMaxClusters));
+		const int smem = (int) risltc::mlp_tc_smem_bytes(risltc::kMaxClusters);
+		cudaError_t e = cudaFuncSetAttribute(risltc::mlp_logits_tc_kernel<false>,
+		                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+		if (e == cudaSuccess)
+			e = cudaFuncSetAttribute(risltc::mlp_logits_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 		if (e != cudaSuccess) return e;
 		configured.fetch_or(bit);
 	}
@@ -756,7 +761,11 @@ cudaError_t launch_logits(risltc_ctx_t* ctx, cudaStream_t stream, const risltc_m
 	// tensor-memory allocations of an SM never wait for each other.
 	const size_t tiles = ((size_t) gbuffer->width * gbuffer->height + risltc::kTcRows - 1) / risltc::kTcRows;
 	const int grid = (int) std::min<size_t>(tiles, (size_t) ctx->sm_count * 2);
-	risltc::mlp_logits_tc_kernel<<<grid, risltc::kTcThreads, risltc::mlp_tc_smem_bytes(m->cluster_count), stream>>>(q);
+	const size_t smem = risltc::mlp_tc_smem_bytes(m->cluster_count);
+	if (logits_f32)
+		risltc::mlp_logits_tc_kernel<true><<<grid, risltc::kTcThreads, smem, stream>>>(q);
+	else
+		risltc::mlp_logits_tc_kernel<false><<<grid, risltc::kTcThreads, smem, stream>>>(q);
 	const cudaError_t e = cudaGetLastError();
 	if (e == cudaSuccess) ctx->kernel_launches += 1;
 	return e;
@@ -1634,15 +1643,8 @@ EXTERN_C int risltc_model_logits(risltc_ctx_t* ctx, const risltc_model_t* model,
 	if (!ctx || !model || !gbuffer || !gbuffer->planes || !logits || model->ctx != ctx || gbuffer->width == 0 ||
 	    gbuffer->height == 0)
 		return RISLTC_ERROR_INVALID_ARGUMENT;
-	const size_t count = (size_t) gbuffer->width * gbuffer->height * model->cluster_count;
-	int st = reserve_logits(ctx, count);
-	if (st) return st;
-	cudaError_t e = launch_logits(ctx, ctx->stream, model, gbuffer, ctx->d_logits);
-	if (e == cudaSuccess) {
-		risltc::bf16_to_f32_kernel<<<256, 256, 0, ctx->stream>>>(ctx->d_logits, logits, count);
-		e = cudaGetLastError();
-	}
-	return cuda_status(e);
+	cudaSetDevice(ctx->device);
+	return cuda_status(launch_logits(ctx, ctx->stream, model, gbuffer, nullptr, logits));
 }
 
 EXTERN_C int risltc_model_set_training(risltc_model_t* model, int enable, float learning_rate, uint32_t pixel_stride) {

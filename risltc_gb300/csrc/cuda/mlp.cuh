@@ -72,6 +72,7 @@ struct MlpParams {
 	int k_count;                   // clusters, a multiple of 8
 	float center[3], inv_half_extent;
 	__nv_bfloat16* logits;         // [pixel][k_count]
+	float* logits_f32;             // the same as FP32 instead, where the caller wants that
 	uint32_t* error;               // the context's error word
 	uint32_t skip_issue;           // fault injection: issue no tensor-core products
 };
@@ -122,17 +123,6 @@ static __global__ void mlp_convert_kernel(const float* params, __nv_bfloat16* we
 		if (slot >= 0) weights[slot] = __float2bfloat16_rn(mlp_padding_weight(j) ? 0.0f : params[j]);
 	}
 }
-
-// BF16 logits to FP32 (for inspection).
-static __global__ void bf16_to_f32_kernel(const __nv_bfloat16* in, float* out, size_t count) {
-	for (size_t j = blockIdx.x * (size_t) blockDim.x + threadIdx.x; j < count; j += (size_t) gridDim.x * blockDim.x)
-		out[j] = __bfloat162float(in[j]);
-}
-
-}  // namespace risltc
-
-namespace risltc {
-
 // ----------------------------------------------------------------- training --
 // Online training of the proposal on the RIS candidates of a frame: for each
 // training pixel the candidates' weights w = p_hat / p (the LTC-CP target

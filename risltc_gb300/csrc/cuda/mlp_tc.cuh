@@ -11,7 +11,9 @@
 // columns 0..63, D3 in 64..191), and each warp moves its 32 rows (pixels)
 // from tensor memory to registers for the epilogues: bias, ReLU and BF16
 // rounding back into shared memory for the next product, or bias and BF16
-// rounding of the logits to global memory.  Every wait on the tensor cores
+// rounding of the logits to global memory (as BF16 for the proposal kernel, or
+// widened to FP32 for a caller of risltc_model_logits: a separate pass over
+// 0.8 GB took 0.9 of that call's 1.1 ms at 960x540 with 256 clusters).  Every wait on the tensor cores
 // is bounded; on a timeout the kernel records kErrorTensorWait, waits once
 // more (bounded) for its products in flight, frees its tensor memory and
 // returns.
@@ -149,7 +151,15 @@ static_assert(kMlpInputs * kTcRows * 4 <= kTcRows * kMlpHidden * 2, "inputs fit 
 // G-buffer plane of MLP input k (position, normal, outgoing, roughness).
 RL_DEV int mlp_input_plane(int k) { return k < 9 ? k : 16; }
 
-static __global__ void __launch_bounds__(kTcThreads, 1) mlp_logits_tc_kernel(MlpParams pr) {
+// Eight FP32 values to 32-byte aligned memory in one store (a whole sector).
+RL_DEV void store8(float* dst, const float (&v)[8]) {
+	asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+	             "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+	             : "memory");
+}
+
+// kF32: the logits go to pr.logits_f32.
+template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp_logits_tc_kernel(MlpParams pr) {
 	extern __shared__ __align__(1024) unsigned char tc_smem[];
 	const int k_count = pr.k_count;
 	const MlpLayout lay = mlp_layout(k_count);
@@ -316,7 +326,10 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_logits_tc_kernel(Mlp
 				tc_load32(d3 + lane_base + (uint32_t) c, v);
 				tc_wait_load();
 				if (row < np) {
-					__nv_bfloat16* dst = pr.logits + (size_t) row * k_count + c0 + c;
+					const size_t at = (size_t) row * k_count + c0 + c;
+					// Rows are multiples of 32 bytes; the caller's buffer may
+					// have any alignment.
+					const bool aligned = (reinterpret_cast<uintptr_t>(pr.logits_f32) & 31) == 0;
 #pragma unroll
 					for (int q = 0; q != 4; ++q) {
 						const int j0 = c0 + c + 8 * q;
@@ -329,7 +342,23 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_logits_tc_kernel(Mlp
 							o[h] = pack_bf16x2(__uint_as_float(v[j]) + b3[c0 + c + j],
 							                   __uint_as_float(v[j + 1]) + b3[c0 + c + j + 1]);
 						}
-						*reinterpret_cast<uint4*>(dst + 8 * q) = out;
+						if (!kF32) {
+							*reinterpret_cast<uint4*>(pr.logits + at + 8 * q) = out;
+						} else {
+							float wide[8];
+#pragma unroll
+							for (int h = 0; h != 4; ++h) {
+								wide[2 * h] = __uint_as_float(o[h] << 16);
+								wide[2 * h + 1] = __uint_as_float(o[h] & 0xffff0000u);
+							}
+							float* const dst = pr.logits_f32 + at + 8 * q;
+							if (aligned) {
+								store8(dst, wide);
+							} else {
+#pragma unroll
+								for (int h = 0; h != 8; ++h) dst[h] = wide[h];
+							}
+						}
 					}
 				}
 			}
