@@ -23,14 +23,14 @@ namespace risltc {
 cudaError_t launch_proposal(const ProposalParams& p, cudaStream_t stream, int grid);
 cudaError_t launch_shade(const ShadeParams& p, cudaStream_t stream, int grid, cudaEvent_t* events, bool fast);
 cudaError_t launch_trace_exact(const SceneView& s, const float4* rays, uint32_t count, uint32_t* hits, uint32_t* error,
-                               cudaStream_t stream, int grid);
+                               uint32_t* cursor, cudaStream_t stream, int grid, int resident);
 }  // namespace risltc
 
 struct risltc_ctx_s {
 	int device;
 	cudaStream_t stream;
 	int sm_count;
-	uint32_t* d_error;
+	uint32_t* d_error;  // the error word, then the fetch cursor of risltc_trace_shadow
 	// Staging for risltc_shade_host, grown on demand.
 	float* d_gbuffer;
 	uint32_t* d_primitive;
@@ -287,8 +287,8 @@ EXTERN_C int risltc_ctx_create(risltc_ctx_t** out, int device, void* stream) {
 	ctx->device = device;
 	ctx->stream = (cudaStream_t) stream;
 	cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device);
-	if ((e = cudaMalloc(&ctx->d_error, sizeof(uint32_t))) != cudaSuccess ||
-	    (e = cudaMemsetAsync(ctx->d_error, 0, sizeof(uint32_t), ctx->stream)) != cudaSuccess) {
+	if ((e = cudaMalloc(&ctx->d_error, 2 * sizeof(uint32_t))) != cudaSuccess ||
+	    (e = cudaMemsetAsync(ctx->d_error, 0, 2 * sizeof(uint32_t), ctx->stream)) != cudaSuccess) {
 		cudaFree(ctx->d_error);
 		free(ctx);
 		return cuda_status(e);
@@ -1428,13 +1428,18 @@ EXTERN_C int risltc_shade_host(risltc_ctx_t* ctx, const risltc_scene_t* scene, u
 	return risltc_ctx_check(ctx);
 }
 
+// Blocks of the query kernels that fit an SM (their registers allow ten or
+// eleven).
+static constexpr int kTraceBlocksPerSm = 10;
+
 EXTERN_C int risltc_trace_shadow(risltc_ctx_t* ctx, const risltc_scene_t* scene, const float* rays, uint32_t ray_count,
                                  uint32_t* hits) {
 	if (!ctx || !scene || (ray_count && (!rays || !hits))) return RISLTC_ERROR_INVALID_ARGUMENT;
 	if (ray_count == 0) return RISLTC_OK;
 	cudaSetDevice(ctx->device);
+	const int blocks = (int) (((size_t) ray_count + 127) / 128);
 	cudaError_t e = risltc::launch_trace_exact(scene->view, (const float4*) rays, ray_count, hits, ctx->d_error,
-	                                           ctx->stream, grid_for(ctx, ray_count));
+	                                           ctx->d_error + 1, ctx->stream, blocks, ctx->sm_count * kTraceBlocksPerSm);
 	if (e == cudaSuccess) ctx->kernel_launches += 1;
 	return cuda_status(e);
 }

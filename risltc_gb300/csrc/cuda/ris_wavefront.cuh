@@ -353,15 +353,15 @@ static __global__ void __launch_bounds__(128) shadow_scatter_kernel(const __grid
 #ifndef RISLTC_TRACE_REFILL
 #define RISLTC_TRACE_REFILL 8
 #endif
-// Persistent any-hit tracing of the queue (queue[0] rays; queue[1] is the
-// fetch cursor, zero at launch).  Each lane holds one ray and advances it by
-// one unit of work (a triangle test or an inner node) per iteration;
-// whenever RISLTC_TRACE_REFILL or more lanes of a warp are idle they fetch
-// the next rays together, so lanes do not wait for the warp's longest ray.
-template <class P>
-__global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_kernel(SceneView s, const ShadowRay* rays, uint32_t* queue,
-                                                           uint8_t* hits, uint32_t* error) {
-	const uint32_t n = queue[0];
+// Persistent any-hit tracing of n queued rays (*cursor is the fetch cursor,
+// zero at launch).  Each lane holds one ray and advances it by one unit of
+// work (a triangle test or an inner node) per iteration; whenever
+// RISLTC_TRACE_REFILL or more lanes of a warp are idle they fetch the next
+// rays together, so lanes do not wait for the warp's longest ray.  Queue
+// supplies ray k (its origin, direction and interval; returns the slot of its
+// outcome) and takes outcomes.
+template <class P, class Queue>
+RL_DEV void trace_queue(const SceneView& s, const Queue& queue, uint32_t n, uint32_t* cursor, uint32_t* error) {
 	const uint32_t lane = threadIdx.x % 32;
 	int32_t stack[kBvhStack];
 	TraceRay r;
@@ -373,19 +373,20 @@ __global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_ker
 		if (!drained && __popc(idle) >= RISLTC_TRACE_REFILL) {
 			const int leader = __ffs(idle) - 1;
 			uint32_t base = 0;
-			if ((int) lane == leader) base = atomicAdd(queue + 1, (uint32_t) __popc(idle));
+			if ((int) lane == leader) base = atomicAdd(cursor, (uint32_t) __popc(idle));
 			base = __shfl_sync(0xffffffffu, base, leader);
 			drained = base + (uint32_t) __popc(idle) >= n;
 			if (!busy) {
 				const uint32_t k = base + (uint32_t) __popc(idle & ((1u << lane) - 1u));
 				if (k < n) {
-					const float4 a = __ldg(&rays[k].origin_slot), b = __ldg(&rays[k].dir_tmax);
-					slot = __float_as_uint(a.w);
-					const int st = trace_begin<P>(s, r, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), 1.0e-3f, b.w);
+					f3 o, d;
+					float t_min, t_max;
+					slot = queue.ray(k, o, d, t_min, t_max);
+					const int st = trace_begin<P>(s, r, o, d, t_min, t_max);
 					if (st == kTraceContinue)
 						busy = true;
 					else
-						hits[slot] = st == kTraceHit ? 1 : 0;
+						queue.outcome(slot, st == kTraceHit);
 				}
 			}
 			continue;
@@ -393,11 +394,51 @@ __global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_ker
 		if (busy) {
 			const int st = trace_step<P>(s, r, stack, error);
 			if (st != kTraceContinue) {
-				hits[slot] = st == kTraceHit ? 1 : 0;
+				queue.outcome(slot, st == kTraceHit);
 				busy = false;
 			}
 		}
 	}
+}
+
+// The shading phase's rays (queue[0] of them; queue[1] is the cursor).
+struct ShadowQueue {
+	const ShadowRay* rays;
+	uint8_t* hits;
+	RL_DEV uint32_t ray(uint32_t k, f3& o, f3& d, float& t_min, float& t_max) const {
+		const float4 a = __ldg(&rays[k].origin_slot), b = __ldg(&rays[k].dir_tmax);
+		o = mk3(a.x, a.y, a.z);
+		d = mk3(b.x, b.y, b.z);
+		t_min = 1.0e-3f;
+		t_max = b.w;
+		return __float_as_uint(a.w);
+	}
+	RL_DEV void outcome(uint32_t slot, bool hit) const { hits[slot] = hit ? 1 : 0; }
+};
+template <class P>
+__global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_kernel(SceneView s, const ShadowRay* rays, uint32_t* queue,
+                                                           uint8_t* hits, uint32_t* error) {
+	trace_queue<P>(s, ShadowQueue{rays, hits}, queue[0], queue + 1, error);
+}
+
+// A caller's rays (risltc_trace_shadow).
+struct CallerQueue {
+	const float4* rays;
+	uint32_t* hits;
+	RL_DEV uint32_t ray(uint32_t k, f3& o, f3& d, float& t_min, float& t_max) const {
+		const float4 a = rays[2 * (size_t) k], b = rays[2 * (size_t) k + 1];
+		o = mk3(a.x, a.y, a.z);
+		d = mk3(b.x, b.y, b.z);
+		t_min = a.w;
+		t_max = b.w;
+		return k;
+	}
+	RL_DEV void outcome(uint32_t slot, bool hit) const { hits[slot] = hit ? 1u : 0u; }
+};
+template <class P>
+__global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) trace_shadow_queue_kernel(SceneView s, const float4* rays, uint32_t count,
+                                                                 uint32_t* hits, uint32_t* cursor, uint32_t* error) {
+	trace_queue<P>(s, CallerQueue{rays, hits}, count, cursor, error);
 }
 
 // The resolve phase of pixel i (all frames of the call).
