@@ -481,14 +481,14 @@ EXTERN_C void risltc_scene_destroy(risltc_scene_t* scene);
  * records between the candidate and shading kernels (used by the default
  * configuration: LTC-CP, light_reservoir, one light sample).  risltc_shade
  * grows the scratch itself when needed (device allocations: these records,
- * the candidate kernel's p_hat slots and, with shadow rays, the ray queue,
- * whose per-light counters depend on the scene) and configures each kernel
+ * the candidate kernel's p_hat slots and, with shadow rays, the ray queue)
+ * and configures each kernel
  * on its first launch.  After one call, later calls that need no more
  * scratch (no more pixels, frames, lights, candidates or clusters) make no
  * allocation and no configuration call; a default-configuration call made
  * after one such call can be captured into a CUDA graph.  Calls with one
  * uniformly drawn light, projected solid angle samples and shadow rays grow
- * scratch of their own (210 bytes per pixel and frame); where it cannot be
+ * scratch of their own (146 bytes per pixel and frame); where it cannot be
  * had, beyond 2^26 pixel-frames and while the stream is being captured they
  * run without it, with the same results, more slowly. */
 EXTERN_C int risltc_ctx_reserve(risltc_ctx_t* ctx, uint32_t width, uint32_t height, uint32_t frame_count);
@@ -527,9 +527,8 @@ typedef struct risltc_batch_item_s {
  * uses the default configuration (LTC-CP, light_reservoir, one light sample
  * and one sample per technique, uniform candidates, shadows on a scene with
  * occluders) with the same numerics and a binned tile shape, the batch runs
- * as one launch per phase for all items (candidate, sample, ray grouping,
- * trace and resolve kernels over the items' concatenated work, in groups of
- * 16 items) on the context's stream; otherwise each item runs its own
+ * as one launch per phase for all items (candidate, sample, trace and
+ * resolve kernels over the items' concatenated work, in groups of 8 items) on the context's stream; otherwise each item runs its own
  * kernels on one of RISLTC_BATCH_STREAMS streams forked from the context's
  * stream and joined back to it.  Either way small frames fill the GPU
  * together and the results equal the items' risltc_shade calls bit for bit.
@@ -608,7 +607,7 @@ EXTERN_C int risltc_trace_shadow(risltc_ctx_t* ctx, const risltc_scene_t* scene,
  * most 64 calls are timed), split into RISLTC_PROFILE_PHASES phases:
  * phase_ms[0] the RIS candidate kernel (or the fused kernel), phase_ms[1] the
  * shading kernel (with its shadow rays, or up to queueing them), phase_ms[2]
- * the grouping of the shadow rays by light (bucket scan and scatter),
+ * 0 (once the grouping of the shadow rays, which are queued as they come),
  * phase_ms[3] the shadow-ray traversal kernel and phase_ms[4] the resolve
  * kernel (0 where a phase is not a kernel of its own), and their number in
  * calls; then enables (enable != 0) or disables timing of the following
@@ -624,8 +623,8 @@ EXTERN_C int risltc_ctx_launch_count(const risltc_ctx_t* ctx, uint64_t* launches
 
 /* The shadow rays that the last risltc_shade call on the context traced
  * through its ray queue (the default configuration with shadows on, and one
- * uniformly drawn light with projected solid angle samples: rays grouped by
- * light, then traced by the persistent kernel); 0 when that call
+ * uniformly drawn light with projected solid angle samples: traced by the
+ * persistent kernel); 0 when that call
  * traced none that way.  Waits for the context's stream.  No counterpart in
  * the reference, whose ray queries run inside the fragment shader; the
  * shadow-ray rate of the benchmark (rays per second) comes from it. */

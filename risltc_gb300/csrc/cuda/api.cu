@@ -55,22 +55,18 @@ struct risltc_ctx_s {
 	size_t logit_capacity;
 	// The shading phase's state between its sample, shadow-ray and resolve
 	// kernels: a 64-byte sample record per pixel-frame, up to two 32-byte
-	// shadow rays per pixel-frame (as staged, then grouped by light), their
-	// outcomes, the queue length and fetch cursor, and the per-light bucket
-	// counters.
+	// shadow rays per pixel-frame and their outcomes.
 	risltc::SampleRecord* d_samples;
-	risltc::ShadowRay* d_staged;
 	risltc::ShadowRay* d_rays;
 	uint8_t* d_hits;
-	uint32_t* d_ray_count;
-	uint32_t* d_light_rays;
 	size_t wavefront_capacity;
-	size_t light_capacity;
-	size_t queue_capacity;  // ray queues (2 words each) in d_ray_count
+	// The launches' counters: one set per frame set of a call.
+	risltc::LaunchCounters* d_counters;
+	size_t counter_capacity;
 	// The scratch of uniform-light calls with queued shadow rays
 	// (uniform_scratch).
 	void* d_uniform;
-	size_t uniform_pixel_frames, uniform_lights;
+	size_t uniform_pixel_frames;
 	// risltc_shade_batch: items run on these streams, forked from and joined
 	// back to the context's stream.
 	cudaStream_t batch_streams[RISLTC_BATCH_STREAMS];
@@ -87,8 +83,8 @@ struct risltc_ctx_s {
 	// Kernels of this library launched through the context (risltc_ctx_launch_count).
 	uint64_t kernel_launches;
 	// Where the last risltc_shade call queued its shadow rays, whose number
-	// risltc_ctx_ray_count reports: 0 nowhere, 1 queue 0 of d_ray_count, 2 the
-	// queue of d_uniform.
+	// risltc_ctx_ray_count reports: 0 nowhere, 1 the queue of d_counters[0], 2
+	// that of d_uniform.
 	int rays_queued;
 	int events_created;
 };
@@ -232,39 +228,31 @@ std::vector<float> child_pair_nodes(const float* nodes, uint32_t node_count) {
 	return out;
 }
 
-int reserve_wavefront(risltc_ctx_t* ctx, size_t pixel_frames, size_t light_count, size_t queues = 1) {
+int reserve_counters(risltc_ctx_t* ctx, size_t sets) {
+	if (sets <= ctx->counter_capacity) return RISLTC_OK;
+	cudaSetDevice(ctx->device);
+	cudaStreamSynchronize(ctx->stream);
+	cudaFree(ctx->d_counters);
+	ctx->d_counters = nullptr;
+	ctx->counter_capacity = 0;
+	const cudaError_t e = cudaMalloc(&ctx->d_counters, sets * sizeof(risltc::LaunchCounters));
+	if (e != cudaSuccess) return cuda_status(e);
+	ctx->counter_capacity = sets;
+	return RISLTC_OK;
+}
+
+int reserve_wavefront(risltc_ctx_t* ctx, size_t pixel_frames) {
 	cudaError_t e = cudaSuccess;
-	if (queues > ctx->queue_capacity) {
-		cudaStreamSynchronize(ctx->stream);
-		cudaFree(ctx->d_ray_count);
-		ctx->d_ray_count = nullptr;
-		ctx->queue_capacity = 0;
-		if ((e = cudaMalloc(&ctx->d_ray_count, 2 * queues * sizeof(uint32_t))) != cudaSuccess) return cuda_status(e);
-		ctx->queue_capacity = queues;
-	}
-	if (light_count > ctx->light_capacity) {
-		cudaStreamSynchronize(ctx->stream);
-		cudaFree(ctx->d_light_rays);
-		ctx->d_light_rays = nullptr;
-		ctx->light_capacity = 0;
-		if ((e = cudaMalloc(&ctx->d_light_rays, light_count * risltc::kLightCounterStride * sizeof(uint32_t))) !=
-		    cudaSuccess)
-			return cuda_status(e);
-		ctx->light_capacity = light_count;
-	}
 	if (pixel_frames <= ctx->wavefront_capacity) return RISLTC_OK;
 	cudaStreamSynchronize(ctx->stream);
 	cudaFree(ctx->d_samples);
-	cudaFree(ctx->d_staged);
 	cudaFree(ctx->d_rays);
 	cudaFree(ctx->d_hits);
 	ctx->d_samples = nullptr;
-	ctx->d_staged = nullptr;
 	ctx->d_rays = nullptr;
 	ctx->d_hits = nullptr;
 	ctx->wavefront_capacity = 0;
 	e = cudaMalloc(&ctx->d_samples, pixel_frames * sizeof(risltc::SampleRecord));
-	if (e == cudaSuccess) e = cudaMalloc(&ctx->d_staged, 2 * pixel_frames * sizeof(risltc::ShadowRay));
 	if (e == cudaSuccess) e = cudaMalloc(&ctx->d_rays, 2 * pixel_frames * sizeof(risltc::ShadowRay));
 	if (e == cudaSuccess) e = cudaMalloc(&ctx->d_hits, 2 * pixel_frames);
 	if (e != cudaSuccess) return cuda_status(e);
@@ -312,11 +300,9 @@ EXTERN_C void risltc_ctx_destroy(risltc_ctx_t* ctx) {
 	cudaFree(ctx->d_candidates);
 	cudaFree(ctx->d_logits);
 	cudaFree(ctx->d_samples);
-	cudaFree(ctx->d_staged);
 	cudaFree(ctx->d_rays);
 	cudaFree(ctx->d_hits);
-	cudaFree(ctx->d_ray_count);
-	cudaFree(ctx->d_light_rays);
+	cudaFree(ctx->d_counters);
 	for (int i = 0; i < ctx->batch_streams_created; ++i) {
 		cudaStreamDestroy(ctx->batch_streams[i]);
 		cudaEventDestroy(ctx->batch_join[i]);
@@ -594,7 +580,7 @@ bool uses_ray_queue(const risltc_scene_t* scene, const risltc_settings_t* s, siz
 
 // The reference's ground-truth estimator (one uniformly drawn light, projected
 // solid angle samples) with its shadow rays queued as above, up to 2^26
-// pixel-frames (13 GB of scratch); larger calls, and calls without scratch,
+// pixel-frames (10 GB of scratch); larger calls, and calls without scratch,
 // run shade_kernel, which gives the same results with inline rays.
 bool may_queue_uniform(const risltc_scene_t* scene, const risltc_settings_t* s, size_t pixel_frames) {
 	return s->light_sampling == light_uniform && s->sample_count_light == 1 && s->sample_count == 1 && s->shadows &&
@@ -611,13 +597,10 @@ struct Scratch {
 	risltc::ProposalCandidate* candidates;
 	__nv_bfloat16* logits;
 	risltc::SampleRecord* samples;
-	risltc::ShadowRay* staged;
 	risltc::ShadowRay* rays;
 	uint8_t* hits;
-	uint32_t* ray_count;
-	uint32_t* light_rays;
-	uint32_t* sample_cursor;  // null: the word after the candidate kernel's tile cursor
-	bool queue_uniform;       // the scratch is uniform_scratch's: may_queue_uniform's route
+	risltc::LaunchCounters* counters;
+	bool queue_uniform;  // the scratch is uniform_scratch's: may_queue_uniform's route
 };
 
 bool uses_proposal(const risltc_settings_t* s) { return s->proposal != risltc_proposal_uniform; }
@@ -784,12 +767,10 @@ int reserve_candidates(risltc_ctx_t* ctx, size_t need) {
 	return RISLTC_OK;
 }
 
-// One region: a p_hat slot per warp of the largest candidate grid, then 64
-// words whose first two are the region's candidate-tile and sample cursors.
-size_t phat_slot_floats(const risltc_ctx_t* ctx) {
+// One region: a p_hat slot per warp of the largest candidate grid.
+size_t phat_region_floats(const risltc_ctx_t* ctx) {
 	return (size_t) ctx->sm_count * risltc::kCandidateBlocksPerSm * risltc::kBinnedWarps * risltc::kPHatSlot;
 }
-size_t phat_region_floats(const risltc_ctx_t* ctx) { return phat_slot_floats(ctx) + 64; }
 
 int reserve_phat(risltc_ctx_t* ctx, int regions) {
 	if (regions <= ctx->phat_regions) return RISLTC_OK;
@@ -845,14 +826,10 @@ risltc::RisParams ris_params(const risltc_ctx_t* ctx, const Scratch& sc, const r
 	r.frame_count = frame_count;
 	r.records = sc.records;
 	r.p_hat_scratch = sc.p_hat;
-	r.tile_cursor = sc.p_hat ? reinterpret_cast<uint32_t*>(sc.p_hat + phat_slot_floats(ctx)) : nullptr;
-	r.sample_cursor = sc.sample_cursor ? sc.sample_cursor : (r.tile_cursor ? r.tile_cursor + 1 : nullptr);
+	r.counters = sc.counters;
 	if (ray_queue) {
 		r.samples = sc.samples;
-		r.staged = sc.staged;
 		r.rays = sc.rays;
-		r.light_rays = sc.light_rays;
-		r.ray_count = sc.ray_count;
 		r.hits = sc.hits;
 	}
 	r.out_rgb = out_rgb;
@@ -946,9 +923,9 @@ int shade_one(risltc_ctx_t* ctx, cudaStream_t stream, const Scratch& sc, const r
 		}
 		e = risltc::launch_ris(r, stream, grid_for(ctx, pixels), grid_for(ctx, 2 * pixels * frame_count), events,
 		                       fast, (int) settings->tile, ctx->sm_count * 16);
-		// Candidates, then the estimator: sample, bucket scan, scatter, trace
-		// and resolve kernels, or one shading kernel with inline rays.
-		if (e == cudaSuccess) ctx->kernel_launches += r.samples ? 6 : 2;
+		// Candidates, then the estimator: sample, trace and resolve kernels,
+		// or one shading kernel with inline rays.
+		if (e == cudaSuccess) ctx->kernel_launches += r.samples ? 4 : 2;
 		if (e == cudaSuccess && train)
 			e = launch_training(ctx, stream, scene, gbuffer, sc.candidates, r.candidate_count, r.train_stride,
 			                    r.train_phase, r.train_shaded, r.records);
@@ -957,8 +934,8 @@ int shade_one(risltc_ctx_t* ctx, cudaStream_t stream, const Scratch& sc, const r
 		                                       out_rgb, accum, reservoirs, true);
 		e = risltc::launch_ris(r, stream, grid_for(ctx, pixels), grid_for(ctx, 2 * pixels * frame_count), events,
 		                       false, 0, 0);
-		// Sample, bucket scan, scatter, trace and resolve kernels.
-		if (e == cudaSuccess) ctx->kernel_launches += 5;
+		// Sample, trace and resolve kernels.
+		if (e == cudaSuccess) ctx->kernel_launches += 3;
 	} else {
 		e = risltc::launch_shade(p, stream, grid_for(ctx, pixels), events, fast);
 		if (e == cudaSuccess) ctx->kernel_launches += 1;
@@ -985,40 +962,30 @@ int check_shade_call(const risltc_ctx_t* ctx, const risltc_scene_t* scene, const
 // configuration refers to.  False where the route is not to be taken: no
 // memory, or the stream is being captured into a graph (which then needs no
 // scratch that a later, larger call would move).
-bool uniform_scratch(risltc_ctx_t* ctx, size_t pixel_frames, size_t light_count, Scratch& sc) {
+bool uniform_scratch(risltc_ctx_t* ctx, size_t pixel_frames, Scratch& sc) {
 	cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
 	if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
 		cudaGetLastError();
 		return false;
 	}
-	if (pixel_frames > ctx->uniform_pixel_frames || light_count > ctx->uniform_lights) {
-		const size_t pf = std::max(pixel_frames, ctx->uniform_pixel_frames);
-		const size_t lights = std::max(light_count, ctx->uniform_lights);
+	if (pixel_frames > ctx->uniform_pixel_frames) {
 		cudaStreamSynchronize(ctx->stream);
 		cudaFree(ctx->d_uniform);
 		ctx->d_uniform = nullptr;
-		ctx->uniform_pixel_frames = ctx->uniform_lights = 0;
-		const size_t bytes = pf * (sizeof(risltc::SampleRecord) + 4 * sizeof(risltc::ShadowRay) +
-		                           sizeof(risltc::ReservoirRecord) + 2) + 256 +
-		                     lights * risltc::kLightCounterStride * sizeof(uint32_t);
-		if (cudaMalloc(&ctx->d_uniform, bytes) != cudaSuccess) {
+		ctx->uniform_pixel_frames = 0;
+		if (cudaMalloc(&ctx->d_uniform, 256 + pixel_frames * (sizeof(risltc::SampleRecord) + 2 * sizeof(risltc::ShadowRay) +
+		                                                      sizeof(risltc::ReservoirRecord) + 2)) != cudaSuccess) {
 			cudaGetLastError();
 			ctx->d_uniform = nullptr;
 			return false;
 		}
-		ctx->uniform_pixel_frames = pf;
-		ctx->uniform_lights = lights;
+		ctx->uniform_pixel_frames = pixel_frames;
 	}
-	// 256 bytes of counters (queue length, fetch cursor, sample cursor), the
-	// per-light counters, then the per-pixel-frame arrays by falling alignment.
+	// 256 bytes for the counters, then the arrays by falling alignment.
 	const size_t pf = ctx->uniform_pixel_frames;
-	uint32_t* const counters = static_cast<uint32_t*>(ctx->d_uniform);
-	sc.ray_count = counters;
-	sc.sample_cursor = counters + 2;
-	sc.light_rays = counters + 64;
-	sc.samples = reinterpret_cast<risltc::SampleRecord*>(sc.light_rays + ctx->uniform_lights * risltc::kLightCounterStride);
-	sc.staged = reinterpret_cast<risltc::ShadowRay*>(sc.samples + pf);
-	sc.rays = sc.staged + 2 * pf;
+	sc.counters = static_cast<risltc::LaunchCounters*>(ctx->d_uniform);
+	sc.samples = reinterpret_cast<risltc::SampleRecord*>(static_cast<char*>(ctx->d_uniform) + 256);
+	sc.rays = reinterpret_cast<risltc::ShadowRay*>(sc.samples + pf);
 	sc.records = reinterpret_cast<risltc::ReservoirRecord*>(sc.rays + 2 * pf);
 	sc.hits = reinterpret_cast<uint8_t*>(sc.records + pf);
 	sc.queue_uniform = true;
@@ -1040,14 +1007,12 @@ int shade_on_context(risltc_ctx_t* ctx, const risltc_scene_t* scene, const rislt
 	if (uses_ris_pipeline(settings)) {
 		if ((st = reserve_records(ctx, pixel_frames))) return st;
 		if ((st = reserve_phat(ctx, 1))) return st;
-		if (uses_ray_queue(scene, settings, pixel_frames) &&
-		    (st = reserve_wavefront(ctx, pixel_frames, scene->view.light_count)))
-			return st;
+		if ((st = reserve_counters(ctx, 1))) return st;
+		if (uses_ray_queue(scene, settings, pixel_frames) && (st = reserve_wavefront(ctx, pixel_frames))) return st;
 	}
-	Scratch sc{ctx->d_records, ctx->d_phat, ctx->d_candidates, ctx->d_logits, ctx->d_samples, ctx->d_staged,
-	           ctx->d_rays, ctx->d_hits, ctx->d_ray_count, ctx->d_light_rays};
-	if (may_queue_uniform(scene, settings, pixel_frames))
-		uniform_scratch(ctx, pixel_frames, scene->view.light_count, sc);
+	Scratch sc{ctx->d_records, ctx->d_phat, ctx->d_candidates, ctx->d_logits,
+	           ctx->d_samples, ctx->d_rays, ctx->d_hits, ctx->d_counters};
+	if (may_queue_uniform(scene, settings, pixel_frames)) uniform_scratch(ctx, pixel_frames, sc);
 	st = shade_one(ctx, ctx->stream, sc, scene, gbuffer, settings, noise_seed, animate, frame_count, out_rgb, accum,
 	               reservoirs, events);
 	ctx->rays_queued =
@@ -1230,23 +1195,21 @@ bool batch_is_fused(const risltc_batch_item_t* items, uint32_t item_count) {
 }
 
 // The whole batch with one launch per phase (groups of kBatchItems items),
-// on the context's stream; the scratch is reserved.  queues: the items' ray
-// queues, followed by the trace's fetch cursor.
-int shade_batch_fused(risltc_ctx_t* ctx, const risltc_batch_item_t* items, uint32_t item_count, size_t queues) {
+// on the context's stream; the scratch is reserved (a set of counters per
+// item, then one for the batch's cursors).
+int shade_batch_fused(risltc_ctx_t* ctx, const risltc_batch_item_t* items, uint32_t item_count) {
 	const risltc_tile_t tile = items[0].settings.tile;
 	const bool fast = items[0].settings.numerics == risltc_numerics_fast;
 	const uint32_t px_per_tile = tile_pixels(tile);
-	size_t r_off = 0, w_off = 0, l_off = 0;
+	size_t r_off = 0, w_off = 0;
 	for (uint32_t g0 = 0; g0 < item_count; g0 += risltc::kBatchItems) {
 		const uint32_t gn = std::min<uint32_t>(item_count - g0, (uint32_t) risltc::kBatchItems);
 		risltc::RisBatch b;
 		memset(&b, 0, sizeof(b));
 		b.count = gn;
 		b.p_hat_scratch = ctx->d_phat;
-		b.tile_cursor = reinterpret_cast<uint32_t*>(ctx->d_phat + phat_slot_floats(ctx));
-		b.ray_cursor = ctx->d_ray_count + 2 * queues;
+		b.counters = ctx->d_counters + item_count;
 		uint32_t tiles = 0, pixels = 0, pfs = 0;
-		const size_t l_begin = l_off;
 		for (uint32_t k = 0; k != gn; ++k) {
 			const risltc_batch_item_t& it = items[g0 + k];
 			const uint32_t np = it.gbuffer.width * it.gbuffer.height;
@@ -1255,36 +1218,33 @@ int shade_batch_fused(risltc_ctx_t* ctx, const risltc_batch_item_t* items, uint3
 			sc.records = ctx->d_records + r_off;
 			sc.p_hat = ctx->d_phat;
 			sc.samples = ctx->d_samples + w_off;
-			sc.staged = ctx->d_staged + 2 * w_off;
 			sc.rays = ctx->d_rays + 2 * w_off;
 			sc.hits = ctx->d_hits + 2 * w_off;
-			sc.ray_count = ctx->d_ray_count + 2 * (size_t) (g0 + k);
-			sc.light_rays = ctx->d_light_rays + l_off * risltc::kLightCounterStride;
+			sc.counters = ctx->d_counters + g0 + k;
 			b.item[k] = ris_params(ctx, sc, it.scene, &it.gbuffer, &it.settings, it.noise->random_seed, it.animate,
 			                       it.frame_count, it.out_rgb, it.accum, it.reservoirs, true);
 			b.tile_begin[k] = tiles;
 			b.pixel_begin[k] = pixels;
-			b.pf_begin[k] = pfs;
+			b.ray_begin[k] = 2 * pfs;
 			tiles += (np + px_per_tile - 1) / px_per_tile;
-			pixels += np;
+			pixels += (np + 31) / 32 * 32;
 			pfs += pf;
 			r_off += pf;
 			w_off += pf;
-			l_off += (size_t) it.scene->view.light_count;
 		}
 		b.tile_begin[gn] = tiles;
 		b.pixel_begin[gn] = pixels;
-		b.pf_begin[gn] = pfs;
-		cudaError_t e = cudaMemsetAsync(ctx->d_light_rays + l_begin * risltc::kLightCounterStride, 0,
-		                                sizeof(uint32_t) * (l_off - l_begin) * risltc::kLightCounterStride, ctx->stream);
+		b.ray_begin[gn] = 2 * pfs;
+		// The counters of this group's items, of the later ones and of the batch.
+		cudaError_t e = cudaMemsetAsync(ctx->d_counters + g0, 0, (item_count - g0 + 1) * sizeof(risltc::LaunchCounters),
+		                                ctx->stream);
 		if (e == cudaSuccess)
 			e = fast ? risltc::launch_candidates_batch_fast(b, ctx->stream, ctx->sm_count * 16, (int) tile)
 			         : risltc::launch_candidates_batch_exact(b, ctx->stream, ctx->sm_count * 16, (int) tile);
 		if (e == cudaSuccess)
-			e = risltc::launch_batch_estimator(b, ctx->stream, grid_for(ctx, pixels), grid_for(ctx, pfs),
-			                                   grid_for(ctx, 2 * (size_t) pfs));
+			e = risltc::launch_batch_estimator(b, ctx->stream, grid_for(ctx, pixels), grid_for(ctx, 2 * (size_t) pfs));
 		if (e != cudaSuccess) return cuda_status(e);
-		ctx->kernel_launches += 6;
+		ctx->kernel_launches += 4;
 	}
 	for (uint32_t i = 0; i != item_count; ++i) items[i].noise->random_seed += items[i].frame_count;
 	return RISLTC_OK;
@@ -1296,7 +1256,7 @@ EXTERN_C int risltc_shade_batch(risltc_ctx_t* ctx, const risltc_batch_item_t* it
 	if (!ctx || (!items && item_count)) return RISLTC_ERROR_INVALID_ARGUMENT;
 	if (item_count == 0) return RISLTC_OK;
 	// Validate everything before any work; size the scratch for all items.
-	size_t records = 0, wavefront = 0, lights = 0, queues = 0, candidates = 0, logits = 0;
+	size_t records = 0, wavefront = 0, candidates = 0, logits = 0;
 	for (uint32_t i = 0; i != item_count; ++i) {
 		const risltc_batch_item_t& it = items[i];
 		if (!valid_call(it.scene, &it.gbuffer, it.noise, it.frame_count) || it.scene->ctx != ctx)
@@ -1310,11 +1270,7 @@ EXTERN_C int risltc_shade_batch(risltc_ctx_t* ctx, const risltc_batch_item_t* it
 		if (it.settings.proposal == risltc_proposal_learned)
 			logits += (size_t) it.gbuffer.width * it.gbuffer.height * it.scene->clusters.count;
 		if (uses_ris_pipeline(&it.settings)) records += pf;
-		if (uses_ray_queue(it.scene, &it.settings, pf)) {
-			wavefront += pf;
-			lights += (size_t) it.scene->view.light_count;
-			++queues;
-		}
+		if (uses_ray_queue(it.scene, &it.settings, pf)) wavefront += pf;
 	}
 	cudaSetDevice(ctx->device);
 	int st;
@@ -1322,9 +1278,10 @@ EXTERN_C int risltc_shade_batch(risltc_ctx_t* ctx, const risltc_batch_item_t* it
 	if (records && (st = reserve_phat(ctx, RISLTC_BATCH_STREAMS))) return st;
 	if (candidates && (st = reserve_candidates(ctx, candidates))) return st;
 	if (logits && (st = reserve_logits(ctx, logits))) return st;
-	// One more queue slot than items: the whole-batch trace's fetch cursor.
-	if (queues && (st = reserve_wavefront(ctx, wavefront, lights, queues + 1))) return st;
-	if (batch_is_fused(items, item_count)) return shade_batch_fused(ctx, items, item_count, queues);
+	// One more set of counters than items: the whole batch's cursors.
+	if (records && (st = reserve_counters(ctx, (size_t) item_count + 1))) return st;
+	if (wavefront && (st = reserve_wavefront(ctx, wavefront))) return st;
+	if (batch_is_fused(items, item_count)) return shade_batch_fused(ctx, items, item_count);
 	cudaError_t e = cudaSuccess;
 	if (!ctx->batch_streams_created) {
 		e = cudaEventCreateWithFlags(&ctx->batch_fork, cudaEventDisableTiming);
@@ -1340,7 +1297,7 @@ EXTERN_C int risltc_shade_batch(risltc_ctx_t* ctx, const risltc_batch_item_t* it
 	if ((e = cudaEventRecord(ctx->batch_fork, ctx->stream)) != cudaSuccess) return cuda_status(e);
 	for (int k = 0; k != streams; ++k)
 		if ((e = cudaStreamWaitEvent(ctx->batch_streams[k], ctx->batch_fork, 0)) != cudaSuccess) return cuda_status(e);
-	size_t r_off = 0, w_off = 0, l_off = 0, q_off = 0, c_off = 0, g_off = 0;
+	size_t r_off = 0, w_off = 0, c_off = 0, g_off = 0;
 	for (uint32_t i = 0; i != item_count; ++i) {
 		const risltc_batch_item_t& it = items[i];
 		const size_t pf = (size_t) it.gbuffer.width * it.gbuffer.height * it.frame_count;
@@ -1348,6 +1305,7 @@ EXTERN_C int risltc_shade_batch(risltc_ctx_t* ctx, const risltc_batch_item_t* it
 		if (uses_ris_pipeline(&it.settings)) {
 			sc.records = ctx->d_records + r_off;
 			sc.p_hat = ctx->d_phat + phat_region_floats(ctx) * (i % RISLTC_BATCH_STREAMS);
+			sc.counters = ctx->d_counters + i;
 			r_off += pf;
 		}
 		if (uses_proposal(&it.settings)) {
@@ -1360,14 +1318,9 @@ EXTERN_C int risltc_shade_batch(risltc_ctx_t* ctx, const risltc_batch_item_t* it
 		}
 		if (uses_ray_queue(it.scene, &it.settings, pf)) {
 			sc.samples = ctx->d_samples + w_off;
-			sc.staged = ctx->d_staged + 2 * w_off;
 			sc.rays = ctx->d_rays + 2 * w_off;
 			sc.hits = ctx->d_hits + 2 * w_off;
-			sc.ray_count = ctx->d_ray_count + 2 * q_off;
-			sc.light_rays = ctx->d_light_rays + l_off * risltc::kLightCounterStride;
 			w_off += pf;
-			l_off += (size_t) it.scene->view.light_count;
-			++q_off;
 		}
 		st = shade_one(ctx, ctx->batch_streams[i % RISLTC_BATCH_STREAMS], sc, it.scene, &it.gbuffer, &it.settings,
 		               it.noise->random_seed, it.animate, it.frame_count, it.out_rgb, it.accum, it.reservoirs,
@@ -1447,10 +1400,10 @@ EXTERN_C int risltc_trace_shadow(risltc_ctx_t* ctx, const risltc_scene_t* scene,
 EXTERN_C int risltc_ctx_ray_count(risltc_ctx_t* ctx, uint32_t* rays) {
 	if (!ctx || !rays) return RISLTC_ERROR_INVALID_ARGUMENT;
 	*rays = 0;
-	const void* queue = ctx->rays_queued == 2 ? ctx->d_uniform : ctx->d_ray_count;
-	if (!ctx->rays_queued || !queue) return RISLTC_OK;
+	const auto* counters = ctx->rays_queued == 2 ? static_cast<const risltc::LaunchCounters*>(ctx->d_uniform) : ctx->d_counters;
+	if (!ctx->rays_queued || !counters) return RISLTC_OK;
 	cudaSetDevice(ctx->device);
-	cudaError_t e = cudaMemcpyAsync(rays, queue, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream);
+	cudaError_t e = cudaMemcpyAsync(rays, &counters->rays, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream);
 	if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
 	return cuda_status(e);
 }

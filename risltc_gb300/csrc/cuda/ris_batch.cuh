@@ -1,16 +1,15 @@
 // ris_batch.cuh - the wavefront pipeline of the default configuration run
 // over a batch of frames (risltc_shade_batch) with one launch per phase: the
-// candidate, sample, bucket-scan, scatter, trace and resolve kernels each
-// take their work units (warp tiles, pixels, lights, pixel-frames, rays)
-// from the concatenation of all items' units, so a batch of small and large
-// frames fills the GPU in six launches instead of six per item.
+// candidate, sample, trace and resolve kernels each take their work units
+// (warp tiles, pixels, rays) from the concatenation of all items' units, so a
+// batch of small and large frames fills the GPU in four launches instead of
+// four per item.
 //
 // Every unit runs the single-frame kernels' body (binned_tile, sample_pixel,
-// light_bucket_scan, scatter_pixel_frame, the trace loop, resolve_pixel) with
-// its item's parameters, so each item's results are bit-identical to its own
-// risltc_shade call.  The items' parameters travel in kernel parameter space
-// (RisBatch, about 4.6 KB for 16 items) and are captured by value into a
-// CUDA graph.
+// the trace loop, resolve_pixel) with its item's parameters, so each item's
+// results are bit-identical to its own risltc_shade call.  The items'
+// parameters travel in kernel parameter space (RisBatch, about 2.2 KB for 8
+// items) and are captured by value into a CUDA graph.
 #pragma once
 #include "ris_binned.cuh"
 #include "ris_wavefront.cuh"
@@ -19,21 +18,22 @@ namespace risltc {
 
 // Items per whole-batch launch; risltc_shade_batch runs larger batches in
 // groups of this many.
-constexpr int kBatchItems = 16;
+constexpr int kBatchItems = 8;
 
 struct RisBatch {
 	uint32_t count;
 	// Prefix sums over the items of their candidate tiles (kPixels pixels
-	// each, for the tile shape of the launch), pixels and pixel-frames.
+	// each, for the tile shape of the launch) and of their pixels, each item's
+	// rounded up to whole warps of 32, and of their queue places (two per
+	// pixel-frame).
 	uint32_t tile_begin[kBatchItems + 1];
 	uint32_t pixel_begin[kBatchItems + 1];
-	uint32_t pf_begin[kBatchItems + 1];
+	uint32_t ray_begin[kBatchItems + 1];
 	// The candidate kernel's per-warp p_hat slots (for the launch's grid).
 	float* p_hat_scratch;
-	uint32_t* tile_cursor;  // the next warp tile over all items (zeroed before each launch)
-	// Fetch cursor of the batch's concatenated ray queue (zeroed by the scan
-	// kernel); the items' queue lengths are in their ray_count[0].
-	uint32_t* ray_cursor;
+	// The batch's cursors over all items' units; the items' ray counts are in
+	// their own counters.  Zeroed before the launches, as the items' are.
+	LaunchCounters* counters;
 	RisParams item[kBatchItems];
 };
 
@@ -59,7 +59,7 @@ ris_candidates_batch_kernel(const __grid_constant__ RisBatch b) {
 	Tile& tile = reinterpret_cast<Tile*>(smem_raw)[threadIdx.x / 32];
 	float* const phat = b.p_hat_scratch + (size_t) (blockIdx.x * kBinnedWarps + threadIdx.x / 32) * kPHatSlot;
 	const uint32_t tiles = b.tile_begin[b.count];
-	for (uint32_t u = next_warp_tile(b.tile_cursor); u < tiles; u = next_warp_tile(b.tile_cursor)) {
+	for (uint32_t u = next_warp_tile(&b.counters->tile); u < tiles; u = next_warp_tile(&b.counters->tile)) {
 		const uint32_t k = batch_item(b.tile_begin, b.count, u);
 		binned_tile<P, kPixels, kChunk>(b.item[k], tile, phat, u - b.tile_begin[k]);
 	}
@@ -73,8 +73,6 @@ cudaError_t launch_candidates_batch(const RisBatch& b, cudaStream_t stream, int 
 	const cudaError_t e = configure_candidate_kernel(ris_candidates_batch_kernel<P, kPixels, kChunk>,
 	                                                 binned_smem_bytes<P, kPixels, kChunk>(), configured, resident, device);
 	if (e != cudaSuccess) return e;
-	const cudaError_t z = cudaMemsetAsync(b.tile_cursor, 0, sizeof(uint32_t), stream);
-	if (z != cudaSuccess) return z;
 	const size_t blocks = ((size_t) b.tile_begin[b.count] + kBinnedWarps - 1) / kBinnedWarps;
 	const int grid = (int) std::max<size_t>(
 	    1, std::min<size_t>(blocks, (size_t) std::min(grid_cap, resident[device & 63].load())));
@@ -86,25 +84,10 @@ cudaError_t launch_candidates_batch(const RisBatch& b, cudaStream_t stream, int 
 template <class P>
 __global__ void __launch_bounds__(kSampleThreads, RISLTC_SAMPLE_MIN_BLOCKS) ris_sample_batch_kernel(const __grid_constant__ RisBatch b) {
 	__shared__ PsaPolygon poly[kSampleThreads];
-	const uint32_t total = b.pixel_begin[b.count];
-	for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < total; u += gridDim.x * blockDim.x) {
-		const uint32_t k = batch_item(b.pixel_begin, b.count, u);
+	const uint32_t chunks = b.pixel_begin[b.count] / 32;
+	for (uint32_t c = next_warp_tile(&b.counters->sample); c < chunks; c = next_warp_tile(&b.counters->sample)) {
+		const uint32_t u = c * 32 + threadIdx.x % 32, k = batch_item(b.pixel_begin, b.count, c * 32);
 		sample_pixel<P, false>(b.item[k], u - b.pixel_begin[k], poly[threadIdx.x]);
-	}
-}
-
-// One block of 1024 threads per item.
-static __global__ void __launch_bounds__(1024) light_bucket_scan_batch_kernel(const __grid_constant__ RisBatch b) {
-	const RisParams& pr = b.item[blockIdx.x];
-	light_bucket_scan(pr.light_rays, (uint32_t) pr.scene.light_count, pr.ray_count);
-	if (blockIdx.x == 0 && threadIdx.x == 0) *b.ray_cursor = 0;
-}
-
-static __global__ void __launch_bounds__(128) shadow_scatter_batch_kernel(const __grid_constant__ RisBatch b) {
-	const uint32_t total = b.pf_begin[b.count];
-	for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < total; u += gridDim.x * blockDim.x) {
-		const uint32_t k = batch_item(b.pf_begin, b.count, u);
-		scatter_pixel_frame(b.item[k], u - b.pf_begin[k]);
 	}
 }
 
@@ -113,17 +96,7 @@ static __global__ void __launch_bounds__(128) shadow_scatter_batch_kernel(const 
 // each lane traverses its ray's item's BVH and writes its item's outcome.
 template <class P>
 __global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_batch_kernel(const __grid_constant__ RisBatch b) {
-	__shared__ uint32_t ray_begin[kBatchItems + 1];
-	if (threadIdx.x == 0) {
-		uint32_t total = 0;
-		for (uint32_t k = 0; k != b.count; ++k) {
-			ray_begin[k] = total;
-			total += b.item[k].ray_count[0];
-		}
-		ray_begin[b.count] = total;
-	}
-	__syncthreads();
-	const uint32_t n = ray_begin[b.count];
+	const uint32_t n = b.ray_begin[b.count];
 	const uint32_t lane = threadIdx.x % 32;
 	uint32_t* const error = b.item[0].error;
 	int32_t stack[kBvhStack];
@@ -138,21 +111,21 @@ __global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_bat
 		if (!drained && __popc(idle) >= RISLTC_TRACE_REFILL) {
 			const int leader = __ffs(idle) - 1;
 			uint32_t base = 0;
-			if ((int) lane == leader) base = atomicAdd(b.ray_cursor, (uint32_t) __popc(idle));
+			if ((int) lane == leader) base = atomicAdd(&b.counters->fetch, (uint32_t) __popc(idle));
 			base = __shfl_sync(0xffffffffu, base, leader);
 			drained = base + (uint32_t) __popc(idle) >= n;
 			if (!busy) {
 				const uint32_t g = base + (uint32_t) __popc(idle & ((1u << lane) - 1u));
 				if (g < n) {
-					const uint32_t k = batch_item(ray_begin, b.count, g);
+					const uint32_t k = batch_item(b.ray_begin, b.count, g);
 					const RisParams& pr = b.item[k];
 					s.pairs = pr.scene.pairs;
 					s.triangles = pr.scene.triangles;
 					s.triangle_count = pr.scene.triangle_count;
 					hits = pr.hits;
-					const ShadowRay* ray = pr.rays + (g - ray_begin[k]);
-					const float4 a = __ldg(&ray->origin_slot), d = __ldg(&ray->dir_tmax);
-					slot = __float_as_uint(a.w);
+					slot = g - b.ray_begin[k];
+					const ShadowRay* ray = pr.rays + slot;
+					const float4 a = __ldg(&ray->origin), d = __ldg(&ray->dir_tmax);
 					const int st = trace_begin<P>(s, r, mk3(a.x, a.y, a.z), mk3(d.x, d.y, d.z), 1.0e-3f, d.w);
 					if (st == kTraceContinue)
 						busy = true;
@@ -186,8 +159,7 @@ cudaError_t launch_candidates_batch_exact(const RisBatch& b, cudaStream_t stream
 cudaError_t launch_candidates_batch_fast(const RisBatch& b, cudaStream_t stream, int grid_cap, int tile);
 cudaError_t launch_candidates_batch_tile_exact(const RisBatch& b, cudaStream_t stream, int grid_cap, int tile);
 cudaError_t launch_candidates_batch_tile_fast(const RisBatch& b, cudaStream_t stream, int grid_cap, int tile);
-// Sample, scan, scatter, trace and resolve kernels of the batch, with the
-// given grids (the scan runs one block per item).
-cudaError_t launch_batch_estimator(const RisBatch& b, cudaStream_t stream, int pixel_grid, int pf_grid, int ray_grid);
+// Sample, trace and resolve kernels of the batch, with the given grids.
+cudaError_t launch_batch_estimator(const RisBatch& b, cudaStream_t stream, int pixel_grid, int ray_grid);
 
 }  // namespace risltc

@@ -704,7 +704,7 @@ ris_candidates_binned_kernel(const __grid_constant__ RisParams pr) {
 	Tile& tile = reinterpret_cast<Tile*>(smem_raw)[threadIdx.x / 32];
 	float* const phat = pr.p_hat_scratch + (size_t) (blockIdx.x * kBinnedWarps + threadIdx.x / 32) * kPHatSlot;
 	const uint32_t tiles = (pr.width * pr.height + kPixels - 1) / kPixels;
-	for (uint32_t t = next_warp_tile(pr.tile_cursor); t < tiles; t = next_warp_tile(pr.tile_cursor))
+	for (uint32_t t = next_warp_tile(&pr.counters->tile); t < tiles; t = next_warp_tile(&pr.counters->tile))
 		binned_tile<P, kPixels, kChunk>(pr, tile, phat, t);
 }
 
@@ -758,8 +758,6 @@ cudaError_t launch_candidates_binned(const RisParams& p, cudaStream_t stream, in
 	const cudaError_t e = configure_candidate_kernel(ris_candidates_binned_kernel<P, kPixels, kChunk>,
 	                                                 binned_smem_bytes<P, kPixels, kChunk>(), configured, resident, device);
 	if (e != cudaSuccess) return e;
-	const cudaError_t z = cudaMemsetAsync(p.tile_cursor, 0, sizeof(uint32_t), stream);
-	if (z != cudaSuccess) return z;
 	ris_candidates_binned_kernel<P, kPixels, kChunk>
 	    <<<std::min(grid, resident[device & 63].load()), 32 * kBinnedWarps, binned_smem_bytes<P, kPixels, kChunk>(),
 	       stream>>>(p);

@@ -33,6 +33,14 @@ RL_DEV uint32_t next_warp_tile(uint32_t* cursor) {
 	return __shfl_sync(0xffffffffu, t, 0);
 }
 
+// The counters of one frame set's launches, zeroed before them.
+struct LaunchCounters {
+	uint32_t tile;    // the binned candidate kernel's next warp tile
+	uint32_t sample;  // the sample kernel's next 32 pixels
+	uint32_t rays;    // shadow rays to trace (risltc_ctx_ray_count)
+	uint32_t fetch;   // the trace kernel's next queue entry
+};
+
 struct RisParams {
 	SceneView scene;
 	const float* gbuffer;
@@ -56,8 +64,7 @@ struct RisParams {
 	// floats per warp of the grid); null selects the one-thread-per-pixel
 	// candidate kernel.
 	float* p_hat_scratch;
-	uint32_t* tile_cursor;         // the binned candidate kernel's next warp tile (zeroed before each launch)
-	uint32_t* sample_cursor;       // the sample kernel's next 32 pixels (zeroed before each launch)
+	LaunchCounters* counters;  // null where no kernel that needs them runs
 	// Candidates drawn by a proposal ([frame][pixel][candidate]); null: each
 	// candidate is drawn uniformly from the pixel's noise as in the reference.
 	const ProposalCandidate* candidates;
@@ -71,10 +78,7 @@ struct RisParams {
 	float* train_shaded;
 	// Shadow rays traced in their own pass (null: traced in ris_shade_kernel).
 	struct SampleRecord* samples;  // [frame][pixel]
-	struct ShadowRay* staged;      // [frame][pixel][technique], as generated
-	struct ShadowRay* rays;        // the traced ones grouped by light
-	uint32_t* light_rays;          // per light: ray count, then bucket cursor
-	uint32_t* ray_count;           // [queue length, trace fetch cursor]
+	struct ShadowRay* rays;        // [frame][pixel][technique]
 	uint8_t* hits;                 // [frame][pixel][technique] occlusion
 	float* out_rgb;
 	double* accum;
@@ -324,12 +328,6 @@ template <class P> __global__ void __launch_bounds__(kShadeThreads) ris_shade_ke
 	}
 }
 
-// Words between consecutive lights' ray counters (the sample and scatter
-// kernels' atomics and the bucket scan): one 32-byte sector per counter
-// spreads the millions of atomics per launch over many L2 slices (packed
-// counters: ray sort + trace 1.64 ms per 1080p frame; one per sector: 1.53).
-constexpr uint32_t kLightCounterStride = 8;
-
 // Blocks of 128 threads for one thread per pixel, at most grid_cap.
 inline int grid_for_pixels(size_t pixels, int grid_cap) {
 	const size_t blocks = (pixels + 127) / 128;
@@ -346,33 +344,29 @@ cudaError_t launch_candidates_tile_exact(const RisParams& p, cudaStream_t stream
 cudaError_t launch_candidates_tile_fast(const RisParams& p, cudaStream_t stream, int grid_cap, int tile);
 cudaError_t launch_ris_shade(const RisParams& p, cudaStream_t stream, int grid);
 cudaError_t launch_ris_sample(const RisParams& p, cudaStream_t stream, int grid);
-cudaError_t launch_shadow_sort(const RisParams& p, cudaStream_t stream, int grid);
 cudaError_t launch_shadow_trace(const RisParams& p, cudaStream_t stream, int grid);
 cudaError_t launch_ris_resolve(const RisParams& p, cudaStream_t stream, int grid);
 
 // The candidate kernel (fast or exact numerics, tile shape `tile`, at most
 // grid_cap blocks; none with p.uniform_light), then the shading phase (always exact): ris_shade_kernel,
-// or with p.samples set the sample kernel, the shadow rays' grouping by light
-// and trace, and the resolve kernel.  events (may be null) holds five events,
-// recorded before, between and after the phases (the last three together for
-// ris_shade_kernel).
+// or with p.samples set the sample kernel, the shadow rays' trace and the
+// resolve kernel.  events (may be null) holds RISLTC_PROFILE_PHASES + 1 events,
+// recorded before, between and after the phases (those of phases that are no
+// kernel together).
 inline cudaError_t launch_ris(const RisParams& p, cudaStream_t stream, int grid, int trace_grid, cudaEvent_t* events,
                               bool fast, int tile, int grid_cap) {
+	cudaError_t e = p.counters ? cudaMemsetAsync(p.counters, 0, sizeof(LaunchCounters), stream) : cudaSuccess;
+	if (e != cudaSuccess) return e;
 	if (events) cudaEventRecord(events[0], stream);
-	cudaError_t e = cudaSuccess;
 	if (!p.uniform_light)
 		e = fast ? launch_candidates_fast(p, stream, grid_cap, tile) : launch_candidates_exact(p, stream, grid_cap, tile);
 	if (e != cudaSuccess) return e;
 	if (events) cudaEventRecord(events[1], stream);
 	if (p.samples) {
-		e = cudaMemsetAsync(p.light_rays, 0, sizeof(uint32_t) * p.scene.light_count * kLightCounterStride, stream);
-		if (e == cudaSuccess) e = cudaMemsetAsync(p.sample_cursor, 0, sizeof(uint32_t), stream);
-		if (e == cudaSuccess) e = launch_ris_sample(p, stream, grid);
+		e = launch_ris_sample(p, stream, grid);
 		if (e != cudaSuccess) return e;
-		if (events) cudaEventRecord(events[2], stream);
-		e = launch_shadow_sort(p, stream, grid);
-		if (e != cudaSuccess) return e;
-		if (events) cudaEventRecord(events[3], stream);
+		if (events)
+			for (int k = 2; k != 4; ++k) cudaEventRecord(events[k], stream);
 		e = launch_shadow_trace(p, stream, trace_grid);
 		if (e != cudaSuccess) return e;
 		if (events) cudaEventRecord(events[4], stream);

@@ -40,15 +40,10 @@ cudaError_t launch_ris_sample(const RisParams& p, cudaStream_t stream, int grid)
 		ris_sample_kernel<ExactNumerics, false><<<grid, kSampleThreads, 0, stream>>>(p);
 	return cudaGetLastError();
 }
-cudaError_t launch_shadow_sort(const RisParams& p, cudaStream_t stream, int grid) {
-	light_bucket_scan_kernel<<<1, 1024, 0, stream>>>(p.light_rays, (uint32_t) p.scene.light_count, p.ray_count);
-	cudaError_t e = cudaGetLastError();
-	if (e != cudaSuccess) return e;
-	shadow_scatter_kernel<<<grid, 128, 0, stream>>>(p);
-	return cudaGetLastError();
-}
 cudaError_t launch_shadow_trace(const RisParams& p, cudaStream_t stream, int grid) {
-	shadow_trace_kernel<ExactNumerics><<<grid, 128, 0, stream>>>(p.scene, p.rays, p.ray_count, p.hits, p.error);
+	const uint32_t count = 2u * p.width * p.height * p.frame_count;
+	shadow_trace_kernel<ExactNumerics>
+	    <<<grid, 128, 0, stream>>>(p.scene, p.rays, count, &p.counters->fetch, p.hits, p.error);
 	return cudaGetLastError();
 }
 cudaError_t launch_ris_resolve(const RisParams& p, cudaStream_t stream, int grid) {
@@ -59,14 +54,10 @@ cudaError_t launch_candidates_batch_exact(const RisBatch& b, cudaStream_t stream
 	if (tile == risltc_tile_32x8) return launch_candidates_batch<ExactNumerics, 32, 8>(b, stream, grid_cap);
 	return launch_candidates_batch_tile_exact(b, stream, grid_cap, tile);
 }
-cudaError_t launch_batch_estimator(const RisBatch& b, cudaStream_t stream, int pixel_grid, int pf_grid, int ray_grid) {
+cudaError_t launch_batch_estimator(const RisBatch& b, cudaStream_t stream, int pixel_grid, int ray_grid) {
 	ris_sample_batch_kernel<ExactNumerics><<<pixel_grid, kSampleThreads, 0, stream>>>(b);
 	cudaError_t e = cudaGetLastError();
 	if (e != cudaSuccess) return e;
-	light_bucket_scan_batch_kernel<<<b.count, 1024, 0, stream>>>(b);
-	if ((e = cudaGetLastError()) != cudaSuccess) return e;
-	shadow_scatter_batch_kernel<<<pf_grid, 128, 0, stream>>>(b);
-	if ((e = cudaGetLastError()) != cudaSuccess) return e;
 	shadow_trace_batch_kernel<ExactNumerics><<<ray_grid, 128, 0, stream>>>(b);
 	if ((e = cudaGetLastError()) != cudaSuccess) return e;
 	ris_resolve_batch_kernel<ExactNumerics><<<pixel_grid, 128, 0, stream>>>(b);
