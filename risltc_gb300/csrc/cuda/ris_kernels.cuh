@@ -299,7 +299,8 @@ template <class P> __global__ void __launch_bounds__(kShadeThreads) ris_shade_ke
 				Light l;
 				load_light(pr.scene, r.light_index, l);
 				uint32_t seed = r.seed;
-				f3 color = psa_mis_shade<P>(sp, sd, ltc, l, seed, true, true, polys[0][threadIdx.x], polys[1][threadIdx.x]);
+				f3 color = psa_mis_shade<P>(sp, sd, ltc, l, light_record(pr.scene, r.light_index), seed, true, true, polys[0][threadIdx.x],
+				                                polys[1][threadIdx.x]);
 				float W = P::div(r.w_sum, (float) pr.candidate_count * r.p_hat);
 				if (r.p_hat == 0.0f) W = 0.0f;
 				f3 cw = scale(color, W);

@@ -98,7 +98,7 @@ RL_DEV uint32_t psa_mis_emit(const ShadeParams& pr, bool peters, const ShadingDa
 	for (int j = 0; j != 2; ++j) {
 		const uint32_t vc = prepare_space_record<P>(j == 0 ? ltc.world_to_shading
 		                                                  : mul(ltc.shading_to_cosine, ltc.world_to_shading),
-		                                           record, poly, fa);
+		                                           record, l.vertex_count, poly, fa);
 		psa[j] = vc == 0 ? 0.0f : poly.psa;
 		if (j == 0 && (vc == 0 || psa[0] == 0.0f)) {
 			store_contributions(dst, 0, splat(0.0f), splat(0.0f));

@@ -291,41 +291,53 @@ template <class P> RL_DEV f3 ltc_cp_target(const ShadingData& sd, Ltc ltc, const
 // evaluate_polygonal_light_shading (peters = false, :458-550)
 // One polygon's transform to local space, clip_polygon and
 // prepare_projected_solid_angle_polygon_sampling (shading_pass.frag.glsl:
-// 315-336).  Out of line so that the kernels hold one copy of this long
-// code, shared by the diffuse and specular passes.  Returns the clipped
-// vertex count (0: nothing left, p untouched).
+// 315-336), the n vertices read from the light's device record.  Returns the
+// clipped vertex count (0: nothing left).  The vertices go straight into p; a
+// partially clipped polygon is then written over them in clip_polygon's
+// output order, its run above the horizon transformed again.  Without vertex
+// arrays there is no local memory and little code: the sample kernel, whose
+// instruction fetches were a fifth of its stalls, takes 3.28 instead of
+// 3.64 ms per 4-frame 1080p launch.
 template <class P>
-__device__ __noinline__ uint32_t prepare_space(mat43 w2l, const Light& l, PsaPolygon& p, bool fa) {
-	const uint32_t n = l.vertex_count;
-	f3 verts[kMaxPolygonVertices];
-#pragma unroll
-	for (int j = 0; j != kMaxLightVertices; ++j)
-		if (j < (int) n) verts[j] = mul_point(w2l, l.v[j]);
-	const uint32_t vc = clip_polygon<P>(n, verts);
-	if (vc != 0) prepare_psa<P>(p, vc, verts, fa);
+RL_DEV uint32_t prepare_space_record(const mat43& w2l, const float4* record, uint32_t n, PsaPolygon& p, bool fa) {
+	uint32_t mask = 0;  // bit j: vertex j above the horizon
+	float4 q = __ldg(record + kRecordVertex);
+#pragma unroll 1
+	for (uint32_t j = 0; j != n; ++j) {
+		const f3 v = mul_point(w2l, mk3(q.x, q.y, q.z));
+		q = __ldg(record + kRecordVertex + min(j + 1, (uint32_t) kMaxLightVertices - 1));
+		set_psa_vertex(p, j, v);
+		mask |= (v.z > 0.0f ? 1u : 0u) << j;
+	}
+	uint32_t vc = n;
+	if (mask != (1u << n) - 1u) {
+		if (mask == 0) return 0;
+		const uint32_t k = __popc(mask), s = clip_run_start(n, mask);
+		if (s == n) return 0;
+		const uint32_t e = clip_wrap(s + k - 1, n);
+		const f3 entry = iz0<P>(psa_vertex(p, clip_wrap(s + n - 1, n)), psa_vertex(p, s));
+		const f3 exit = iz0<P>(psa_vertex(p, e), psa_vertex(p, clip_wrap(e + 1, n)));
+		vc = k + 2;
+		const uint32_t r = clip_rotation(n, k, s);
+#pragma unroll 1
+		for (uint32_t slot = 0; slot != vc; ++slot) {
+			const uint32_t j = clip_wrap(slot + vc - r, vc);
+			f3 v = j == 0 ? entry : exit;
+			if (j != 0 && j != k + 1) {
+				const float4 w = __ldg(record + kRecordVertex + clip_wrap(s + j - 1, n));
+				v = mul_point(w2l, mk3(w.x, w.y, w.z));
+			}
+			set_psa_vertex(p, slot, v);
+		}
+	}
+	prepare_psa_loaded<P>(p, vc, fa);
 	return vc;
 }
 
-// prepare_space with the vertices read from the light's device record
-// (the same values as load_light gives), so that callers need not keep a
-// Light in memory for the call.  Inlined: its one caller runs it in a loop
-// over the two spaces, so the code is not duplicated, and an out-of-line call
-// saved the caller's live registers to local memory (sample kernel 3.98 ->
-// 3.79 ms per 4-frame 1080p launch inlined).
+// The same out of line, for the kernels that prepare both spaces at once.
 template <class P>
-RL_DEV uint32_t prepare_space_record(const mat43& w2l, const float4* record, PsaPolygon& p, bool fa) {
-	const uint32_t n = __float_as_uint(__ldg(record).w);
-	f3 verts[kMaxPolygonVertices];
-#pragma unroll
-	for (int j = 0; j != kMaxLightVertices; ++j) {
-		if (j < (int) n) {
-			const float4 q = __ldg(record + kRecordVertex + j);
-			verts[j] = mul_point(w2l, mk3(q.x, q.y, q.z));
-		}
-	}
-	const uint32_t vc = clip_polygon<P>(n, verts);
-	if (vc != 0) prepare_psa<P>(p, vc, verts, fa);
-	return vc;
+__device__ __noinline__ uint32_t prepare_space(mat43 w2l, const float4* record, uint32_t n, PsaPolygon& p, bool fa) {
+	return prepare_space_record<P>(w2l, record, n, p, fa);
 }
 
 // The side flip and both polygons' PSA sampling preparations of
@@ -334,12 +346,13 @@ RL_DEV uint32_t prepare_space_record(const mat43& w2l, const float4* record, Psa
 // is zero (the polygon clips to nothing or has no projected solid angle in
 // shading space).
 template <class P>
-RL_DEV bool psa_prepare_both(const ShadeParams& pr, const ShadingData& sd, Ltc& ltc, const Light& l, PsaPolygon& pd,
-                             PsaPolygon& ps) {
+RL_DEV bool psa_prepare_both(const ShadeParams& pr, const ShadingData& sd, Ltc& ltc, const Light& l,
+                             const float4* record, PsaPolygon& pd, PsaPolygon& ps) {
 	const bool fa = pr.fast_atan != 0;
 	side_flip(ltc, sd, l);
-	if (prepare_space<P>(ltc.world_to_shading, l, pd, fa) == 0) return false;
-	if (prepare_space<P>(mul(ltc.shading_to_cosine, ltc.world_to_shading), l, ps, fa) == 0) ps.psa = 0.0f;
+	const uint32_t n = l.vertex_count;
+	if (prepare_space<P>(ltc.world_to_shading, record, n, pd, fa) == 0) return false;
+	if (prepare_space<P>(mul(ltc.shading_to_cosine, ltc.world_to_shading), record, n, ps, fa) == 0) ps.psa = 0.0f;
 	return pd.psa != 0.0f;
 }
 
@@ -349,14 +362,15 @@ RL_DEV bool psa_prepare_both(const ShadeParams& pr, const ShadingData& sd, Ltc& 
 // one index fall in distinct banks; in local memory the resident warps'
 // buffers did not stay in L1.
 constexpr int kShadeThreads = 128;
-// pd and ps are the thread's two polygon buffers.
+// l is the light whose device record is `record`; pd and ps are the thread's
+// two polygon buffers.
 template <class P>
-RL_DEV f3 psa_mis_shade(const ShadeParams& pr, const ShadingData& sd, Ltc ltc, const Light& l, uint32_t& seed,
+RL_DEV f3 psa_mis_shade(const ShadeParams& pr, const ShadingData& sd, Ltc ltc, const Light& l, const float4* record, uint32_t& seed,
                         bool peters, bool visibility_in, PsaPolygon& pd, PsaPolygon& ps) {
 	const bool fa = pr.fast_atan != 0;
 	const bool biased = pr.technique == sample_polygon_projected_solid_angle_biased;
 	f3 result = splat(0.0f);
-	if (!psa_prepare_both<P>(pr, sd, ltc, l, pd, ps)) return result;
+	if (!psa_prepare_both<P>(pr, sd, ltc, l, record, pd, ps)) return result;
 	float specular_weight = ltc.albedo * ps.psa;
 	f3 diffuse_weight = scale(max3(sd.diffuse_albedo, splat(0.01f)), pd.psa);
 	int technique_count = (ps.psa > 0.0f) ? 2 : 1;
@@ -484,7 +498,7 @@ RL_DEV f3 shade_pixel(const ShadeParams& pr, const ShadingData& sd, const Ltc& l
 			load_light(pr.scene, idx, l);
 			bool visibility = true;
 			const f3 shade = area_turk ? area_turk_shade<P>(pr, sd, l, light_sample, false, visibility, seed)
-			                           : psa_mis_shade<P>(pr, sd, ltc, l, seed, peters, true, pd, ps);
+			                           : psa_mis_shade<P>(pr, sd, ltc, l, light_record(pr.scene, idx), seed, peters, true, pd, ps);
 			f3 r = scale(shade, (float) n);
 			float ls = (float) pr.light_samples;
 			r = mk3(P::div(r.x, ls), P::div(r.y, ls), P::div(r.z, ls));
@@ -510,7 +524,7 @@ RL_DEV f3 shade_pixel(const ShadeParams& pr, const ShadingData& sd, const Ltc& l
 					bool dummy_visibility = false;
 					color = area_turk_shade<C>(pr, sd, l, light_sample, false, dummy_visibility, seed);
 				} else {
-					color = psa_mis_shade<C>(pr, sd, ltc, l, seed, false, false, pd, ps);
+					color = psa_mis_shade<C>(pr, sd, ltc, l, light_record(pr.scene, idx), seed, false, false, pd, ps);
 				}
 				float p_hat = C::sqrt(dot(color, color));
 				float w = C::div(p_hat, p);
@@ -533,7 +547,7 @@ RL_DEV f3 shade_pixel(const ShadeParams& pr, const ShadingData& sd, const Ltc& l
 				load_light(pr.scene, res_index, l);
 				bool visibility = true;
 				const f3 color = area_turk ? area_turk_shade<P>(pr, sd, l, res_light_sample, true, visibility, seed)
-				                           : psa_mis_shade<P>(pr, sd, ltc, l, seed, peters, true, pd, ps);
+				                           : psa_mis_shade<P>(pr, sd, ltc, l, light_record(pr.scene, res_index), seed, peters, true, pd, ps);
 				float W = P::div(w_sum, (float) m * sample_value);
 				// The area technique has no p_hat == 0 guard but multiplies by
 				// the traced visibility (shading_pass.frag.glsl:749-756).

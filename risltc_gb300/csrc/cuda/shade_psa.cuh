@@ -148,17 +148,29 @@ RL_DEV void sort_convex_polygon_vertices(PsaPolygon& p) {
 	compare_and_swap(p, 0, 1);
 }
 
-// prepare_projected_solid_angle_polygon_sampling, polygon_sampling.glsl:545-613
-template <class P> RL_DEV void prepare_psa(PsaPolygon& p, uint32_t vc, const f3 v[kMaxPolygonVertices], bool fa) {
+// prepare_projected_solid_angle_polygon_sampling, polygon_sampling.glsl:545-613.
+// prepare_psa_loaded takes the polygon's vertices from p itself: x and y in
+// p.vertices, z in p.sector_psa (whose own values come last).
+RL_DEV f3 psa_vertex(const PsaPolygon& p, uint32_t i) {
+	const f2 v = p.vertices[i];
+	return mk3(v.x, v.y, p.sector_psa[i]);
+}
+RL_DEV void set_psa_vertex(PsaPolygon& p, uint32_t i, f3 v) {
+	p.vertices[i] = mk2(v.x, v.y);
+	p.sector_psa[i] = v.z;
+}
+template <class P> RL_DEV void prepare_psa_loaded(PsaPolygon& p, uint32_t vc, bool fa) {
 	p.vertex_count = vc;
 	p.inner_ellipse_0 = mk2(1.0f, 0.0f);
-	p.vertices[0] = mk2(v[0].x, v[0].y);
-	p.ellipses[0] = ellipse_from_edge<P>(v[0], v[1]);
+	const f3 v0 = psa_vertex(p, 0);
+	f3 v = psa_vertex(p, 1);
+	p.ellipses[0] = ellipse_from_edge<P>(v0, v);
 	f2 previous = p.ellipses[0];
 #pragma unroll 1
 	for (uint32_t i = 1; i != vc; ++i) {
-		p.vertices[i] = mk2(v[i].x, v[i].y);
-		f2 e = ellipse_from_edge<P>(v[i], v[(i + 1 == vc) ? 0 : i + 1]);
+		const f3 next = i + 1 == vc ? v0 : psa_vertex(p, i + 1);
+		f2 e = ellipse_from_edge<P>(v, next);
+		v = next;
 		bool inner = is_inner_ellipse(e);
 		p.ellipses[i] = inner ? previous : e;
 		p.inner_ellipse_0 = (is_inner_ellipse(previous) && !inner) ? previous : p.inner_ellipse_0;
@@ -201,6 +213,12 @@ template <class P> RL_DEV void prepare_psa(PsaPolygon& p, uint32_t vc, const f3 
 			p.psa += p.sector_psa[i];
 		}
 	}
+}
+
+template <class P> RL_DEV void prepare_psa(PsaPolygon& p, uint32_t vc, const f3 v[kMaxPolygonVertices], bool fa) {
+#pragma unroll 1
+	for (uint32_t i = 0; i != vc; ++i) set_psa_vertex(p, i, v[i]);
+	prepare_psa_loaded<P>(p, vc, fa);
 }
 
 // normalize_approx_and_flip, polygon_sampling.glsl:622-634
