@@ -119,6 +119,53 @@ RL_DEV void tc_load32(uint32_t taddr, uint32_t (&v)[32]) {
 	    : "r"(taddr));
 }
 
+// Row `row` of the encoded features (K-major, kMlpFeatures columns) from the
+// pixel's ten inputs, eight BF16 columns per 16-byte store; zeros where the
+// row holds no pixel.  Feature 130, the first padding one, is 1 with `ones`.
+// (One two-byte store per feature took a sixth of the logits call: 191
+// us at 960x540 with 256 clusters, 157 with these and the biases read
+// four at a time.)
+RL_DEV void mlp_encode_row(unsigned char* rows, int row, const float (&x)[kMlpInputs], bool in, bool ones) {
+	float low = 0.0f;
+	uint32_t words[4] = {0u, 0u, 0u, 0u};
+	auto put = [&](int f, float v) {  // f: compile-time constants, ascending
+		if ((f & 1) == 0) {
+			low = v;
+			return;
+		}
+		words[(f >> 1) & 3] = pack_bf16x2(low, v);
+		if ((f & 7) == 7)
+			*reinterpret_cast<uint4*>(rows + tc_offset(row, f - 7, kMlpFeatures)) =
+			    make_uint4(words[0], words[1], words[2], words[3]);
+	};
+#pragma unroll
+	for (int input = 0; input != kMlpInputs; ++input) {
+		float e[13];
+		mlp_encode(x[input], e);
+#pragma unroll
+		for (int kind = 0; kind != 13; ++kind) put(input * 13 + kind, in ? e[kind] : 0.0f);
+	}
+#pragma unroll
+	for (int f = kMlpInputs * 13; f != kMlpFeatures; ++f) put(f, ones && f == kMlpInputs * 13 ? 1.0f : 0.0f);
+}
+
+// Columns c .. c + 31 of row `row` of a hidden layer (K-major, k columns):
+// the accumulators v plus the bias (16-byte aligned), ReLU, BF16.
+RL_DEV void store_hidden(unsigned char* hidden, int row, int c, int k, const uint32_t (&v)[32], const float* bias) {
+#pragma unroll
+	for (int q = 0; q != 4; ++q) {
+		uint32_t o[4];
+#pragma unroll
+		for (int h = 0; h != 2; ++h) {
+			const float4 b = *reinterpret_cast<const float4*>(bias + c + 8 * q + 4 * h);
+			const int j = 8 * q + 4 * h;
+			o[2 * h] = pack_bf16x2(fmaxf(__uint_as_float(v[j]) + b.x, 0.0f), fmaxf(__uint_as_float(v[j + 1]) + b.y, 0.0f));
+			o[2 * h + 1] = pack_bf16x2(fmaxf(__uint_as_float(v[j + 2]) + b.z, 0.0f), fmaxf(__uint_as_float(v[j + 3]) + b.w, 0.0f));
+		}
+		*reinterpret_cast<uint4*>(hidden + tc_offset(row, c + 8 * q, k)) = make_uint4(o[0], o[1], o[2], o[3]);
+	}
+}
+
 // Shared memory of the kernel for k_count clusters: W1, W2, W3 (rows padded
 // to a multiple of 16; together the operand-layout weights of one bulk copy),
 // A1, A2, the biases, three mbarriers (products, weights, inputs) and the
@@ -240,18 +287,7 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 			uint32_t v[32];
 			tc_load32(d12 + lane_base + (uint32_t) c, v);
 			tc_wait_load();
-#pragma unroll
-			for (int q = 0; q != 4; ++q) {
-				uint4 out;
-				uint32_t* o = &out.x;
-#pragma unroll
-				for (int h = 0; h != 4; ++h) {
-					const int j = 8 * q + 2 * h;
-					o[h] = pack_bf16x2(fmaxf(__uint_as_float(v[j]) + bias[c + j], 0.0f),
-					                   fmaxf(__uint_as_float(v[j + 1]) + bias[c + j + 1], 0.0f));
-				}
-				*reinterpret_cast<uint4*>(tc_smem + tl.a2 + tc_offset((int) tid, c + 8 * q, kMlpHidden)) = out;
-			}
+			store_hidden(tc_smem + tl.a2, (int) tid, c, kMlpHidden, v, bias);
 		}
 		fence_async_shared();
 		tc_fence_before();
@@ -266,30 +302,22 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 			if (failed) break;
 			++inputs_waited;
 		}
-		// Encode the tile's pixels into A1.
-		for (int idx = tid; idx < kTcRows * kMlpInputs; idx += kTcThreads) {
-			const int r = idx / kMlpInputs, input = idx % kMlpInputs;
-			const uint32_t i = p0 + (uint32_t) r;
-			float x = 0.0f;
-			if (i < np) {
-				if (bulk_inputs) {
-					x = inputs[input * kTcRows + r];
-					if (input < 3) x = (x - pr.center[input]) * pr.inv_half_extent;
-				} else {
-					x = mlp_input(pr.gbuffer, np, i, pr.center, pr.inv_half_extent, input);
+		// Encode the tile's pixels into A1: thread tid takes row tid.
+		{
+			const uint32_t i = p0 + tid;
+			float x[kMlpInputs];
+#pragma unroll
+			for (int input = 0; input != kMlpInputs; ++input) {
+				x[input] = 0.0f;
+				if (i < np && bulk_inputs) {
+					x[input] = inputs[input * kTcRows + tid];
+					if (input < 3) x[input] = (x[input] - pr.center[input]) * pr.inv_half_extent;
+				} else if (i < np) {
+					x[input] = mlp_input(pr.gbuffer, np, i, pr.center, pr.inv_half_extent, input);
 				}
 			}
-			float e[13];
-			mlp_encode(x, e);
-#pragma unroll
-			for (int kind = 0; kind != 13; ++kind)
-				*reinterpret_cast<__nv_bfloat16*>(tc_smem + tl.a1 + tc_offset(r, input * 13 + kind, kMlpFeatures)) =
-				    __float2bfloat16_rn(i < np ? e[kind] : 0.0f);
+			mlp_encode_row(tc_smem + tl.a1, (int) tid, x, i < np, false);
 		}
-		for (int idx = tid; idx < kTcRows * (kMlpFeatures - 130); idx += kTcThreads)
-			*reinterpret_cast<__nv_bfloat16*>(
-			    tc_smem + tl.a1 + tc_offset(idx / (kMlpFeatures - 130), 130 + idx % (kMlpFeatures - 130), kMlpFeatures)) =
-			    __float2bfloat16_rn(0.0f);
 		fence_async_shared();
 		tc_fence_before();
 		__syncthreads();
@@ -337,10 +365,11 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 						uint4 out;
 						uint32_t* o = &out.x;
 #pragma unroll
-						for (int h = 0; h != 4; ++h) {
-							const int j = 8 * q + 2 * h;
-							o[h] = pack_bf16x2(__uint_as_float(v[j]) + b3[c0 + c + j],
-							                   __uint_as_float(v[j + 1]) + b3[c0 + c + j + 1]);
+						for (int h = 0; h != 2; ++h) {
+							const float4 b = *reinterpret_cast<const float4*>(b3 + j0 + 4 * h);
+							const int j = 8 * q + 4 * h;
+							o[2 * h] = pack_bf16x2(__uint_as_float(v[j]) + b.x, __uint_as_float(v[j + 1]) + b.y);
+							o[2 * h + 1] = pack_bf16x2(__uint_as_float(v[j + 2]) + b.z, __uint_as_float(v[j + 3]) + b.w);
 						}
 						if (!kF32) {
 							*reinterpret_cast<uint4*>(pr.logits + at + 8 * q) = out;

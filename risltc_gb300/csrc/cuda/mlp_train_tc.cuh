@@ -73,6 +73,85 @@ RL_DEV void tc_load16(uint32_t taddr, uint32_t (&v)[16]) {
 RL_DEV float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 RL_DEV float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
+// A training pixel's candidates: the first kHeld of them read once, all loads
+// in flight together, while layer 1 runs (their clusters, too, are then there
+// when the targets are subtracted; re-read in groups of eight, each group
+// waited for memory twice), the rest read where they are needed.
+struct HeldCandidates {
+	static constexpr int kHeld = 32;
+	static constexpr uint32_t kNone = 0xffffffffu;
+	float weight[kHeld];
+	uint32_t cluster[kHeld];  // kNone: no target
+
+	RL_DEV static uint32_t cluster_of(const MlpTrainParams& pr, int light, float w) {
+		return w > 0.0f && (uint32_t) light < pr.light_count ? pr.light_cluster[light] : kNone;
+	}
+	// Returns the total candidate weight (0 where there is no pixel).
+	RL_DEV float load(const ProposalCandidate* cand, int count, bool valid, const MlpTrainParams& pr) {
+		int light[kHeld];
+#pragma unroll
+		for (int c = 0; c != kHeld; ++c) {
+			light[c] = -1;
+			weight[c] = 0.0f;
+			if (valid && c < count) {
+				light[c] = __ldg(&cand[c].light);  // the caller's records may be 4-byte aligned
+				weight[c] = __ldg(&cand[c].pdf);
+			}
+		}
+#pragma unroll
+		for (int c = 0; c != kHeld; ++c) cluster[c] = cluster_of(pr, light[c], weight[c]);
+		float total = 0.0f;
+#pragma unroll
+		for (int c = 0; c != kHeld; ++c)
+			if (c < count) total += weight[c];
+		if (valid) {
+#pragma unroll 8
+			for (int c = kHeld; c < count; ++c) total += cand[c].pdf;
+		}
+		return total;
+	}
+	// target(cluster, weight) of every candidate that has one, in order.
+	template <class Target>
+	RL_DEV void each(const ProposalCandidate* cand, int count, const MlpTrainParams& pr, Target target) const {
+#pragma unroll
+		for (int c = 0; c != kHeld; ++c)
+			if (cluster[c] != kNone) target(cluster[c], weight[c]);
+#pragma unroll 1
+		for (int c = kHeld; c < count; ++c) {
+			const ProposalCandidate q = cand[c];
+			const uint32_t k = cluster_of(pr, q.light, q.pdf);
+			if (k != kNone) target(k, q.pdf);
+		}
+	}
+};
+
+// Adds `weights` of the `columns` FP32 columns of this thread's tensor-memory
+// lane to the gradient at w (16-byte aligned, four per reduction) and the next
+// column to *b; the rest is padding.  All threads call it; those without
+// `active` add nothing.
+RL_DEV void add_gradient(uint32_t taddr, int columns, float* w, int weights, float* b, bool active) {
+	for (int col = 0; col != columns; col += 16) {
+		uint32_t v[16];
+		tc_load16(taddr + (uint32_t) col, v);
+		tc_wait_load();
+		if (!active) continue;
+#pragma unroll
+		for (int q = 0; q != 16; q += 4) {
+			const float4 g = make_float4(__uint_as_float(v[q]), __uint_as_float(v[q + 1]), __uint_as_float(v[q + 2]),
+			                             __uint_as_float(v[q + 3]));
+			const int f = col + q;
+			if (f + 4 <= weights) {
+				if (g.x != 0.0f || g.y != 0.0f || g.z != 0.0f || g.w != 0.0f) atomicAdd(reinterpret_cast<float4*>(w + f), g);
+				continue;
+			}
+			const float one[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+			for (int k = 0; k != 4; ++k)
+				if (f + k <= weights && one[k] != 0.0f) atomicAdd(f + k < weights ? w + f + k : b, one[k]);
+		}
+	}
+}
+
 static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_kernel(MlpTrainParams pr) {
 	extern __shared__ __align__(1024) unsigned char tt_smem[];
 	const int k_count = pr.k_count;
@@ -150,18 +229,7 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_kernel(MlpT
 			uint32_t v[32];
 			tc_load32(tmem + lane_base + (uint32_t) c, v);
 			tc_wait_load();
-#pragma unroll
-			for (int q = 0; q != 4; ++q) {
-				uint4 out;
-				uint32_t* o = &out.x;
-#pragma unroll
-				for (int k = 0; k != 4; ++k) {
-					const int j = 8 * q + 2 * k;
-					o[k] = pack_bf16x2(fmaxf(__uint_as_float(v[j]) + bias[c + j], 0.0f),
-					                   fmaxf(__uint_as_float(v[j + 1]) + bias[c + j + 1], 0.0f));
-				}
-				*reinterpret_cast<uint4*>(tt_smem + h + tc_offset((int) tid, c + 8 * q, kTtHiddenCols)) = out;
-			}
+			store_hidden(tt_smem + h, (int) tid, c, kTtHiddenCols, v, bias);
 		}
 		sync_for_products();
 	};
@@ -201,19 +269,7 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_kernel(MlpT
 #pragma unroll
 			for (int input = 0; input != kMlpInputs; ++input)
 				x[input] = in ? mlp_input(pr.gbuffer, np, my_i, pr.center, pr.inv_half_extent, input) : 0.0f;
-#pragma unroll
-			for (int input = 0; input != kMlpInputs; ++input) {
-				float e[13];
-				mlp_encode(x[input], e);
-#pragma unroll
-				for (int kind = 0; kind != 13; ++kind)
-					*reinterpret_cast<__nv_bfloat16*>(tt_smem + kTtE + tc_offset((int) tid, input * 13 + kind, kMlpFeatures)) =
-					    __float2bfloat16_rn(in ? e[kind] : 0.0f);
-			}
-#pragma unroll
-			for (int f = kTtOnesFeature; f != kMlpFeatures; ++f)
-				*reinterpret_cast<__nv_bfloat16*>(tt_smem + kTtE + tc_offset((int) tid, f, kMlpFeatures)) =
-				    __float2bfloat16_rn(f == kTtOnesFeature ? 1.0f : 0.0f);
+			mlp_encode_row(tt_smem + kTtE, (int) tid, x, in, true);
 		}
 		sync_for_products();
 		issue([&] {
@@ -224,11 +280,8 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_kernel(MlpT
 		// While layer 1 runs: the total candidate weight of this thread's pixel.
 		const ProposalCandidate* cand = pr.candidates + (size_t) my_i * mc;
 		const bool valid = in && !(pr.primitive && pr.primitive[my_i] == 0xffffffffu);
-		float total = 0.0f;
-		if (valid) {
-#pragma unroll 8
-			for (int c = 0; c < mc; ++c) total += cand[c].pdf;
-		}
+		HeldCandidates held;
+		const float total = held.load(cand, mc, valid, pr);
 		const bool learn = valid && total > 0.0f && total <= 3.0e38f;
 		const float wu = pr.shaded ? 1.0f - pr.shadowed_weight : 1.0f;
 		float ss = 0.0f;
@@ -312,15 +365,10 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_kernel(MlpT
 		// into their clusters, the shadowed part into the chosen light's.
 		if (learn) {
 			const float unshadowed = wu / total * pr.inv_batch;
-#pragma unroll 8
-			for (int c = 0; c < mc; ++c) {
-				const ProposalCandidate q = cand[c];
-				if (q.pdf > 0.0f && (uint32_t) q.light < pr.light_count) {
-					__nv_bfloat16* z = reinterpret_cast<__nv_bfloat16*>(
-					    tt_smem + kTtDz + tc_offset((int) tid, (int) pr.light_cluster[q.light], k_pad));
-					*z = __float2bfloat16_rn(__bfloat162float(*z) - unshadowed * q.pdf);
-				}
-			}
+			held.each(cand, mc, pr, [&](uint32_t cluster, float weight) {
+				__nv_bfloat16* z = reinterpret_cast<__nv_bfloat16*>(tt_smem + kTtDz + tc_offset((int) tid, (int) cluster, k_pad));
+				*z = __float2bfloat16_rn(__bfloat162float(*z) - unshadowed * weight);
+			});
 			if (chosen >= 0 && (uint32_t) chosen < pr.light_count && ss > 0.0f) {
 				__nv_bfloat16* z = reinterpret_cast<__nv_bfloat16*>(
 				    tt_smem + kTtDz + tc_offset((int) tid, (int) pr.light_cluster[chosen], k_pad));
@@ -373,46 +421,13 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_kernel(MlpT
 		// Lane tid of each accumulator: cluster (dW3) or hidden unit (dW2, dW1).
 		for (int ch = 0; ch != chunks; ++ch) {
 			const int c = ch * kTcChunk + (int) tid;
-			for (int col = 0; col != kTtHiddenCols; col += 16) {
-				uint32_t v[16];
-				tc_load16(tmem + lane_base + kTtGrad3 + 80 * ch + (uint32_t) col, v);
-				tc_wait_load();
-				if (c >= k_count) continue;
-#pragma unroll
-				for (int q = 0; q != 16; ++q) {
-					const float g = __uint_as_float(v[q]);
-					const int f = col + q;
-					if (g == 0.0f || f > kMlpHidden) continue;
-					atomicAdd(pr.grad + (f < kMlpHidden ? lay.w3 + c * kMlpHidden + f : lay.b3 + c), g);
-				}
-			}
+			add_gradient(tmem + lane_base + kTtGrad3 + 80 * ch, kTtHiddenCols, pr.grad + lay.w3 + (size_t) c * kMlpHidden,
+			             kMlpHidden, pr.grad + lay.b3 + c, c < k_count);
 		}
-		for (int col = 0; col != kTtHiddenCols; col += 16) {
-			uint32_t v[16];
-			tc_load16(tmem + lane_base + kTtGrad2 + (uint32_t) col, v);
-			tc_wait_load();
-			if (tid >= (uint32_t) kMlpHidden) continue;
-#pragma unroll
-			for (int q = 0; q != 16; ++q) {
-				const float g = __uint_as_float(v[q]);
-				const int f = col + q;
-				if (g == 0.0f || f > kMlpHidden) continue;
-				atomicAdd(pr.grad + (f < kMlpHidden ? lay.w2 + (int) tid * kMlpHidden + f : lay.b2 + (int) tid), g);
-			}
-		}
-		for (int col = 0; col != kMlpFeatures; col += 16) {
-			uint32_t v[16];
-			tc_load16(tmem + lane_base + kTtGrad1 + (uint32_t) col, v);
-			tc_wait_load();
-			if (tid >= (uint32_t) kMlpHidden) continue;
-#pragma unroll
-			for (int q = 0; q != 16; ++q) {
-				const float g = __uint_as_float(v[q]);
-				const int f = col + q;
-				if (g == 0.0f || f > kTtOnesFeature) continue;
-				atomicAdd(pr.grad + (f < kTtOnesFeature ? lay.w1 + (int) tid * kMlpFeatures + f : lay.b1 + (int) tid), g);
-			}
-		}
+		add_gradient(tmem + lane_base + kTtGrad2, kTtHiddenCols, pr.grad + lay.w2 + (int) tid * kMlpHidden, kMlpHidden,
+		             pr.grad + lay.b2 + (int) tid, tid < (uint32_t) kMlpHidden);
+		add_gradient(tmem + lane_base + kTtGrad1, kMlpFeatures, pr.grad + lay.w1 + (int) tid * kMlpFeatures, kTtOnesFeature,
+		             pr.grad + lay.b1 + (int) tid, tid < (uint32_t) kMlpHidden);
 	}
 	if (failed) {
 		if (tid == 0) atomicOr(pr.error, kErrorTensorWait);

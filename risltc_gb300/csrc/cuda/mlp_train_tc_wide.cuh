@@ -152,18 +152,7 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_wide_kernel
 			uint32_t v[32];
 			tc_load32(tmem + lane_base + (uint32_t) c, v);
 			tc_wait_load();
-#pragma unroll
-			for (int q = 0; q != 4; ++q) {
-				uint4 out;
-				uint32_t* o = &out.x;
-#pragma unroll
-				for (int k = 0; k != 4; ++k) {
-					const int j = 8 * q + 2 * k;
-					o[k] = pack_bf16x2(fmaxf(__uint_as_float(v[j]) + bias[c + j], 0.0f),
-					                   fmaxf(__uint_as_float(v[j + 1]) + bias[c + j + 1], 0.0f));
-				}
-				*reinterpret_cast<uint4*>(tw_smem + h + tc_offset((int) tid, c + 8 * q, kTtHiddenCols)) = out;
-			}
+			store_hidden(tw_smem + h, (int) tid, c, kTtHiddenCols, v, bias);
 		}
 		sync_for_products();
 	};
@@ -209,19 +198,7 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_wide_kernel
 #pragma unroll
 			for (int input = 0; input != kMlpInputs; ++input)
 				x[input] = in ? mlp_input(pr.gbuffer, np, my_i, pr.center, pr.inv_half_extent, input) : 0.0f;
-#pragma unroll
-			for (int input = 0; input != kMlpInputs; ++input) {
-				float e[13];
-				mlp_encode(x[input], e);
-#pragma unroll
-				for (int kind = 0; kind != 13; ++kind)
-					*reinterpret_cast<__nv_bfloat16*>(tw_smem + kTwE + tc_offset((int) tid, input * 13 + kind, kMlpFeatures)) =
-					    __float2bfloat16_rn(in ? e[kind] : 0.0f);
-			}
-#pragma unroll
-			for (int f = kTtOnesFeature; f != kMlpFeatures; ++f)
-				*reinterpret_cast<__nv_bfloat16*>(tw_smem + kTwE + tc_offset((int) tid, f, kMlpFeatures)) =
-				    __float2bfloat16_rn(f == kTtOnesFeature ? 1.0f : 0.0f);
+			mlp_encode_row(tw_smem + kTwE, (int) tid, x, in, true);
 		}
 		sync_for_products();
 		issue([&] {
@@ -232,11 +209,8 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_wide_kernel
 		// While layer 1 runs: the total candidate weight of this thread's pixel.
 		const ProposalCandidate* cand = pr.candidates + (size_t) my_i * mc;
 		const bool valid = in && !(pr.primitive && pr.primitive[my_i] == 0xffffffffu);
-		float total = 0.0f;
-		if (valid) {
-#pragma unroll 8
-			for (int c = 0; c < mc; ++c) total += cand[c].pdf;
-		}
+		HeldCandidates held;
+		const float total = held.load(cand, mc, valid, pr);
 		const bool learn = valid && total > 0.0f && total <= 3.0e38f;
 		const float wu = pr.shaded ? 1.0f - pr.shadowed_weight : 1.0f;
 		float ss = 0.0f;
@@ -333,16 +307,13 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_wide_kernel
 			}
 			if (learn) {
 				const float unshadowed = wu / total * pr.inv_batch;
-				for (int c = 0; c < mc; ++c) {
-					const ProposalCandidate q = cand[c];
-					if (q.pdf > 0.0f && (uint32_t) q.light < pr.light_count) {
-						const int cl = (int) pr.light_cluster[q.light] - c0;
-						if (cl >= 0 && cl < n) {
-							__nv_bfloat16* zp = reinterpret_cast<__nv_bfloat16*>(tw_smem + kTwDz + tc_offset((int) tid, cl, kTcChunk));
-							*zp = __float2bfloat16_rn(__bfloat162float(*zp) - unshadowed * q.pdf);
-						}
+				held.each(cand, mc, pr, [&](uint32_t cluster, float weight) {
+					const uint32_t cl = cluster - (uint32_t) c0;
+					if (cl < (uint32_t) n) {
+						__nv_bfloat16* zp = reinterpret_cast<__nv_bfloat16*>(tw_smem + kTwDz + tc_offset((int) tid, (int) cl, kTcChunk));
+						*zp = __float2bfloat16_rn(__bfloat162float(*zp) - unshadowed * weight);
 					}
-				}
+				});
 				if (chosen >= 0 && (uint32_t) chosen < pr.light_count && ss > 0.0f) {
 					const int cl = (int) pr.light_cluster[chosen] - c0;
 					if (cl >= 0 && cl < n) {
@@ -368,23 +339,8 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_wide_kernel
 			// Lane tid of dW3_c: cluster c0 + tid; weights and bias added to
 			// the gradient (16-byte aligned rows of 64 floats).
 			const int cl = c0 + (int) tid;
-			for (int col = 0; col != kTtHiddenCols; col += 16) {
-				uint32_t v[16];
-				tc_load16(tmem + lane_base + kTwGrad3 + (uint32_t) col, v);
-				tc_wait_load();
-				if (cl >= k_count) continue;
-				if (col < kMlpHidden) {
-					float4* g = reinterpret_cast<float4*>(pr.grad + lay.w3 + (size_t) cl * kMlpHidden + col);
-#pragma unroll
-					for (int q = 0; q != 4; ++q) {
-						const float4 a = make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]),
-						                             __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]));
-						if (a.x != 0.0f || a.y != 0.0f || a.z != 0.0f || a.w != 0.0f) atomicAdd(g + q, a);
-					}
-				} else if (__uint_as_float(v[0]) != 0.0f) {
-					atomicAdd(pr.grad + lay.b3 + cl, __uint_as_float(v[0]));
-				}
-			}
+			add_gradient(tmem + lane_base + kTwGrad3, kTtHiddenCols, pr.grad + lay.w3 + (size_t) cl * kMlpHidden, kMlpHidden,
+			             pr.grad + lay.b3 + cl, cl < k_count);
 			tc_fence_before();
 			__syncthreads();
 			tc_fence_after();
@@ -415,32 +371,10 @@ static __global__ void __launch_bounds__(kTcThreads, 1) mlp_train_tc_wide_kernel
 		accumulated = true;
 	}
 	if (!failed && accumulated) {
-		for (int col = 0; col != kTtHiddenCols; col += 16) {
-			uint32_t v[16];
-			tc_load16(tmem + lane_base + kTwGrad2 + (uint32_t) col, v);
-			tc_wait_load();
-			if (tid >= (uint32_t) kMlpHidden) continue;
-#pragma unroll
-			for (int q = 0; q != 16; ++q) {
-				const float g = __uint_as_float(v[q]);
-				const int f = col + q;
-				if (g == 0.0f || f > kMlpHidden) continue;
-				atomicAdd(pr.grad + (f < kMlpHidden ? lay.w2 + (int) tid * kMlpHidden + f : lay.b2 + (int) tid), g);
-			}
-		}
-		for (int col = 0; col != kMlpFeatures; col += 16) {
-			uint32_t v[16];
-			tc_load16(tmem + lane_base + kTwGrad1 + (uint32_t) col, v);
-			tc_wait_load();
-			if (tid >= (uint32_t) kMlpHidden) continue;
-#pragma unroll
-			for (int q = 0; q != 16; ++q) {
-				const float g = __uint_as_float(v[q]);
-				const int f = col + q;
-				if (g == 0.0f || f > kTtOnesFeature) continue;
-				atomicAdd(pr.grad + (f < kTtOnesFeature ? lay.w1 + (int) tid * kMlpFeatures + f : lay.b1 + (int) tid), g);
-			}
-		}
+		add_gradient(tmem + lane_base + kTwGrad2, kTtHiddenCols, pr.grad + lay.w2 + (int) tid * kMlpHidden, kMlpHidden,
+		             pr.grad + lay.b2 + (int) tid, tid < (uint32_t) kMlpHidden);
+		add_gradient(tmem + lane_base + kTwGrad1, kMlpFeatures, pr.grad + lay.w1 + (int) tid * kMlpFeatures, kTtOnesFeature,
+		             pr.grad + lay.b1 + (int) tid, tid < (uint32_t) kMlpHidden);
 	}
 	if (failed) {
 		if (tid == 0) atomicOr(pr.error, kErrorTensorWait);
