@@ -82,16 +82,25 @@ RL_DEV int cdf_slot(int k) { return k + (k >> 3); }
 
 // The noise stream of candidate c of a pixel-frame: the pixel's accessor for
 // the frame's second noise number, decorrelated per candidate.
-RL_DEV uint32_t proposal_stream(uint32_t x, uint32_t y, uint32_t width, uint32_t noise_seed, uint32_t f,
-                                uint32_t animate, uint32_t c) {
-	const uint32_t rn = animate ? wang_random_number((noise_seed + f) * 4u + 1u) : 0x123456u;
-	return get_noise_accessor(x, y, width, rn) ^ (c * 0x9E3779B9u);
+RL_DEV uint32_t proposal_number(uint32_t noise_seed, uint32_t f, uint32_t animate) {
+	return animate ? wang_random_number((noise_seed + f) * 4u + 1u) : 0x123456u;
+}
+// pixel: its index in the frame (x + y * width).
+RL_DEV uint32_t proposal_stream(uint32_t pixel, uint32_t number, uint32_t c) {
+	return get_noise_accessor(pixel, 0u, 0u, number) ^ (c * 0x9E3779B9u);
 }
 
 // Words of one warp's cumulative weights in shared memory (with the pads).
 __host__ __device__ inline int proposal_cdf_words(int cluster_count) { return cluster_count + (cluster_count >> 3) + 1; }
 
-static __global__ void __launch_bounds__(32 * kProposalWarps) proposal_kernel(ProposalParams pr) {
+// Blocks per SM the proposal kernel is compiled for (64 registers): learned
+// 4-frame 1080p call with 256 clusters 12.46 ms, against 12.78 with 6, 12.80
+// with 9 and 12.89 with 10.  Bound by issue and the latency of a pixel's chain
+// (two warp scans, the search); redux.sync for the maximum and two levels of
+// the search at a time changed nothing.
+constexpr int kProposalBlocks = 8;
+
+static __global__ void __launch_bounds__(32 * kProposalWarps, kProposalBlocks) proposal_kernel(ProposalParams pr) {
 	extern __shared__ float proposal_smem[];
 	const uint32_t lane = threadIdx.x % 32;
 	const int k_count = pr.clusters.count;
@@ -101,6 +110,18 @@ static __global__ void __launch_bounds__(32 * kProposalWarps) proposal_kernel(Pr
 	const int per_lane = (k_count + 31) / 32;
 	const float a = pr.uniform_fraction;
 	const int k0 = (int) lane * per_lane;  // this lane's block of clusters
+	// What does not change from pixel to pixel: which of the lane's first
+	// clusters are empty, the uniform part of a probability, and the frame,
+	// candidate, noise number and output offset of the lane's first draw.
+	uint32_t empty_mask = 0;
+#pragma unroll
+	for (int j = 0; j != kLogitCache; ++j)
+		if (j < per_lane && k0 + j < k_count && pr.clusters.size_lane[(uint32_t) j * 32 + lane] == 0) empty_mask |= 1u << j;
+	const float uniform_pdf = __frcp_rn((float) n_lights), uniform_part = __fdiv_rn(a, (float) n_lights);
+	const uint32_t per_frame = (uint32_t) pr.candidate_count, draws = pr.frame_count * per_frame;
+	const uint32_t first_f = lane / per_frame, first_c = lane % per_frame;
+	const uint32_t first_number = proposal_number(pr.noise_seed, first_f, pr.animate);
+	ProposalCandidate* const first_out = pr.out + (size_t) first_f * np * per_frame + first_c;
 	const uint32_t stride = gridDim.x * kProposalWarps;
 	// The next pixel's inputs are loaded while the current one is processed
 	// (software pipelining over the warp's pixels): its background flag, its
@@ -110,6 +131,11 @@ static __global__ void __launch_bounds__(32 * kProposalWarps) proposal_kernel(Pr
 		bool skip;
 		f3 x, n;
 		float logit[kLogitCache];
+	};
+	// The mixture's probability of a light of cluster k with `size` lights.
+	auto probability = [&](int k, uint32_t size, float total) -> float {
+		const float mass = cdf[cdf_slot(k)] - (k > 0 ? cdf[cdf_slot(k - 1)] : 0.0f);
+		return __fadd_rn(uniform_part, __fdiv_rn(__fmul_rn(1.0f - a, __fdiv_rn(mass, total)), (float) size));
 	};
 	auto fetch = [&](uint32_t p, Inputs& in) {
 		in.skip = pr.primitive && pr.primitive[p] == 0xffffffffu;
@@ -158,20 +184,21 @@ static __global__ void __launch_bounds__(32 * kProposalWarps) proposal_kernel(Pr
 				if (k0 + j < k_count) logit_max = fmaxf(logit_max, __bfloat162float(row[j]));
 			for (int d = 16; d != 0; d >>= 1) logit_max = fmaxf(logit_max, __shfl_xor_sync(0xffffffffu, logit_max, d));
 		}
+		// The lane's first clusters' inclusive sums stay in registers until the
+		// scan gives their offset; the rest goes through shared memory.
+		float below[kLogitCache];
 #pragma unroll
 		for (int j = 0; j != kLogitCache; ++j) {
-			const int k = k0 + j;
-			if (j < per_lane && k < k_count) {
+			if (j < per_lane && k0 + j < k_count) {
 				const uint32_t t = (uint32_t) j * 32 + lane;
-				const bool empty = pr.clusters.size_lane[t] == 0;
 				float w;
 				if (pr.logits)
-					w = empty ? 0.0f : __expf(cached[j] - logit_max);
+					w = __expf(cached[j] - logit_max);
 				else
-					w = empty ? 0.0f : cluster_weight(pr.clusters.bounds_lane[t], pr.clusters.power_lane[t], x, n);
-				local += w;
-				cdf[cdf_slot(k)] = local;
+					w = cluster_weight(pr.clusters.bounds_lane[t], pr.clusters.power_lane[t], x, n);
+				local += (empty_mask >> j & 1u) ? 0.0f : w;
 			}
+			below[j] = local;
 		}
 		for (int j = kLogitCache; j < per_lane; ++j) {
 			const int k = k0 + j;
@@ -195,57 +222,50 @@ static __global__ void __launch_bounds__(32 * kProposalWarps) proposal_kernel(Pr
 		float excl = __shfl_up_sync(0xffffffffu, incl, 1);
 		excl = lane == 0 ? 0.0f : excl;
 		const float total = __shfl_sync(0xffffffffu, incl, 31);
-		for (int j = 0; j != per_lane; ++j) {
+#pragma unroll
+		for (int j = 0; j != kLogitCache; ++j)
+			if (j < per_lane && k0 + j < k_count) cdf[cdf_slot(k0 + j)] = excl + below[j];
+		for (int j = kLogitCache; j < per_lane; ++j) {
 			const int k = k0 + j;
 			if (k >= k_count) break;
 			cdf[cdf_slot(k)] = excl + cdf[cdf_slot(k)];
 		}
 		__syncwarp();
 		const bool proposal = total > 0.0f && total <= 3.0e38f;
-		const uint32_t x_pix = i % pr.width, y_pix = i / pr.width;
-		const int per_frame = pr.candidate_count;
+		// One draw: its noise stream, light and probability.
+		auto draw = [&](uint32_t s) -> ProposalCandidate {
+			const float u0 = get_noise_1(s), u1 = get_noise_1(s), u2 = get_noise_1(s);
+			if (!proposal || u0 < a) {
+				int light = (int) (u1 * (float) n_lights);
+				light = light > n_lights - 1 ? n_lights - 1 : light;
+				if (!proposal) return ProposalCandidate{light, uniform_pdf};
+				const int k = (int) pr.clusters.light_cluster[light];
+				return ProposalCandidate{light, probability(k, pr.clusters.spans[k].y, total)};
+			}
+			// First cluster whose cumulative weight exceeds u1 * total.
+			const float t = u1 * total;
+			int lo = 0, hi = k_count - 1;
+			while (lo < hi) {
+				const int mid = (lo + hi) >> 1;
+				if (cdf[cdf_slot(mid)] > t)
+					hi = mid;
+				else
+					lo = mid + 1;
+			}
+			// Rounding can leave t at the top: take the last non-empty cluster.
+			uint2 span = pr.clusters.spans[lo];
+			while (lo > 0 && span.y == 0) span = pr.clusters.spans[--lo];
+			uint32_t j = (uint32_t) (u2 * (float) span.y);
+			j = j > span.y - 1 ? span.y - 1 : j;
+			return ProposalCandidate{(int) (span.x + j), probability(lo, span.y, total)};
+		};
 		// The pixel's draws of all frames, spread over the lanes (each draw
 		// has its own noise stream, so any lane may take any draw).
-		const uint32_t draws = pr.frame_count * (uint32_t) per_frame;
-		for (uint32_t d = lane; d < draws; d += 32) {
-			const uint32_t f = d / (uint32_t) per_frame;
-			const int c = (int) (d % (uint32_t) per_frame);
-			{
-				uint32_t s = proposal_stream(x_pix, y_pix, pr.width, pr.noise_seed, f, pr.animate, (uint32_t) c);
-				const float u0 = get_noise_1(s), u1 = get_noise_1(s), u2 = get_noise_1(s);
-				int light;
-				if (!proposal || u0 < a) {
-					light = (int) (u1 * (float) n_lights);
-					light = light > n_lights - 1 ? n_lights - 1 : light;
-				} else {
-					// First cluster whose cumulative weight exceeds u1 * total.
-					const float t = u1 * total;
-					int lo = 0, hi = k_count - 1;
-					while (lo < hi) {
-						const int mid = (lo + hi) >> 1;
-						if (cdf[cdf_slot(mid)] > t)
-							hi = mid;
-						else
-							lo = mid + 1;
-					}
-					// Rounding can leave t at the top: take the last non-empty cluster.
-					uint2 span = pr.clusters.spans[lo];
-					while (lo > 0 && span.y == 0) span = pr.clusters.spans[--lo];
-					const uint32_t first = span.x, size = span.y;
-					uint32_t j = (uint32_t) (u2 * (float) size);
-					j = j > size - 1 ? size - 1 : j;
-					light = (int) (first + j);
-				}
-				float pdf = __frcp_rn((float) n_lights);
-				if (proposal) {
-					const uint32_t k = pr.clusters.light_cluster[light];
-					const float mass = cdf[cdf_slot((int) k)] - (k > 0 ? cdf[cdf_slot((int) k - 1)] : 0.0f);
-					const uint32_t size = pr.clusters.spans[k].y;
-					pdf = __fadd_rn(__fdiv_rn(a, (float) n_lights),
-					                __fdiv_rn(__fmul_rn(1.0f - a, __fdiv_rn(mass, total)), (float) size));
-				}
-				pr.out[((size_t) f * np + i) * per_frame + c] = ProposalCandidate{light, pdf};
-			}
+		if (lane < draws) first_out[(size_t) i * per_frame] = draw(proposal_stream(i, first_number, first_c));
+		for (uint32_t d = lane + 32; d < draws; d += 32) {
+			const uint32_t f = d / per_frame, c = d % per_frame;
+			pr.out[((size_t) f * np + i) * per_frame + c] =
+			    draw(proposal_stream(i, proposal_number(pr.noise_seed, f, pr.animate), c));
 		}
 		__syncwarp();
 	}
