@@ -150,9 +150,9 @@ int grid_for(const risltc_ctx_t* ctx, size_t items) {
 
 // The BVH's device layout for traversal: the root's record {bmin, reference,
 // bmax, 0} (8 floats), then one 16-float record per inner node holding both
-// children: the six box planes {bmin.x, bmin.y, bmin.z, bmax.x, bmax.y,
-// bmax.z} with the children's values side by side, then the two references
-// and two unused words.  A reference is an inner node's record index (>= 0) or
+// children, each as {bmin.x, bmin.y, bmax.x, bmax.y, bmin.z, bmax.z,
+// reference, 0}: the pairs that the slab test's paired operations take.  A
+// reference is an inner node's record index (>= 0) or
 // a leaf, -(1 + (first triangle << 3 | triangle count)) with 1..7 triangles;
 // a larger leaf becomes a small subtree of leaves of at most 7 triangles, all
 // with the leaf's box, so the triangles tested for a ray do not change.  Inner
@@ -201,11 +201,10 @@ std::vector<float> child_pair_nodes(const float* nodes, uint32_t node_count) {
 	// Child `child` (0 or 1) of a record: box_node's box and the reference.
 	auto put = [&](size_t record_at, int child, uint32_t box_node, int32_t ref) {
 		const float* box = nodes + 8 * (size_t) box_node;
-		for (int a = 0; a != 3; ++a) {
-			out[record_at + 2 * a + child] = box[a];
-			out[record_at + 6 + 2 * a + child] = box[4 + a];
-		}
-		memcpy(out.data() + record_at + 12 + child, &ref, sizeof(ref));
+		float* d = out.data() + record_at + 8 * (size_t) child;
+		const float planes[6] = {box[0], box[1], box[4], box[5], box[2], box[6]};
+		memcpy(d, planes, sizeof(planes));
+		memcpy(d + 6, &ref, sizeof(ref));
 	};
 	while (!stack.empty()) {
 		const Pending p = stack.back();
@@ -1381,9 +1380,8 @@ EXTERN_C int risltc_shade_host(risltc_ctx_t* ctx, const risltc_scene_t* scene, u
 	return risltc_ctx_check(ctx);
 }
 
-// Blocks of the query kernels that fit an SM (their registers allow ten or
-// eleven).
-static constexpr int kTraceBlocksPerSm = 10;
+// Blocks of the query kernels that fit an SM.
+static constexpr int kTraceBlocksPerSm = 12;
 
 EXTERN_C int risltc_trace_shadow(risltc_ctx_t* ctx, const risltc_scene_t* scene, const float* rays, uint32_t ray_count,
                                  uint32_t* hits) {

@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_bat
 	const uint32_t n = b.ray_begin[b.count];
 	const uint32_t lane = threadIdx.x % 32;
 	uint32_t* const error = b.item[0].error;
-	int32_t stack[kBvhStack];
+	int32_t stack[kTraceStack];
 	TraceRay r;
 	SceneView s = {};
 	uint8_t* hits = nullptr;
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_bat
 					slot = g - b.ray_begin[k];
 					const ShadowRay* ray = pr.rays + slot;
 					const float4 a = __ldg(&ray->origin), d = __ldg(&ray->dir_tmax);
-					const int st = trace_begin<P>(s, r, mk3(a.x, a.y, a.z), mk3(d.x, d.y, d.z), 1.0e-3f, d.w);
+					const int st = trace_begin<P>(s, r, mk3(a.x, a.y, a.z), mk3(d.x, d.y, d.z), 1.0e-3f, d.w, stack);
 					if (st == kTraceContinue)
 						busy = true;
 					else

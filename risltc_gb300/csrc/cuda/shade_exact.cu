@@ -64,9 +64,9 @@ cudaError_t launch_batch_estimator(const RisBatch& b, cudaStream_t stream, int p
 	return cudaGetLastError();
 }
 // One thread per ray while all of them are resident at once (grid blocks of
-// 128), the persistent queue beyond that: 2M rays against 200k occluders
-// 831 us with a thread per ray, 667 us with the queue, whose cursor
-// is zeroed first.
+// 128), the persistent queue beyond that, whose cursor is zeroed first: 2M rays
+// against 200k occluders took 831 us with a thread per ray, 667 with the queue
+// when it was brought in and 576 with the present traversal.
 cudaError_t launch_trace_exact(const SceneView& s, const float4* rays, uint32_t count, uint32_t* hits, uint32_t* error,
                                uint32_t* cursor, cudaStream_t stream, int grid, int resident) {
 	if (grid <= resident) {

@@ -43,46 +43,55 @@ struct ShadeParams {
 // brute-force test of all triangles given conservative boxes; only the order
 // of the tests differs, which an any-hit query does not see.
 struct TraceRay {
-	f3 o, d;
-	float inv[3];
+	f3 no, d;         // the negated origin (slab differences are sums), the direction
+	f3 inv;
 	float t_min, t_max;
-	int32_t node;     // next reference to visit (kNoNode: pop the stack)
-	uint32_t leaf_first, leaf_left;  // triangles of the current leaf still to test
+	// The next unit of work: an inner node's index (>= 0), or the rest of a
+	// leaf as its reference is written, -(1 + (first << 3 | triangles left)).
+	int32_t work;
 	int sp;
 	uint32_t visits;
 	bool minmax;      // no slab product can be NaN: the min/max form applies
 };
 
 enum : int { kTraceContinue = 0, kTraceMiss = 1, kTraceHit = 2 };
-constexpr int32_t kNoNode = INT32_MIN;
+constexpr int32_t kStackEnd = INT32_MIN;  // at the bottom of every stack
+constexpr int kTraceStack = kBvhStack + 1;
 
-// Slab test of one box against the ray's [t_min, t_max]; *entry gets the
-// entry distance.  Per axis t0 = (bmin - o) * inv, t1 = (bmax - o) * inv;
-// the interval is narrowed by min(t0, t1) and max(t0, t1), an endpoint that
-// is NaN leaving its side unchanged.  When no product can be NaN (finite box
-// and origin, finite non-zero inv) the same result comes from IEEE min/max
-// instructions, used then.
-RL_DEV bool ray_box(const TraceRay& r, float4 lo, float4 hi, float* entry) {
-	const float bmin[3] = {lo.x, lo.y, lo.z}, bmax[3] = {hi.x, hi.y, hi.z};
-	const float org[3] = {r.o.x, r.o.y, r.o.z};
-	float t0s = r.t_min, t1s = r.t_max;
+RL_DEV float max3f(float a, float b, float c) {
+	float d;
+	asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+	return d;
+}
+RL_DEV float min3f(float a, float b, float c) {
+	float d;
+	asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+	return d;
+}
+
+// Slab test of one box, {bmin.x, bmin.y, bmax.x, bmax.y} and {bmin.z, bmax.z},
+// against the ray's [t_min, t_max]; *entry gets the entry distance.  Per axis
+// t0 = (bmin - o) * inv, t1 = (bmax - o) * inv; the interval is narrowed by
+// min(t0, t1) and max(t0, t1), an endpoint that is NaN leaving its side
+// unchanged.  When no product can be NaN (finite box and origin, finite
+// non-zero inv) the same result comes from IEEE min/max instructions, used
+// then.
+RL_DEV bool ray_box(const TraceRay& r, float4 xy, float2 z, float* entry) {
+	const float2 no = make_float2(r.no.x, r.no.y), inv = make_float2(r.inv.x, r.inv.y);
+	const float2 t0 = __fmul2_rn(__fadd2_rn(make_float2(xy.x, xy.y), no), inv);
+	const float2 t1 = __fmul2_rn(__fadd2_rn(make_float2(xy.z, xy.w), no), inv);
+	const float2 tz = __fmul2_rn(__fadd2_rn(z, make_float2(r.no.z, r.no.z)), make_float2(r.inv.z, r.inv.z));
 	if (r.minmax) {
+		*entry = fmaxf(r.t_min, max3f(fminf(t0.x, t1.x), fminf(t0.y, t1.y), fminf(tz.x, tz.y)));
+		return *entry <= fminf(r.t_max, min3f(fmaxf(t0.x, t1.x), fmaxf(t0.y, t1.y), fmaxf(tz.x, tz.y)));
+	}
+	const float a[3] = {t0.x, t0.y, tz.x}, b[3] = {t1.x, t1.y, tz.y};
+	float t0s = r.t_min, t1s = r.t_max;
 #pragma unroll
-		for (int ax = 0; ax != 3; ++ax) {
-			const float t0 = (bmin[ax] - org[ax]) * r.inv[ax];
-			const float t1 = (bmax[ax] - org[ax]) * r.inv[ax];
-			t0s = fmaxf(t0s, fminf(t0, t1));
-			t1s = fminf(t1s, fmaxf(t0, t1));
-		}
-	} else {
-#pragma unroll
-		for (int ax = 0; ax != 3; ++ax) {
-			const float t0 = (bmin[ax] - org[ax]) * r.inv[ax];
-			const float t1 = (bmax[ax] - org[ax]) * r.inv[ax];
-			const float tn = t0 < t1 ? t0 : t1, tf = t0 < t1 ? t1 : t0;
-			if (tn == tn && tn > t0s) t0s = tn;
-			if (tf == tf && tf < t1s) t1s = tf;
-		}
+	for (int ax = 0; ax != 3; ++ax) {
+		const float tn = a[ax] < b[ax] ? a[ax] : b[ax], tf = a[ax] < b[ax] ? b[ax] : a[ax];
+		if (tn == tn && tn > t0s) t0s = tn;
+		if (tf == tf && tf < t1s) t1s = tf;
 	}
 	*entry = t0s;
 	return t0s <= t1s;
@@ -97,7 +106,7 @@ template <class P> RL_DEV bool ray_triangle(const TraceRay& r, const float4* t) 
 	const float det = dot(e1, p);
 	if (!(det != 0.0f)) return false;
 	const float id = P::rcp(det);
-	const f3 sv = sub(r.o, v0);
+	const f3 sv = mk3(-r.no.x - v0.x, -r.no.y - v0.y, -r.no.z - v0.z);
 	const float u = dot(sv, p) * id;
 	if (!(u >= 0.0f && u <= 1.0f)) return false;
 	const f3 q = cross(sv, e1);
@@ -107,142 +116,83 @@ template <class P> RL_DEV bool ray_triangle(const TraceRay& r, const float4* t) 
 	return tt >= r.t_min && tt <= r.t_max;
 }
 
-// Sets up the ray and tests the root box: kTraceMiss, or kTraceContinue.
-template <class P> RL_DEV int trace_begin(const SceneView& s, TraceRay& r, f3 o, f3 d, float t_min, float t_max) {
-	r.o = o;
+// Sets up the ray and its stack and tests the root box: kTraceMiss, or
+// kTraceContinue.
+template <class P>
+RL_DEV int trace_begin(const SceneView& s, TraceRay& r, f3 o, f3 d, float t_min, float t_max, int32_t* stack) {
+	r.no = neg(o);
 	r.d = d;
-	r.inv[0] = P::rcp(d.x);
-	r.inv[1] = P::rcp(d.y);
-	r.inv[2] = P::rcp(d.z);
+	r.inv = mk3(P::rcp(d.x), P::rcp(d.y), P::rcp(d.z));
 	r.t_min = t_min;
 	r.t_max = t_max;
-	r.sp = 0;
+	stack[0] = kStackEnd;
+	r.sp = 1;
 	r.visits = 0;
-	r.leaf_left = 0;
-	r.leaf_first = 0;
 	// Boxes are finite (the scene rejects non-finite triangles); with a
 	// finite origin and finite non-zero inv no slab product is NaN, and with
 	// t_min and t_max not NaN neither is an interval end.
 	r.minmax = !isnan(t_min) && !isnan(t_max);
-	const float oc[3] = {o.x, o.y, o.z};
+	const float oc[3] = {o.x, o.y, o.z}, inv[3] = {r.inv.x, r.inv.y, r.inv.z};
 #pragma unroll
-	for (int ax = 0; ax != 3; ++ax)
-		r.minmax = r.minmax && isfinite(oc[ax]) && isfinite(r.inv[ax]) && r.inv[ax] != 0.0f;
+	for (int ax = 0; ax != 3; ++ax) r.minmax = r.minmax && isfinite(oc[ax]) && isfinite(inv[ax]) && inv[ax] != 0.0f;
 	if (s.triangle_count == 0) return kTraceMiss;
 	const float4 lo = __ldg(s.pairs), hi = __ldg(s.pairs + 1);
 	float entry;
-	if (!ray_box(r, lo, hi, &entry)) return kTraceMiss;
-	r.node = __float_as_int(lo.w);
+	if (!ray_box(r, make_float4(lo.x, lo.y, hi.x, hi.y), make_float2(lo.z, hi.z), &entry)) return kTraceMiss;
+	r.work = __float_as_int(lo.w);
 	return kTraceContinue;
 }
 
-// The ray's next unit of work: kWorkTriangle (the current leaf's next
-// triangle) or kWorkNode (an inner node), resolving the current reference or
-// the top of the stack and opening leaves on the way; kWorkDone when nothing
-// is left.  Calling it again before the work is done returns the same unit.
-enum : int { kWorkTriangle = 0, kWorkNode = 1, kWorkDone = 2 };
-RL_DEV int trace_next(TraceRay& r, const int32_t* stack) {
-	if (r.leaf_left != 0) return kWorkTriangle;
-	for (;;) {
-		if (r.node == kNoNode) {
-			if (r.sp == 0) return kWorkDone;
-			r.node = stack[--r.sp];
-		}
-		if (r.node >= 0) return kWorkNode;
-		const uint32_t code = (uint32_t) (-(r.node + 1));
-		r.leaf_first = code >> 3;
-		r.leaf_left = code & 7u;
-		r.node = kNoNode;
-		if (r.leaf_left != 0) return kWorkTriangle;
-	}
-}
-
-// One triangle test of the current leaf: kTraceHit or kTraceContinue.
-template <class P> RL_DEV int trace_triangle(const SceneView& s, TraceRay& r) {
-	const bool hit = ray_triangle<P>(r, s.triangles + 3 * (size_t) r.leaf_first);
-	++r.leaf_first;
-	--r.leaf_left;
-	return hit ? kTraceHit : kTraceContinue;
-}
-
-RL_DEV float max3f(float a, float b, float c) {
-	float d;
-	asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-	return d;
-}
-RL_DEV float min3f(float a, float b, float c) {
-	float d;
-	asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-	return d;
-}
-
-// One inner node: both child boxes, the nearer hit child next and the other
-// pushed.  kTraceContinue, or kTraceMiss with the error recorded when the
-// stack is full.  Two 32-byte loads; the two children's slab distances are
-// the lanes of paired subtractions and multiplications, ray_box's operations
-// (trace kernel 4.54 -> 4.40 ms per 4-frame 1080p launch with 1M occluders).
-// Bound by issue (70% of the slots at 11 of 32 active lanes).  Four-child
-// nodes in the same form (128 bytes, nearest child first) took 5.09 ms.
-RL_DEV int trace_node(const SceneView& s, TraceRay& r, int32_t* stack, uint32_t* error) {
-	const float4* n = s.pairs + 2 + 4 * (size_t) r.node;
-	const RecordWords p = load_words(n), q = load_words(n + 2);
-	const int32_t ref0 = __float_as_int(q.b.x), ref1 = __float_as_int(q.b.y);
-	float e0, e1;
-	bool h0, h1;
-	if (r.minmax) {
-		const float2 lo[3] = {make_float2(p.a.x, p.a.y), make_float2(p.a.z, p.a.w), make_float2(p.b.x, p.b.y)};
-		const float2 hi[3] = {make_float2(p.b.z, p.b.w), make_float2(q.a.x, q.a.y), make_float2(q.a.z, q.a.w)};
-		const float o[3] = {r.o.x, r.o.y, r.o.z};
-		float2 near[3], far[3];
-#pragma unroll
-		for (int ax = 0; ax != 3; ++ax) {
-			const float2 no = make_float2(-o[ax], -o[ax]), inv = make_float2(r.inv[ax], r.inv[ax]);
-			const float2 t0 = __fmul2_rn(__fadd2_rn(lo[ax], no), inv), t1 = __fmul2_rn(__fadd2_rn(hi[ax], no), inv);
-			near[ax] = make_float2(fminf(t0.x, t1.x), fminf(t0.y, t1.y));
-			far[ax] = make_float2(fmaxf(t0.x, t1.x), fmaxf(t0.y, t1.y));
-		}
-		e0 = fmaxf(r.t_min, max3f(near[0].x, near[1].x, near[2].x));
-		e1 = fmaxf(r.t_min, max3f(near[0].y, near[1].y, near[2].y));
-		h0 = e0 <= fminf(r.t_max, min3f(far[0].x, far[1].x, far[2].x));
-		h1 = e1 <= fminf(r.t_max, min3f(far[0].y, far[1].y, far[2].y));
-	} else {
-		h0 = ray_box(r, make_float4(p.a.x, p.a.z, p.b.x, 0.0f), make_float4(p.b.z, q.a.x, q.a.z, 0.0f), &e0);
-		h1 = ray_box(r, make_float4(p.a.y, p.a.w, p.b.y, 0.0f), make_float4(p.b.w, q.a.y, q.a.w, 0.0f), &e1);
-	}
-	if (h0 && h1) {
-		if (r.sp >= kBvhStack) {
-			atomicOr(error, kErrorTraversalLimit);
-			return kTraceMiss;
-		}
-		// The nearer child first: an occluder near the origin ends the
-		// query early.
-		const bool second_first = e1 < e0;
-		stack[r.sp++] = second_first ? ref0 : ref1;
-		r.node = second_first ? ref1 : ref0;
-	} else {
-		r.node = h0 ? ref0 : (h1 ? ref1 : kNoNode);
-	}
-	return kTraceContinue;
-}
-
-// One step: one triangle test or one inner node.  Gives up after
-// kTraversalLimit steps or on a stack overflow, records the error and
-// reports "not occluded".
+// One step: one triangle test or one inner node (the nearer hit child next,
+// since an occluder near the origin ends the query early, and the other
+// pushed).  A node is two 32-byte loads; its slab distances are paired
+// operations on (x, y) and on the two z planes, which need no operand twice
+// but the origin's and the direction's z.  Gives up after kTraversalLimit
+// steps or on a stack overflow, records the error and reports "not occluded".
+// Compiled for 12 blocks of 128 threads per SM (40 registers) the trace kernel
+// takes 3.36 ms per 4-frame 1080p launch with 1M occluders; the form before
+// (the children's planes side by side, every operand needed twice, leaf and
+// node references apart) 4.10.
 template <class P> RL_DEV int trace_step(const SceneView& s, TraceRay& r, int32_t* stack, uint32_t* error) {
 	if (++r.visits > kTraversalLimit) {
 		atomicOr(error, kErrorTraversalLimit);
 		return kTraceMiss;
 	}
-	const int work = trace_next(r, stack);
-	if (work == kWorkDone) return kTraceMiss;
-	return work == kWorkTriangle ? trace_triangle<P>(s, r) : trace_node(s, r, stack, error);
+	bool pop;
+	if (r.work >= 0) {
+		const float4* n = s.pairs + 2 + 4 * (size_t) r.work;
+		const RecordWords a = load_words(n), b = load_words(n + 2);
+		float e0, e1;
+		const bool h0 = ray_box(r, a.a, make_float2(a.b.x, a.b.y), &e0), h1 = ray_box(r, b.a, make_float2(b.b.x, b.b.y), &e1);
+		const int32_t ref0 = __float_as_int(a.b.z), ref1 = __float_as_int(b.b.z);
+		const bool second = h1 && !(h0 && e0 <= e1);  // the child to go on with
+		r.work = second ? ref1 : ref0;
+		pop = !h0 && !h1;
+		if (h0 && h1) {
+			if (r.sp >= kTraceStack) {
+				atomicOr(error, kErrorTraversalLimit);
+				return kTraceMiss;
+			}
+			stack[r.sp++] = second ? ref0 : ref1;
+		}
+	} else {
+		const uint32_t code = ~(uint32_t) r.work;
+		if (ray_triangle<P>(r, s.triangles + 3 * (size_t) (code >> 3))) return kTraceHit;
+		r.work -= 7;  // the next triangle, one fewer left
+		pop = (~(uint32_t) r.work & 7u) == 0;
+	}
+	if (pop) {
+		r.work = stack[--r.sp];
+		if (r.work == kStackEnd) return kTraceMiss;
+	}
+	return kTraceContinue;
 }
 
 // Any-hit query; true if occluded.
 template <class P> RL_DEV bool any_hit(const SceneView& s, f3 o, f3 d, float t_min, float t_max, uint32_t* error) {
 	TraceRay r;
-	int32_t stack[kBvhStack];
-	int st = trace_begin<P>(s, r, o, d, t_min, t_max);
+	int32_t stack[kTraceStack];
+	int st = trace_begin<P>(s, r, o, d, t_min, t_max, stack);
 	while (st == kTraceContinue) st = trace_step<P>(s, r, stack, error);
 	return st == kTraceHit;
 }
