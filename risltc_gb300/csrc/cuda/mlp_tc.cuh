@@ -198,12 +198,23 @@ static_assert(kMlpInputs * kTcRows * 4 <= kTcRows * kMlpHidden * 2, "inputs fit 
 // G-buffer plane of MLP input k (position, normal, outgoing, roughness).
 RL_DEV int mlp_input_plane(int k) { return k < 9 ? k : 16; }
 
-// Eight FP32 values to 32-byte aligned memory in one store (a whole sector).
-RL_DEV void store8(float* dst, const float (&v)[8]) {
-	asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]),
-	             "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-	             : "memory");
-}
+// The logits' staging: rows of 256 bytes, 272 apart (lanes' 16-byte words of
+// one index fall in distinct banks), in A1, from which a warp writes two
+// rows per instruction.  (Each lane storing to its own row occupied the L1
+// data pipe for three quarters of the call: 157 us at 960x540 with 256
+// clusters, 127 staged.  One bulk copy per row segment: 146 with 256
+// bytes, 199 with 128, about 14 cycles per copy.)
+constexpr int kLogitStage = 256, kLogitStride = 272;
+static_assert(kTcRows * kLogitStride <= kTcRows * kMlpFeatures * 2, "a tile's staged logits fit in A1");
+
+template <bool kF32> struct LogitType {
+	using type = __nv_bfloat16;
+	RL_DEV static type* rows(const MlpParams& pr) { return pr.logits; }
+};
+template <> struct LogitType<true> {
+	using type = float;
+	RL_DEV static type* rows(const MlpParams& pr) { return pr.logits_f32; }
+};
 
 // kF32: the logits go to pr.logits_f32.
 template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp_logits_tc_kernel(MlpParams pr) {
@@ -294,6 +305,10 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 		__syncthreads();
 		tc_fence_after();
 	};
+	using Out = typename LogitType<kF32>::type;
+	Out* const logits = LogitType<kF32>::rows(pr);
+	constexpr int kStage = kLogitStage / (int) sizeof(Out);  // columns
+	const bool wide_stores = (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
 	for (uint32_t tile = blockIdx.x; tile < tiles && !failed; tile += gridDim.x) {
 		const uint32_t p0 = tile * kTcRows;
 		if (bulk_inputs) {
@@ -353,43 +368,52 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 				uint32_t v[32];
 				tc_load32(d3 + lane_base + (uint32_t) c, v);
 				tc_wait_load();
-				if (row < np) {
-					const size_t at = (size_t) row * k_count + c0 + c;
-					// Rows are multiples of 32 bytes; the caller's buffer may
-					// have any alignment.
-					const bool aligned = (reinterpret_cast<uintptr_t>(pr.logits_f32) & 31) == 0;
+				const int at = c % kStage;  // of the staged columns
+				unsigned char* const staged = tc_smem + tl.a1 + tid * kLogitStride + at * (int) sizeof(Out);
 #pragma unroll
-					for (int q = 0; q != 4; ++q) {
-						const int j0 = c0 + c + 8 * q;
-						if (j0 + 8 > k_count) continue;  // k_count is a multiple of 8
-						uint4 out;
-						uint32_t* o = &out.x;
+				for (int q = 0; q != 4; ++q) {
+					const int j0 = c0 + c + 8 * q;
+					if (j0 + 8 > k_count) continue;  // k_count is a multiple of 8
+					uint32_t o[4];
 #pragma unroll
-						for (int h = 0; h != 2; ++h) {
-							const float4 b = *reinterpret_cast<const float4*>(b3 + j0 + 4 * h);
-							const int j = 8 * q + 4 * h;
-							o[2 * h] = pack_bf16x2(__uint_as_float(v[j]) + b.x, __uint_as_float(v[j + 1]) + b.y);
-							o[2 * h + 1] = pack_bf16x2(__uint_as_float(v[j + 2]) + b.z, __uint_as_float(v[j + 3]) + b.w);
-						}
-						if (!kF32) {
-							*reinterpret_cast<uint4*>(pr.logits + at + 8 * q) = out;
-						} else {
-							float wide[8];
+					for (int h = 0; h != 2; ++h) {
+						const float4 b = *reinterpret_cast<const float4*>(b3 + j0 + 4 * h);
+						const int j = 8 * q + 4 * h;
+						o[2 * h] = pack_bf16x2(__uint_as_float(v[j]) + b.x, __uint_as_float(v[j + 1]) + b.y);
+						o[2 * h + 1] = pack_bf16x2(__uint_as_float(v[j + 2]) + b.z, __uint_as_float(v[j + 3]) + b.w);
+					}
+					if (!kF32) {
+						*reinterpret_cast<uint4*>(staged + 16 * q) = make_uint4(o[0], o[1], o[2], o[3]);
+					} else {
 #pragma unroll
-							for (int h = 0; h != 4; ++h) {
-								wide[2 * h] = __uint_as_float(o[h] << 16);
-								wide[2 * h + 1] = __uint_as_float(o[h] & 0xffff0000u);
-							}
-							float* const dst = pr.logits_f32 + at + 8 * q;
-							if (aligned) {
-								store8(dst, wide);
-							} else {
-#pragma unroll
-								for (int h = 0; h != 8; ++h) dst[h] = wide[h];
-							}
-						}
+						for (int h = 0; h != 2; ++h)
+							*reinterpret_cast<uint4*>(staged + 32 * q + 16 * h) =
+							    make_uint4(o[2 * h] << 16, o[2 * h] & 0xffff0000u, o[2 * h + 1] << 16, o[2 * h + 1] & 0xffff0000u);
 					}
 				}
+				// With the stage full (or its last columns in it) the warp
+				// writes its rows' columns first .. end - 1, two rows of up to
+				// 256 bytes at a time.
+				const int first = c0 + c - at, end = min(c0 + c + 32, k_count);
+				if ((at + 32 != kStage && c + 32 < n) || end <= first) continue;
+				__syncwarp();
+				const unsigned char* const stage = tc_smem + tl.a1 + (tid & ~31u) * kLogitStride;
+				const uint32_t row0 = p0 + (tid & ~31u);
+				if (wide_stores) {
+					const int word = (int) (tid % 16);
+					const bool mine = 16 * word < (end - first) * (int) sizeof(Out);
+#pragma unroll 4
+					for (uint32_t r = tid % 32 / 16; r < 32; r += 2)
+						if (mine && row0 + r < np)
+							*reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(logits + (size_t) (row0 + r) * k_count + first) + 16 * word) =
+							    *reinterpret_cast<const uint4*>(stage + r * kLogitStride + 16 * word);
+				} else {
+					for (uint32_t r = 0; r != 32 && row0 + r < np; ++r)
+						for (int k = (int) (tid % 32); k < end - first; k += 32)
+							logits[(size_t) (row0 + r) * k_count + first + k] =
+							    reinterpret_cast<const Out*>(stage + r * kLogitStride)[k];
+				}
+				__syncwarp();
 			}
 			tc_fence_before();
 			__syncthreads();
