@@ -731,7 +731,7 @@ cudaError_t launch_logits(risltc_ctx_t* ctx, cudaStream_t stream, const risltc_m
 	static std::atomic<uint64_t> configured{0};
 	const uint64_t bit = 1ull << (ctx->device & 63);
 	if (!(configured.load() & bit)) {
-		const int smem = (int) risltc::mlp_tc_smem_bytes(risltc::kMaxClusters);
+		const int smem = (int) risltc::kTcSmemLimit;
 		cudaError_t e = cudaFuncSetAttribute(risltc::mlp_logits_tc_kernel<false>,
 		                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 		if (e == cudaSuccess)
@@ -739,15 +739,17 @@ cudaError_t launch_logits(risltc_ctx_t* ctx, cudaStream_t stream, const risltc_m
 		if (e != cudaSuccess) return e;
 		configured.fetch_or(bit);
 	}
-	// At most two CTAs per SM fit in shared memory, so the two 256-column
-	// tensor-memory allocations of an SM never wait for each other.
+	// One CTA per SM (each takes more than half of its shared memory), so no
+	// tensor-memory allocation waits for another.
 	const size_t tiles = ((size_t) gbuffer->width * gbuffer->height + risltc::kTcRows - 1) / risltc::kTcRows;
-	const int grid = (int) std::min<size_t>(tiles, (size_t) ctx->sm_count * 2);
-	const size_t smem = risltc::mlp_tc_smem_bytes(m->cluster_count);
+	const int grid = (int) std::min<size_t>(tiles, (size_t) ctx->sm_count);
+	const risltc::TcLayout layout = risltc::tc_layout(m->cluster_count);
+	const size_t smem = layout.total;
+	const int threads = risltc::kTcThreads * (int) layout.groups;
 	if (logits_f32)
-		risltc::mlp_logits_tc_kernel<true><<<grid, risltc::kTcThreads, smem, stream>>>(q);
+		risltc::mlp_logits_tc_kernel<true><<<grid, threads, smem, stream>>>(q);
 	else
-		risltc::mlp_logits_tc_kernel<false><<<grid, risltc::kTcThreads, smem, stream>>>(q);
+		risltc::mlp_logits_tc_kernel<false><<<grid, threads, smem, stream>>>(q);
 	const cudaError_t e = cudaGetLastError();
 	if (e == cudaSuccess) ctx->kernel_launches += 1;
 	return e;

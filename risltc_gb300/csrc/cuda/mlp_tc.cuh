@@ -1,22 +1,28 @@
 // mlp_tc.cuh - the proposal MLP's forward pass on the 5th-generation tensor
 // cores (tcgen05, sm_100 family).
 //
-// One CTA of four warps per tile of 128 pixels.  The encoded features
-// (128 x 144), the hidden activations (128 x 64) and the three weight
-// matrices live in shared memory as K-major BF16 operands in 8x8 core
-// matrices (no swizzle); one thread issues the products
+// One CTA per SM holds the three weight matrices and works on up to four tiles
+// of 128 pixels at once, one per group of four warps.  The encoded features
+// (128 x 144), the hidden activations (128 x 64) and the weights live in
+// shared memory as K-major BF16 operands in 8x8 core matrices (no swizzle);
+// one thread of a group issues the products
 //   D1 = A1 W1^T (K = 144), D2 = A2 W2^T (K = 64), D3 = A3 W3^T (K = 64,
 //   up to 128 clusters per product)
-// with FP32 accumulators in tensor memory (256 columns per CTA: D1 and D2 in
-// columns 0..63, D3 in 64..191), and each warp moves its 32 rows (pixels)
+// with FP32 accumulators in the group's 128 columns of tensor memory (each
+// product replaces the one before, which the group has read by then), and each
+// warp moves its 32 rows (pixels)
 // from tensor memory to registers for the epilogues: bias, ReLU and BF16
 // rounding back into shared memory for the next product, or bias and BF16
 // rounding of the logits to global memory (as BF16 for the proposal kernel, or
 // widened to FP32 for a caller of risltc_model_logits: a separate pass over
-// 0.8 GB took 0.9 of that call's 1.1 ms at 960x540 with 256 clusters).  Every wait on the tensor cores
-// is bounded; on a timeout the kernel records kErrorTensorWait, waits once
-// more (bounded) for its products in flight, frees its tensor memory and
-// returns.
+// 0.8 GB took 0.9 of that call's 1.1 ms at 960x540 with 256 clusters).  A
+// tile is a chain of waits (inputs, four or more products, epilogues), so what
+// counts is how many tiles an SM has in flight: that call takes 119 us with
+// four sharing the weights, 127 us with two CTAs of one tile each.  Bounds now:
+// its 531 MB of writes (78 us) and the shared-memory data pipe (half busy).
+// Every wait on the tensor cores is bounded; on a timeout the kernel records
+// kErrorTensorWait, waits once more (bounded) for its products in flight,
+// frees its tensor memory and returns.
 #pragma once
 #include "mlp.cuh"
 
@@ -24,7 +30,6 @@ namespace risltc {
 
 constexpr int kTcRows = 128;      // pixels per tile: M of every product
 constexpr int kTcThreads = 128;   // warp w reads tensor-memory lanes 32w .. 32w + 31
-constexpr uint32_t kTcColumns = 256;
 constexpr int kTcChunk = 128;     // clusters per layer-3 product (N)
 constexpr uint64_t kTcWaitNs = 1000000000ull;  // a tensor-core wait gives up after one second
 constexpr uint32_t kErrorTensorWait = 1u << 2;  // error-word bit: a tensor-core wait ran out
@@ -168,12 +173,18 @@ RL_DEV void store_hidden(unsigned char* hidden, int row, int c, int k, const uin
 
 // Shared memory of the kernel for k_count clusters: W1, W2, W3 (rows padded
 // to a multiple of 16; together the operand-layout weights of one bulk copy),
-// A1, A2, the biases, three mbarriers (products, weights, inputs) and the
-// tensor memory address.  A tile's 10 input rows (128 floats each) are
-// staged in the first 5 KB of A2, which is free from a tile's last layer-3
-// product until the next tile's first epilogue.
+// the groups' buffers, the biases, two mbarriers per group (products, inputs),
+// one for the weights and the tensor memory address.  A group's buffer holds
+// its tile's encoded features (A1) and, once layer 1 has read them, the hidden
+// activations (A2) at the same place and the staged logits behind those; after
+// it the tile's 10 input rows (128 floats each), which arrive while the tile
+// before is worked on.  As many groups as fit, up to kTcMaxGroups.
+constexpr int kTcMaxGroups = 4;
+constexpr uint32_t kTcA1Bytes = kTcRows * kMlpFeatures * 2, kTcA2Bytes = kTcRows * kMlpHidden * 2;
+constexpr uint32_t kTcInputBytes = kMlpInputs * kTcRows * 4, kTcGroupBytes = kTcA1Bytes + kTcInputBytes;
+constexpr uint32_t kTcSmemLimit = 232448;  // 227 KB
 struct TcLayout {
-	uint32_t w1, w2, w3, a1, a2, b1, b2, b3, bar, slot, total, weight_bytes;
+	uint32_t w1, w2, w3, group, b1, b2, b3, bar, slot, total, weight_bytes, groups;
 	int k_pad;
 };
 __host__ __device__ inline TcLayout tc_layout(int k_count) {
@@ -183,29 +194,42 @@ __host__ __device__ inline TcLayout tc_layout(int k_count) {
 	l.w1 = 0;
 	l.w2 = l.w1 + kMlpHidden * kMlpFeatures * 2;
 	l.w3 = l.w2 + kMlpHidden * kMlpHidden * 2;
-	l.a1 = l.w3 + (uint32_t) l.k_pad * kMlpHidden * 2;
-	l.a2 = l.a1 + kTcRows * kMlpFeatures * 2;
-	l.b1 = l.a2 + kTcRows * kMlpHidden * 2;
+	l.group = l.w3 + (uint32_t) l.k_pad * kMlpHidden * 2;
+	const uint32_t rest = (2 * kMlpHidden + (uint32_t) l.k_pad) * 4 + (2 * kTcMaxGroups + 2) * 8;
+	l.groups = (kTcSmemLimit - l.group - rest) / kTcGroupBytes;
+	if (l.groups > kTcMaxGroups) l.groups = kTcMaxGroups;
+	l.b1 = l.group + l.groups * kTcGroupBytes;
 	l.b2 = l.b1 + kMlpHidden * 4;
 	l.b3 = l.b2 + kMlpHidden * 4;
-	l.bar = (l.b3 + (uint32_t) l.k_pad * 4 + 7) / 8 * 8;
-	l.slot = l.bar + 3 * 8;
+	l.bar = l.b3 + (uint32_t) l.k_pad * 4;
+	l.slot = l.bar + (2 * kTcMaxGroups + 1) * 8;
 	l.total = l.slot + 8;
 	return l;
 }
-static_assert(kMlpInputs * kTcRows * 4 <= kTcRows * kMlpHidden * 2, "inputs fit in A2");
 
 // G-buffer plane of MLP input k (position, normal, outgoing, roughness).
 RL_DEV int mlp_input_plane(int k) { return k < 9 ? k : 16; }
 
-// The logits' staging: rows of 256 bytes, 272 apart (lanes' 16-byte words of
-// one index fall in distinct banks), in A1, from which a warp writes two
-// rows per instruction.  (Each lane storing to its own row occupied the L1
-// data pipe for three quarters of the call: 157 us at 960x540 with 256
-// clusters, 127 staged.  One bulk copy per row segment: 146 with 256
-// bytes, 199 with 128, about 14 cycles per copy.)
-constexpr int kLogitStage = 256, kLogitStride = 272;
-static_assert(kTcRows * kLogitStride <= kTcRows * kMlpFeatures * 2, "a tile's staged logits fit in A1");
+// The logits' staging: rows of 128 bytes, 144 apart (lanes' 16-byte words of
+// one index fall in distinct banks), from which a warp writes four rows per
+// instruction.  (Each lane storing to its own row occupied the L1 data pipe
+// for three quarters of the call: 157 us at 960x540 with 256 clusters, 127
+// staged.  One bulk copy per row segment: 146 us with 256 bytes, 199 with 128,
+// about 14 cycles per copy.)
+constexpr int kLogitStage = 128, kLogitStride = 144;
+static_assert(kTcA2Bytes + kTcRows * kLogitStride <= kTcA1Bytes, "a tile's staged logits fit behind its hidden activations");
+
+// The barrier of a group's four warps, and the same with the OR of a predicate.
+RL_DEV void group_sync(uint32_t group) { asm volatile("bar.sync %0, 128;\n" ::"r"(group + 1) : "memory"); }
+RL_DEV bool group_any(uint32_t group, bool value) {
+	uint32_t any;
+	asm volatile(
+	    "{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.or.pred q, %2, 128, p;\nselp.u32 %0, 1, 0, q;\n}\n"
+	    : "=r"(any)
+	    : "r"((uint32_t) value), "r"(group + 1)
+	    : "memory");
+	return any != 0;
+}
 
 template <bool kF32> struct LogitType {
 	using type = __nv_bfloat16;
@@ -217,23 +241,25 @@ template <> struct LogitType<true> {
 };
 
 // kF32: the logits go to pr.logits_f32.
-template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp_logits_tc_kernel(MlpParams pr) {
+template <bool kF32> static __global__ void __launch_bounds__(kTcThreads * kTcMaxGroups, 1) mlp_logits_tc_kernel(MlpParams pr) {
 	extern __shared__ __align__(1024) unsigned char tc_smem[];
 	const int k_count = pr.k_count;
 	const MlpLayout lay = mlp_layout(k_count);
 	const TcLayout tl = tc_layout(k_count);
-	const uint32_t tid = threadIdx.x, warp = tid / 32;
+	// Group g (four warps) has its own tiles; thread tid of it takes row tid.
+	const uint32_t group = threadIdx.x / kTcThreads, tid = threadIdx.x % kTcThreads, warp = tid / 32;
 	const uint32_t base = smem_address(tc_smem);
 	float* b1 = reinterpret_cast<float*>(tc_smem + tl.b1);
 	float* b2 = reinterpret_cast<float*>(tc_smem + tl.b2);
 	float* b3 = reinterpret_cast<float*>(tc_smem + tl.b3);
-	const float* inputs = reinterpret_cast<const float*>(tc_smem + tl.a2);  // [10][128] while staged
-	for (int j = tid; j < kMlpHidden; j += kTcThreads) {
+	const uint32_t a1 = tl.group + group * kTcGroupBytes, a2 = a1, stage = a2 + kTcA2Bytes, in = a1 + kTcA1Bytes;
+	const float* inputs = reinterpret_cast<const float*>(tc_smem + in);  // [10][128]
+	for (uint32_t j = threadIdx.x; j < (uint32_t) kMlpHidden; j += blockDim.x) {
 		b1[j] = pr.params[lay.b1 + j];
 		b2[j] = pr.params[lay.b2 + j];
 	}
-	for (int j = tid; j < tl.k_pad; j += kTcThreads) b3[j] = j < k_count ? pr.params[lay.b3 + j] : 0.0f;
-	const uint32_t bar = base + tl.bar, bar_weights = bar + 8, bar_inputs = bar + 16;
+	for (int j = (int) threadIdx.x; j < tl.k_pad; j += (int) blockDim.x) b3[j] = j < k_count ? pr.params[lay.b3 + j] : 0.0f;
+	const uint32_t bar_weights = base + tl.bar, bar = bar_weights + 8 + 16 * group, bar_inputs = bar + 8;
 	const uint32_t np = pr.width * pr.height;
 	const uint32_t tiles = (np + kTcRows - 1) / kTcRows;
 	// A tile's input rows come by bulk copy when every row is 16-byte aligned
@@ -247,22 +273,23 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 			const uint32_t p0 = tile * kTcRows, rows = min((uint32_t) kTcRows, np - p0);
 			mbarrier_expect_bytes(bar_inputs, kMlpInputs * rows * 4);
 			for (int k = 0; k != kMlpInputs; ++k)
-				bulk_copy_to_shared(base + tl.a2 + k * kTcRows * 4, pr.gbuffer + (size_t) mlp_input_plane(k) * np + p0,
+				bulk_copy_to_shared(base + in + k * kTcRows * 4, pr.gbuffer + (size_t) mlp_input_plane(k) * np + p0,
 				                    rows * 4, bar_inputs);
 		}
 		++inputs_issued;
 	};
-	if (tid == 0) {
-		for (int k = 0; k != 3; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar + 8 * k) : "memory");
+	if (threadIdx.x == 0) {
+		for (uint32_t i = 0; i != 1 + 2 * tl.groups; ++i)
+			asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_weights + 8 * i) : "memory");
 		asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 		// The weights in one bulk copy.
 		mbarrier_expect_bytes(bar_weights, tl.weight_bytes);
 		bulk_copy_to_shared(base + tl.w1, pr.weights, tl.weight_bytes, bar_weights);
 	}
-	if (bulk_inputs && blockIdx.x < tiles) fetch_inputs(blockIdx.x);  // the first tile's inputs
-	if (warp == 0) {
+	const uint32_t columns = tl.groups > 2 ? 512u : tl.groups * 128u;  // a power of two
+	if (threadIdx.x < 32) {
 		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(base + tl.slot),
-		             "r"(kTcColumns)
+		             "r"(columns)
 		             : "memory");
 		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
 	}
@@ -271,14 +298,16 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 	__syncthreads();
 	tc_fence_after();
 	const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tc_smem + tl.slot);
-	const uint32_t d12 = tmem, d3 = tmem + 64;
+	const uint32_t d = tmem + 128 * group;  // the group's products, one after another
+	const uint32_t first_tile = blockIdx.x + group * gridDim.x, tile_step = gridDim.x * tl.groups;
+	if (bulk_inputs && first_tile < tiles) fetch_inputs(first_tile);  // the first tile's inputs
 	const uint32_t lane_base = (warp * 32) << 16;  // this warp's tensor-memory lanes
 	uint32_t parity = 0;
 	bool product_pending = false;
 	const bool weights_ok = __syncthreads_or(!tc_wait(bar_weights, 0)) == 0;
 	bool failed = !weights_ok;
-	// One product group: issued by thread 0, then every thread waits for it.
-	// With pr.skip_issue (fault injection) nothing is issued or committed, so
+	// Products in a row: issued by the group's thread 0, then all of its threads
+	// wait for them.  With pr.skip_issue (fault injection) nothing is issued or committed, so
 	// the wait runs out.
 	auto run = [&](auto issue) {
 		if (tid == 0 && !pr.skip_issue) {
@@ -287,7 +316,7 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 		}
 		const bool ok = tc_wait(bar, parity);
 		parity ^= 1u;
-		failed = __syncthreads_or(!ok) != 0;
+		failed = group_any(group, !ok);
 		product_pending = failed && !pr.skip_issue;
 		tc_fence_after();
 	};
@@ -296,24 +325,25 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 	auto hidden_epilogue = [&](const float* bias) {
 		for (int c = 0; c != kMlpHidden; c += 32) {
 			uint32_t v[32];
-			tc_load32(d12 + lane_base + (uint32_t) c, v);
+			tc_load32(d + lane_base + (uint32_t) c, v);
 			tc_wait_load();
-			store_hidden(tc_smem + tl.a2, (int) tid, c, kMlpHidden, v, bias);
+			store_hidden(tc_smem + a2, (int) tid, c, kMlpHidden, v, bias);
 		}
 		fence_async_shared();
 		tc_fence_before();
-		__syncthreads();
+		group_sync(group);
 		tc_fence_after();
 	};
 	using Out = typename LogitType<kF32>::type;
 	Out* const logits = LogitType<kF32>::rows(pr);
 	constexpr int kStage = kLogitStage / (int) sizeof(Out);  // columns
+	constexpr uint32_t kWords = kLogitStage / 16;
 	const bool wide_stores = (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
-	for (uint32_t tile = blockIdx.x; tile < tiles && !failed; tile += gridDim.x) {
+	for (uint32_t tile = first_tile; tile < tiles && !failed; tile += tile_step) {
 		const uint32_t p0 = tile * kTcRows;
 		if (bulk_inputs) {
 			// This tile's input rows (issued during the previous tile).
-			failed = __syncthreads_or(!tc_wait(bar_inputs, inputs_waited & 1u)) != 0;
+			failed = group_any(group, !tc_wait(bar_inputs, inputs_waited & 1u));
 			if (failed) break;
 			++inputs_waited;
 		}
@@ -331,45 +361,43 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 					x[input] = mlp_input(pr.gbuffer, np, i, pr.center, pr.inv_half_extent, input);
 				}
 			}
-			mlp_encode_row(tc_smem + tl.a1, (int) tid, x, i < np, false);
+			mlp_encode_row(tc_smem + a1, (int) tid, x, i < np, false);
 		}
 		fence_async_shared();
 		tc_fence_before();
-		__syncthreads();
+		group_sync(group);
 		tc_fence_after();
+		// The inputs are encoded: the next tile's arrive while this one is worked on.
+		if (bulk_inputs && tile + tile_step < tiles) fetch_inputs(tile + tile_step);
 		run([&] {
 			for (int k = 0; k != kMlpFeatures / 16; ++k)
-				tc_mma(d12, tc_descriptor(base + tl.a1 + 256 * k, kMlpFeatures),
+				tc_mma(d, tc_descriptor(base + a1 + 256 * k, kMlpFeatures),
 				       tc_descriptor(base + tl.w1 + 256 * k, kMlpFeatures), tc_instruction(kTcRows, kMlpHidden), k > 0);
 		});
 		if (failed) break;
 		hidden_epilogue(b1);
 		run([&] {
 			for (int k = 0; k != kMlpHidden / 16; ++k)
-				tc_mma(d12, tc_descriptor(base + tl.a2 + 256 * k, kMlpHidden),
+				tc_mma(d, tc_descriptor(base + a2 + 256 * k, kMlpHidden),
 				       tc_descriptor(base + tl.w2 + 256 * k, kMlpHidden), tc_instruction(kTcRows, kMlpHidden), k > 0);
 		});
 		if (failed) break;
 		hidden_epilogue(b2);
-		const uint32_t row = p0 + tid;
 		for (int c0 = 0; c0 < tl.k_pad && !failed; c0 += kTcChunk) {
 			const int n = min(kTcChunk, tl.k_pad - c0);
 			run([&] {
 				for (int k = 0; k != kMlpHidden / 16; ++k)
-					tc_mma(d3, tc_descriptor(base + tl.a2 + 256 * k, kMlpHidden),
+					tc_mma(d, tc_descriptor(base + a2 + 256 * k, kMlpHidden),
 					       tc_descriptor(base + tl.w3 + (uint32_t) c0 * 128 + 256 * k, kMlpHidden),
 					       tc_instruction(kTcRows, n), k > 0);
 			});
 			if (failed) break;
-			// After the tile's last product A2 is free: the next tile's inputs
-			// arrive there while this tile's logits are written.
-			if (c0 + kTcChunk >= tl.k_pad && bulk_inputs && tile + gridDim.x < tiles) fetch_inputs(tile + gridDim.x);
 			for (int c = 0; c < n; c += 32) {
 				uint32_t v[32];
-				tc_load32(d3 + lane_base + (uint32_t) c, v);
+				tc_load32(d + lane_base + (uint32_t) c, v);
 				tc_wait_load();
 				const int at = c % kStage;  // of the staged columns
-				unsigned char* const staged = tc_smem + tl.a1 + tid * kLogitStride + at * (int) sizeof(Out);
+				unsigned char* const staged = tc_smem + stage + tid * kLogitStride + at * (int) sizeof(Out);
 #pragma unroll
 				for (int q = 0; q != 4; ++q) {
 					const int j0 = c0 + c + 8 * q;
@@ -392,31 +420,31 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 					}
 				}
 				// With the stage full (or its last columns in it) the warp
-				// writes its rows' columns first .. end - 1, two rows of up to
-				// 256 bytes at a time.
+				// writes its rows' columns first .. end - 1, four rows of up to
+				// 128 bytes at a time.
 				const int first = c0 + c - at, end = min(c0 + c + 32, k_count);
 				if ((at + 32 != kStage && c + 32 < n) || end <= first) continue;
 				__syncwarp();
-				const unsigned char* const stage = tc_smem + tl.a1 + (tid & ~31u) * kLogitStride;
+				const unsigned char* const rows = tc_smem + stage + (tid & ~31u) * kLogitStride;
 				const uint32_t row0 = p0 + (tid & ~31u);
 				if (wide_stores) {
-					const int word = (int) (tid % 16);
+					const int word = (int) (tid % kWords);
 					const bool mine = 16 * word < (end - first) * (int) sizeof(Out);
 #pragma unroll 4
-					for (uint32_t r = tid % 32 / 16; r < 32; r += 2)
+					for (uint32_t r = tid % 32 / kWords; r < 32; r += 32 / kWords)
 						if (mine && row0 + r < np)
 							*reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(logits + (size_t) (row0 + r) * k_count + first) + 16 * word) =
-							    *reinterpret_cast<const uint4*>(stage + r * kLogitStride + 16 * word);
+							    *reinterpret_cast<const uint4*>(rows + r * kLogitStride + 16 * word);
 				} else {
 					for (uint32_t r = 0; r != 32 && row0 + r < np; ++r)
 						for (int k = (int) (tid % 32); k < end - first; k += 32)
 							logits[(size_t) (row0 + r) * k_count + first + k] =
-							    reinterpret_cast<const Out*>(stage + r * kLogitStride)[k];
+							    reinterpret_cast<const Out*>(rows + r * kLogitStride)[k];
 				}
 				__syncwarp();
 			}
 			tc_fence_before();
-			__syncthreads();
+			group_sync(group);
 			tc_fence_after();
 		}
 	}
@@ -430,12 +458,10 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads, 1) mlp
 	}
 	tc_fence_before();
 	__syncthreads();
-	if (warp == 0) {
+	if (threadIdx.x < 32) {
 		tc_fence_after();
-		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTcColumns) : "memory");
+		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(columns) : "memory");
 	}
 }
-
-inline size_t mlp_tc_smem_bytes(int k_count) { return tc_layout(k_count).total; }
 
 }  // namespace risltc
