@@ -61,6 +61,20 @@ RL_DEV void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t instruction, uin
 	    : "memory");
 }
 
+// `steps` products of consecutive 16-element steps along K: a and b are the
+// first step's descriptors, a_step and b_step the bytes from one step to the
+// next.  D starts from zero unless `accumulate`.  (Built anew for each product,
+// the descriptors cost the issuing thread about 100 cycles a product.)
+RL_DEV void tc_mma_steps(uint32_t d, uint64_t a, uint32_t a_step, uint64_t b, uint32_t b_step, uint32_t instruction,
+                         int steps, bool accumulate) {
+#pragma unroll 4
+	for (int k = 0; k < steps; ++k) {
+		tc_mma(d, a, b, instruction, accumulate || k > 0);
+		a += a_step >> 4;
+		b += b_step >> 4;
+	}
+}
+
 // The mbarrier at shared address bar completes its phase when the products
 // issued so far by this thread are done.
 RL_DEV void tc_commit(uint32_t bar) {
@@ -130,6 +144,8 @@ RL_DEV void tc_load32(uint32_t taddr, uint32_t (&v)[32]) {
 // (One two-byte store per feature took a sixth of the logits call: 191
 // us at 960x540 with 256 clusters, 157 with these and the biases read
 // four at a time.)
+// kFirst, kLast: only the 16-byte words kFirst .. kLast - 1 of the row.
+template <int kFirst = 0, int kLast = kMlpFeatures / 8>
 RL_DEV void mlp_encode_row(unsigned char* rows, int row, const float (&x)[kMlpInputs], bool in, bool ones) {
 	float low = 0.0f;
 	uint32_t words[4] = {0u, 0u, 0u, 0u};
@@ -139,12 +155,13 @@ RL_DEV void mlp_encode_row(unsigned char* rows, int row, const float (&x)[kMlpIn
 			return;
 		}
 		words[(f >> 1) & 3] = pack_bf16x2(low, v);
-		if ((f & 7) == 7)
+		if ((f & 7) == 7 && f / 8 >= kFirst && f / 8 < kLast)
 			*reinterpret_cast<uint4*>(rows + tc_offset(row, f - 7, kMlpFeatures)) =
 			    make_uint4(words[0], words[1], words[2], words[3]);
 	};
 #pragma unroll
 	for (int input = 0; input != kMlpInputs; ++input) {
+		if (input * 13 + 12 < 8 * kFirst || input * 13 >= 8 * kLast) continue;
 		float e[13];
 		mlp_encode(x[input], e);
 #pragma unroll
@@ -154,11 +171,12 @@ RL_DEV void mlp_encode_row(unsigned char* rows, int row, const float (&x)[kMlpIn
 	for (int f = kMlpInputs * 13; f != kMlpFeatures; ++f) put(f, ones && f == kMlpInputs * 13 ? 1.0f : 0.0f);
 }
 
-// Columns c .. c + 31 of row `row` of a hidden layer (K-major, k columns):
-// the accumulators v plus the bias (16-byte aligned), ReLU, BF16.
-RL_DEV void store_hidden(unsigned char* hidden, int row, int c, int k, const uint32_t (&v)[32], const float* bias) {
+// kColumns columns from c on of row `row` of a hidden layer (K-major, k
+// columns): the accumulators v plus the bias (16-byte aligned), ReLU, BF16.
+template <int kColumns>
+RL_DEV void store_hidden(unsigned char* hidden, int row, int c, int k, const uint32_t (&v)[kColumns], const float* bias) {
 #pragma unroll
-	for (int q = 0; q != 4; ++q) {
+	for (int q = 0; q != kColumns / 8; ++q) {
 		uint32_t o[4];
 #pragma unroll
 		for (int h = 0; h != 2; ++h) {
@@ -370,26 +388,23 @@ template <bool kF32> static __global__ void __launch_bounds__(kTcThreads * kTcMa
 		// The inputs are encoded: the next tile's arrive while this one is worked on.
 		if (bulk_inputs && tile + tile_step < tiles) fetch_inputs(tile + tile_step);
 		run([&] {
-			for (int k = 0; k != kMlpFeatures / 16; ++k)
-				tc_mma(d, tc_descriptor(base + a1 + 256 * k, kMlpFeatures),
-				       tc_descriptor(base + tl.w1 + 256 * k, kMlpFeatures), tc_instruction(kTcRows, kMlpHidden), k > 0);
+			tc_mma_steps(d, tc_descriptor(base + a1, kMlpFeatures), 256, tc_descriptor(base + tl.w1, kMlpFeatures), 256,
+			             tc_instruction(kTcRows, kMlpHidden), kMlpFeatures / 16, false);
 		});
 		if (failed) break;
 		hidden_epilogue(b1);
 		run([&] {
-			for (int k = 0; k != kMlpHidden / 16; ++k)
-				tc_mma(d, tc_descriptor(base + a2 + 256 * k, kMlpHidden),
-				       tc_descriptor(base + tl.w2 + 256 * k, kMlpHidden), tc_instruction(kTcRows, kMlpHidden), k > 0);
+			tc_mma_steps(d, tc_descriptor(base + a2, kMlpHidden), 256, tc_descriptor(base + tl.w2, kMlpHidden), 256,
+			             tc_instruction(kTcRows, kMlpHidden), kMlpHidden / 16, false);
 		});
 		if (failed) break;
 		hidden_epilogue(b2);
 		for (int c0 = 0; c0 < tl.k_pad && !failed; c0 += kTcChunk) {
 			const int n = min(kTcChunk, tl.k_pad - c0);
 			run([&] {
-				for (int k = 0; k != kMlpHidden / 16; ++k)
-					tc_mma(d, tc_descriptor(base + a2 + 256 * k, kMlpHidden),
-					       tc_descriptor(base + tl.w3 + (uint32_t) c0 * 128 + 256 * k, kMlpHidden),
-					       tc_instruction(kTcRows, n), k > 0);
+				tc_mma_steps(d, tc_descriptor(base + a2, kMlpHidden), 256,
+				             tc_descriptor(base + tl.w3 + (uint32_t) c0 * 128, kMlpHidden), 256, tc_instruction(kTcRows, n),
+				             kMlpHidden / 16, false);
 			});
 			if (failed) break;
 			for (int c = 0; c < n; c += 32) {
