@@ -684,7 +684,7 @@ cudaError_t launch_training(risltc_ctx_t* ctx, cudaStream_t stream, const risltc
 		ctx->inject &= ~(uint32_t) RISLTC_FAULT_TRAIN_TENSOR_WAIT;
 		const int blocks = (int) std::min<uint32_t>((n_train + risltc::kTcRows - 1) / risltc::kTcRows,
 		                                            (uint32_t) ctx->sm_count);
-		risltc::mlp_train_tc_kernel<<<blocks, risltc::kTcThreads, risltc::kTtSmemBytes, stream>>>(t);
+		risltc::mlp_train_tc_kernel<<<blocks, risltc::kTtThreads, risltc::kTtSmemBytes, stream>>>(t);
 	} else if (m->cluster_count <= risltc::kTwMaxClusters && !(m->training_flags & RISLTC_TRAIN_CUDA_CORES)) {
 		// More than 256 clusters: the output layer in chunks of 128.
 		t.skip_issue = (ctx->inject & RISLTC_FAULT_TRAIN_TENSOR_WAIT) ? 1u : 0u;
