@@ -3,17 +3,17 @@
 // gradient, the backward products and the weight gradients of a training
 // step, with BF16 operands and FP32 accumulators.
 //
-// One CTA of four warps per SM takes tiles of 128 training pixels.  All
-// operands live in shared memory in the K-major 8x8 core-matrix layout of
+// One CTA of 16 warps per SM takes tiles of 128 training pixels, four threads to
+// a pixel, each with a quarter of every row's columns.  All operands live in shared memory in the K-major 8x8 core-matrix layout of
 // the forward pass ([pixel][feature] for activations and gradients,
 // [out][in] for weights).  The products that contract over the pixels (the
 // weight gradients) and over a weight matrix's rows (the input gradients)
 // read the same bytes through MN-major descriptors, so nothing is stored
 // twice.  Per tile:
 //   D1 = E W1^T, H1 = ReLU(D1 + b1); D2 = H1 W2^T, H2 = ReLU(D2 + b2);
-//   logits in chunks of 128 clusters, BF16 into DZ, softmax per pixel;
+//   logits in chunks of 128 clusters, BF16 in registers, softmax per pixel;
 //   DZ = (q - T) / B as in the CUDA-core kernel (each thread subtracts its
-//   own pixel's target T from its row);
+//   own columns' part of the target T);
 //   dh2 = DZ W3 and dW3 += DZ^T [H2 | 1]; DZ2 = dh2 * [H2 > 0];
 //   dh1 = DZ2 W2 and dW2 += DZ2^T [H1 | 1]; DZ1 = dh1 * [H1 > 0];
 //   dW1 += DZ1^T E (feature 130 of E is 1, so its column is db1).
@@ -24,6 +24,15 @@
 // dW2, 368..511 dW1.  The hidden layers' M = 64 weight-gradient products run
 // at M = 128; their upper 64 rows read the following bytes of shared memory
 // and are discarded.
+//
+// What bounds it: a tile is a chain (products, epilogues, softmax) with nothing
+// else on the SM to run meanwhile, 37 thousand cycles long for 256 clusters and
+// 32 candidates: about 8 of them products, 10 the logits and their two passes of
+// exponentials, 7 the candidates.  So the chain's links are split over 16 warps,
+// and the next tile's candidates and inputs are fetched behind the backward
+// products.  One step of 129,600 pixels takes 145 us; with four warps, a thread
+// per pixel, 207 us; of that the candidates, which each thread read for itself,
+// were the largest part, and with more warps alone they grew (225 us).
 #pragma once
 #include "mlp_tc.cuh"
 
