@@ -691,7 +691,7 @@ cudaError_t launch_training(risltc_ctx_t* ctx, cudaStream_t stream, const risltc
 		ctx->inject &= ~(uint32_t) RISLTC_FAULT_TRAIN_TENSOR_WAIT;
 		const int blocks = (int) std::min<uint32_t>((n_train + risltc::kTcRows - 1) / risltc::kTcRows,
 		                                            (uint32_t) ctx->sm_count);
-		risltc::mlp_train_tc_wide_kernel<<<blocks, risltc::kTcThreads, risltc::kTwSmemBytes, stream>>>(t);
+		risltc::mlp_train_tc_wide_kernel<<<blocks, risltc::kTtThreads, risltc::kTwSmemBytes, stream>>>(t);
 	} else {
 		// Two blocks per SM where their shared memory fits (up to about 500
 		// clusters), one otherwise.

@@ -93,57 +93,11 @@ RL_DEV void tc_load16(uint32_t taddr, uint32_t (&v)[16]) {
 RL_DEV float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 RL_DEV float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
-// A training pixel's candidates: the first kHeld of them read once, all loads
-// in flight together, while layer 1 runs (their clusters, too, are then there
-// when the targets are subtracted; re-read in groups of eight, each group
-// waited for memory twice), the rest read where they are needed.
-struct HeldCandidates {
-	static constexpr int kHeld = 32;
-	static constexpr uint32_t kNone = 0xffffffffu;
-	float weight[kHeld];
-	uint32_t cluster[kHeld];  // kNone: no target
-
-	RL_DEV static uint32_t cluster_of(const MlpTrainParams& pr, int light, float w) {
-		return w > 0.0f && (uint32_t) light < pr.light_count ? pr.light_cluster[light] : kNone;
-	}
-	// Returns the total candidate weight (0 where there is no pixel).
-	RL_DEV float load(const ProposalCandidate* cand, int count, bool valid, const MlpTrainParams& pr) {
-		int light[kHeld];
-#pragma unroll
-		for (int c = 0; c != kHeld; ++c) {
-			light[c] = -1;
-			weight[c] = 0.0f;
-			if (valid && c < count) {
-				light[c] = __ldg(&cand[c].light);  // the caller's records may be 4-byte aligned
-				weight[c] = __ldg(&cand[c].pdf);
-			}
-		}
-#pragma unroll
-		for (int c = 0; c != kHeld; ++c) cluster[c] = cluster_of(pr, light[c], weight[c]);
-		float total = 0.0f;
-#pragma unroll
-		for (int c = 0; c != kHeld; ++c)
-			if (c < count) total += weight[c];
-		if (valid) {
-#pragma unroll 8
-			for (int c = kHeld; c < count; ++c) total += cand[c].pdf;
-		}
-		return total;
-	}
-	// target(cluster, weight) of every candidate that has one, in order.
-	template <class Target>
-	RL_DEV void each(const ProposalCandidate* cand, int count, const MlpTrainParams& pr, Target target) const {
-#pragma unroll
-		for (int c = 0; c != kHeld; ++c)
-			if (cluster[c] != kNone) target(cluster[c], weight[c]);
-#pragma unroll 1
-		for (int c = kHeld; c < count; ++c) {
-			const ProposalCandidate q = cand[c];
-			const uint32_t k = cluster_of(pr, q.light, q.pdf);
-			if (k != kNone) target(k, q.pdf);
-		}
-	}
-};
+// The cluster of a candidate, kNoCluster where it is no target.
+constexpr uint32_t kNoCluster = 0xffffffffu;
+RL_DEV uint32_t candidate_cluster(const MlpTrainParams& pr, int light, float w) {
+	return w > 0.0f && (uint32_t) light < pr.light_count ? pr.light_cluster[light] : kNoCluster;
+}
 
 // Where row `row`'s candidate c is staged: a row's weights in eight 16-byte
 // words and its clusters in four, permuted so that eight consecutive rows' words
@@ -210,7 +164,7 @@ template <int kRows> struct CandidateFetch {
 #pragma unroll
 		for (int k = 0; k != kBatch; ++k)
 			cluster[k] = weight[k] > 0.0f && (uint32_t) light[k] < pr.light_count ? load_here(pr.light_cluster + light[k])
-			                                                                     : HeldCandidates::kNone;
+			                                                                     : kNoCluster;
 	}
 	// clusters: 0xffff for none.
 	RL_DEV void stage(float* weights, uint16_t* clusters) const {
@@ -575,8 +529,8 @@ static __global__ void __launch_bounds__(kTtThreads, 1) mlp_train_tc_kernel(MlpT
 #pragma unroll 1
 			for (int c = kTtHeld; c < mc; ++c) {
 				const ProposalCandidate q = cand[c];
-				const uint32_t cluster = HeldCandidates::cluster_of(pr, q.light, q.pdf);
-				if (cluster != HeldCandidates::kNone && mine(cluster)) subtract(cluster, unshadowed * q.pdf);
+				const uint32_t cluster = candidate_cluster(pr, q.light, q.pdf);
+				if (cluster != kNoCluster && mine(cluster)) subtract(cluster, unshadowed * q.pdf);
 			}
 			if (chosen >= 0 && (uint32_t) chosen < pr.light_count && ss > 0.0f) {
 				const uint32_t cluster = pr.light_cluster[chosen];
