@@ -493,14 +493,12 @@ def kernel_table(prof, samples_per_step, info, fp32_peak, peaks):
     # One launch of each kernel per step (all spp frames in one call).
     kernels = {"ris_candidates_binned_kernel": {"ms_per_launch": prof["candidates"] / calls},
                "ris_sample_kernel": {"ms_per_launch": prof["shade"] / calls},
-               "light_bucket_scan_kernel + shadow_scatter_kernel": {"ms_per_launch": prof["ray_sort"] / calls},
                "shadow_trace_kernel": {"ms_per_launch": prof["shadow_trace"] / calls},
                "ris_resolve_kernel": {"ms_per_launch": prof["resolve"] / calls}}
     if info and "flops_per_sample" in info:
         kernels["ris_candidates_binned_kernel"]["flops_per_sample"] = info["candidate_flops_per_sample"]
         kernels["ris_sample_kernel"]["flops_per_sample"] = info["shade_flops_per_sample"]
         kernels["shadow_trace_kernel"]["flops_per_sample"] = info["trace_flops_per_sample"]
-        kernels["light_bucket_scan_kernel + shadow_scatter_kernel"]["flops_per_sample"] = 0.0
         kernels["ris_resolve_kernel"]["flops_per_sample"] = 0.0
         tk = kernels["shadow_trace_kernel"]
         tk["node_triangle_bytes_per_sample"] = info["trace_bytes_per_sample"]

@@ -107,9 +107,9 @@ class Context:
     def profile(self, enable=True):
         """Per-kernel CUDA-event times (ms) of the shading calls since the last
         call, then switches timing on or off.  Returns a dict: candidates
-        (or the fused kernel), shade, ray_sort (bucket scan and scatter),
-        shadow_trace and resolve (0 where the phase is not a kernel of its
-        own), and calls."""
+        (or the fused kernel), shade, ray_sort (no kernel of its own any more:
+        the rays keep pixel order), shadow_trace and resolve (0 where the phase
+        is not a kernel of its own), and calls."""
         ms = (ctypes.c_float * 5)()
         calls = ctypes.c_uint32(0)
         check(self._lib.risltc_ctx_profile(self._h, int(enable), ms, ctypes.byref(calls)), "risltc_ctx_profile")

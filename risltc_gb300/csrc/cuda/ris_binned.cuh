@@ -36,9 +36,9 @@ namespace risltc {
 
 // Blocks per SM the candidate kernel is compiled for (register budget).
 // Exact numerics 6 (80 registers): 8.46 ms per 4-frame 1080p launch with
-// 16,384 lights against 8.89 with 5, 9.30 with 4 and 9.05 with 7.  Fast
-// numerics 5: 1.71 ms per 2-frame 720p launch with 4,096 lights against 1.80
-// with 4 and 1.81 with 6.
+// 16,384 lights against 8.89 with 5, 9.30 with 4 and 9.05 with 7 (8.33 now).
+// Fast numerics 5: 1.71 ms per 2-frame 720p launch with 4,096 lights against
+// 1.80 with 4 and 1.81 with 6 (1.67 now).
 #ifndef RISLTC_BINNED_MIN_BLOCKS_EXACT
 #define RISLTC_BINNED_MIN_BLOCKS_EXACT 6
 #endif
