@@ -838,6 +838,11 @@ risltc::RisParams ris_params(const risltc_ctx_t* ctx, const Scratch& sc, const r
 	r.reservoirs = reservoirs;
 	r.error = ctx->d_error;
 	r.neg_zero = -0.0f;
+	// Small calls, up to a wave of the estimator (16 warps per SM, 32 pixels
+	// each): 64x64 through host buffers 109 instead of 113 us, 256x256 43.5
+	// instead of 46.8.  Larger ones lose: blocks that come in early fix the SM's
+	// division of L1 and shared memory (961x541, 3 frames: 2.35 against 2.29 ms).
+	r.overlap = (size_t) r.width * r.height * frame_count <= (size_t) ctx->sm_count * 16 * 32 ? 1 : 0;
 	return r;
 }
 

@@ -701,6 +701,7 @@ template <class P, int kPixels, int kChunk>
 __global__ void __launch_bounds__(32 * kBinnedWarps, BinnedMinBlocks<P>::value)
 ris_candidates_binned_kernel(const __grid_constant__ RisParams pr) {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
+	allow_next();
 	using Tile = WarpTile<BinnedSuper<P>::value, kPixels, kChunk>;
 	Tile& tile = reinterpret_cast<Tile*>(smem_raw)[threadIdx.x / 32];
 	float* const phat = pr.p_hat_scratch + (size_t) (blockIdx.x * kBinnedWarps + threadIdx.x / 32) * kPHatSlot;

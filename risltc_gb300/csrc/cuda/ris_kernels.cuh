@@ -24,6 +24,28 @@ struct ReservoirRecord {
 	uint32_t seed;  // noise state after the candidate loop
 };
 
+// A kernel launched with launch_behind and `overlap` may start while the kernel
+// before it in its stream drains: wait_for_previous is its first statement and
+// returns when that kernel is complete and its writes are visible.  allow_next,
+// in the kernel before, lets the next one's blocks come in as its own leave (a
+// kernel that was itself launched so must wait first).
+RL_DEV void wait_for_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+RL_DEV void allow_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+template <class... Params, class... Args>
+inline cudaError_t launch_behind(bool overlap, void (*kernel)(Params...), int grid, int threads, cudaStream_t stream,
+                                 Args... args) {
+	cudaLaunchAttribute attribute = {};
+	attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attribute.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t config = {};
+	config.gridDim = dim3((unsigned) grid);
+	config.blockDim = dim3((unsigned) threads);
+	config.stream = stream;
+	config.attrs = &attribute;
+	config.numAttrs = overlap ? 1 : 0;
+	return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
 // The warp's next tile from the launch's cursor (lane 0 takes it, the warp
 // shares it): warps take tiles as they finish the previous one, so no warp
 // is left with a tail of tiles while the others idle.
@@ -98,6 +120,7 @@ struct RisParams {
 	risltc_reservoir_t* reservoirs;
 	uint32_t* error;
 	float neg_zero;  // -0: the addend of PairExact::mul, unknown to the code generator
+	uint32_t overlap;  // the call's kernels may start while the one before drains (launch_behind)
 };
 
 // Sum of integrate_edge over the n edges of an unclipped polygon in slot

@@ -277,6 +277,7 @@ template <class P, bool kUniform> RL_DEV void sample_pixel(const RisParams& pr, 
 // Each warp takes 32 consecutive pixels at a time from the launch's cursor.
 template <class P, bool kUniform>
 __global__ void __launch_bounds__(kSampleThreads, RISLTC_SAMPLE_MIN_BLOCKS) ris_sample_kernel(const __grid_constant__ RisParams pr) {
+	wait_for_previous();
 	__shared__ PsaPolygon poly[kSampleThreads];
 	const uint32_t np = pr.width * pr.height;
 	const uint32_t chunks = (np + 31) / 32;
@@ -353,6 +354,7 @@ template <class P> RL_DEV void estimate_pixel(const RisParams& pr, uint32_t i, P
 // 24.8 against 25.4 us at 256x256 (one partial wave).
 template <class P>
 __global__ void __launch_bounds__(kSampleThreads, RISLTC_SAMPLE_MIN_BLOCKS) ris_estimate_kernel(const __grid_constant__ RisParams pr) {
+	wait_for_previous();
 	__shared__ PsaPolygon poly[kSampleThreads];
 	const uint32_t np = pr.width * pr.height;
 	const uint32_t chunks = (np + 31) / 32;
@@ -436,6 +438,7 @@ struct ShadowQueue {
 template <class P>
 __global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_kernel(SceneView s, const ShadowRay* rays,
                                                            uint32_t count, uint32_t* cursor, uint8_t* hits, uint32_t* error) {
+	allow_next();
 	trace_queue<P>(s, ShadowQueue{rays, hits}, count, cursor, error);
 }
 
@@ -527,6 +530,7 @@ template <class P> RL_DEV void resolve_pixel(const RisParams& pr, uint32_t i) {
 }
 
 template <class P> __global__ void __launch_bounds__(128) ris_resolve_kernel(const __grid_constant__ RisParams pr) {
+	wait_for_previous();
 	const uint32_t np = pr.width * pr.height;
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x)
 		resolve_pixel<P>(pr, i);
