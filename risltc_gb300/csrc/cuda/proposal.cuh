@@ -141,8 +141,10 @@ static __global__ void __launch_bounds__(32 * kProposalWarps, kProposalBlocks) p
 		in.skip = pr.primitive && pr.primitive[p] == 0xffffffffu;
 		if (pr.logits) {
 			const __nv_bfloat16* row = pr.logits + (size_t) p * k_count + k0;
-			if (per_lane == kLogitCache && k_count % kLogitCache == 0) {
-				// The lane's 8 logits in one 16-byte load.
+			if (per_lane == kLogitCache && k_count % kLogitCache == 0 && k0 < k_count) {
+				// The lane's 8 logits in one 16-byte load (its block lies wholly
+				// in the row; the last lanes' blocks of 232, 240 and 248 clusters
+				// lie wholly past it, in the next pixel's row or past the buffer).
 				const uint4 q = __ldg(reinterpret_cast<const uint4*>(row));
 				const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
