@@ -478,11 +478,14 @@ template <> RL_DEV void deferred_candidate<FastNumerics>(const float4* f, const 
 }
 
 // The reservoir's test rnd < w / w_sum (insert_in_reservoir) for w > 0: the
-// division is needed only where rnd * w_sum lies within 2^-20 of w, or where
-// a product might leave the normal range.
+// division is needed only where t = rnd * w_sum lies within 2^-20 of w, or out
+// of the range in which t and w / w_sum are sure to be normal numbers.  With t
+// normal, t < w means a quotient above rnd, which is a multiple of 2^-32 and not
+// 0 then; t > w means that the rounded quotient, however small, is below rnd.
+// (A rnd of 0 is refused only where the quotient underflows to 0: it divides.)
 template <class P> RL_DEV bool reservoir_accepts(float rnd, float w, float w_sum) {
 	const float t = rnd * w_sum;
-	const bool normal = w > 1e-25f && w_sum < 1e30f;
+	const bool normal = t > 1e-25f && w_sum < 1e30f;
 	if (normal && t < w * (1.0f - 0x1p-20f)) return true;
 	if (normal && t > w * (1.0f + 0x1p-20f)) return false;
 	return rnd < P::div(w, w_sum);
