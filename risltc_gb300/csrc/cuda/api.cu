@@ -31,6 +31,10 @@ struct risltc_ctx_s {
 	cudaStream_t stream;
 	int sm_count;
 	uint32_t* d_error;  // the error word, then the fetch cursor of risltc_trace_shadow
+	// The counters of risltc_shade calls' launches (allocated with the context:
+	// a captured call's graph refers to them, and risltc_ctx_ray_count reads the
+	// last call's).
+	risltc::LaunchCounters* d_counters;
 	// Staging for risltc_shade_host, grown on demand.
 	float* d_gbuffer;
 	uint32_t* d_primitive;
@@ -60,9 +64,9 @@ struct risltc_ctx_s {
 	risltc::ShadowRay* d_rays;
 	uint8_t* d_hits;
 	size_t wavefront_capacity;
-	// The launches' counters: one set per frame set of a call.
-	risltc::LaunchCounters* d_counters;
-	size_t counter_capacity;
+	// The counters of risltc_shade_batch calls' launches, one set per frame set.
+	risltc::LaunchCounters* d_batch_counters;
+	size_t batch_counter_capacity;
 	// The scratch of uniform-light calls with queued shadow rays
 	// (uniform_scratch).
 	void* d_uniform;
@@ -83,8 +87,8 @@ struct risltc_ctx_s {
 	// Kernels of this library launched through the context (risltc_ctx_launch_count).
 	uint64_t kernel_launches;
 	// Where the last risltc_shade call queued its shadow rays, whose number
-	// risltc_ctx_ray_count reports: 0 nowhere, 1 the queue of d_counters[0], 2
-	// that of d_uniform.
+	// risltc_ctx_ray_count reports: 0 nowhere, 1 the queue of d_counters, 2 that
+	// of d_uniform.
 	int rays_queued;
 	int events_created;
 };
@@ -227,16 +231,16 @@ std::vector<float> child_pair_nodes(const float* nodes, uint32_t node_count) {
 	return out;
 }
 
-int reserve_counters(risltc_ctx_t* ctx, size_t sets) {
-	if (sets <= ctx->counter_capacity) return RISLTC_OK;
+int reserve_batch_counters(risltc_ctx_t* ctx, size_t sets) {
+	if (sets <= ctx->batch_counter_capacity) return RISLTC_OK;
 	cudaSetDevice(ctx->device);
 	cudaStreamSynchronize(ctx->stream);
-	cudaFree(ctx->d_counters);
-	ctx->d_counters = nullptr;
-	ctx->counter_capacity = 0;
-	const cudaError_t e = cudaMalloc(&ctx->d_counters, sets * sizeof(risltc::LaunchCounters));
+	cudaFree(ctx->d_batch_counters);
+	ctx->d_batch_counters = nullptr;
+	ctx->batch_counter_capacity = 0;
+	const cudaError_t e = cudaMalloc(&ctx->d_batch_counters, sets * sizeof(risltc::LaunchCounters));
 	if (e != cudaSuccess) return cuda_status(e);
-	ctx->counter_capacity = sets;
+	ctx->batch_counter_capacity = sets;
 	return RISLTC_OK;
 }
 
@@ -275,7 +279,8 @@ EXTERN_C int risltc_ctx_create(risltc_ctx_t** out, int device, void* stream) {
 	ctx->stream = (cudaStream_t) stream;
 	cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device);
 	if ((e = cudaMalloc(&ctx->d_error, 2 * sizeof(uint32_t))) != cudaSuccess ||
-	    (e = cudaMemsetAsync(ctx->d_error, 0, 2 * sizeof(uint32_t), ctx->stream)) != cudaSuccess) {
+	    (e = cudaMemsetAsync(ctx->d_error, 0, 2 * sizeof(uint32_t), ctx->stream)) != cudaSuccess ||
+	    (e = cudaMalloc(&ctx->d_counters, sizeof(risltc::LaunchCounters))) != cudaSuccess) {
 		cudaFree(ctx->d_error);
 		free(ctx);
 		return cuda_status(e);
@@ -302,6 +307,7 @@ EXTERN_C void risltc_ctx_destroy(risltc_ctx_t* ctx) {
 	cudaFree(ctx->d_rays);
 	cudaFree(ctx->d_hits);
 	cudaFree(ctx->d_counters);
+	cudaFree(ctx->d_batch_counters);
 	for (int i = 0; i < ctx->batch_streams_created; ++i) {
 		cudaStreamDestroy(ctx->batch_streams[i]);
 		cudaEventDestroy(ctx->batch_join[i]);
@@ -1013,7 +1019,6 @@ int shade_on_context(risltc_ctx_t* ctx, const risltc_scene_t* scene, const rislt
 	if (uses_ris_pipeline(settings)) {
 		if ((st = reserve_records(ctx, pixel_frames))) return st;
 		if ((st = reserve_phat(ctx, 1))) return st;
-		if ((st = reserve_counters(ctx, 1))) return st;
 		if (uses_ray_queue(scene, settings, pixel_frames) && (st = reserve_wavefront(ctx, pixel_frames))) return st;
 	}
 	Scratch sc{ctx->d_records, ctx->d_phat, ctx->d_candidates, ctx->d_logits,
@@ -1214,7 +1219,7 @@ int shade_batch_fused(risltc_ctx_t* ctx, const risltc_batch_item_t* items, uint3
 		memset(&b, 0, sizeof(b));
 		b.count = gn;
 		b.p_hat_scratch = ctx->d_phat;
-		b.counters = ctx->d_counters + item_count;
+		b.counters = ctx->d_batch_counters + item_count;
 		uint32_t tiles = 0, pixels = 0, pfs = 0;
 		for (uint32_t k = 0; k != gn; ++k) {
 			const risltc_batch_item_t& it = items[g0 + k];
@@ -1226,7 +1231,7 @@ int shade_batch_fused(risltc_ctx_t* ctx, const risltc_batch_item_t* items, uint3
 			sc.samples = ctx->d_samples + w_off;
 			sc.rays = ctx->d_rays + 2 * w_off;
 			sc.hits = ctx->d_hits + 2 * w_off;
-			sc.counters = ctx->d_counters + g0 + k;
+			sc.counters = ctx->d_batch_counters + g0 + k;
 			b.item[k] = ris_params(ctx, sc, it.scene, &it.gbuffer, &it.settings, it.noise->random_seed, it.animate,
 			                       it.frame_count, it.out_rgb, it.accum, it.reservoirs, true);
 			b.tile_begin[k] = tiles;
@@ -1242,8 +1247,8 @@ int shade_batch_fused(risltc_ctx_t* ctx, const risltc_batch_item_t* items, uint3
 		b.pixel_begin[gn] = pixels;
 		b.ray_begin[gn] = 2 * pfs;
 		// The counters of this group's items, of the later ones and of the batch.
-		cudaError_t e = cudaMemsetAsync(ctx->d_counters + g0, 0, (item_count - g0 + 1) * sizeof(risltc::LaunchCounters),
-		                                ctx->stream);
+		cudaError_t e = cudaMemsetAsync(ctx->d_batch_counters + g0, 0,
+		                                (item_count - g0 + 1) * sizeof(risltc::LaunchCounters), ctx->stream);
 		if (e == cudaSuccess)
 			e = fast ? risltc::launch_candidates_batch_fast(b, ctx->stream, ctx->sm_count * 16, (int) tile)
 			         : risltc::launch_candidates_batch_exact(b, ctx->stream, ctx->sm_count * 16, (int) tile);
@@ -1285,7 +1290,7 @@ EXTERN_C int risltc_shade_batch(risltc_ctx_t* ctx, const risltc_batch_item_t* it
 	if (candidates && (st = reserve_candidates(ctx, candidates))) return st;
 	if (logits && (st = reserve_logits(ctx, logits))) return st;
 	// One more set of counters than items: the whole batch's cursors.
-	if (records && (st = reserve_counters(ctx, (size_t) item_count + 1))) return st;
+	if (records && (st = reserve_batch_counters(ctx, (size_t) item_count + 1))) return st;
 	if (wavefront && (st = reserve_wavefront(ctx, wavefront))) return st;
 	if (batch_is_fused(items, item_count)) return shade_batch_fused(ctx, items, item_count);
 	cudaError_t e = cudaSuccess;
@@ -1311,7 +1316,7 @@ EXTERN_C int risltc_shade_batch(risltc_ctx_t* ctx, const risltc_batch_item_t* it
 		if (uses_ris_pipeline(&it.settings)) {
 			sc.records = ctx->d_records + r_off;
 			sc.p_hat = ctx->d_phat + phat_region_floats(ctx) * (i % RISLTC_BATCH_STREAMS);
-			sc.counters = ctx->d_counters + i;
+			sc.counters = ctx->d_batch_counters + i;
 			r_off += pf;
 		}
 		if (uses_proposal(&it.settings)) {
