@@ -490,7 +490,9 @@ EXTERN_C void risltc_scene_destroy(risltc_scene_t* scene);
  * uniformly drawn light, projected solid angle samples and shadow rays grow
  * scratch of their own (146 bytes per pixel and frame); where it cannot be
  * had, beyond 2^26 pixel-frames and while the stream is being captured they
- * run without it, with the same results, more slowly. */
+ * run without it, with the same results, more slowly.  It is given back when
+ * another allocation of the context finds no memory; a size that found none,
+ * or was given back, is not tried again. */
 EXTERN_C int risltc_ctx_reserve(risltc_ctx_t* ctx, uint32_t width, uint32_t height, uint32_t frame_count);
 
 /* Shades frame_count consecutive frames of the G-buffer (device pointers).
@@ -643,6 +645,11 @@ EXTERN_C int risltc_ctx_check(risltc_ctx_t* ctx);
 #define RISLTC_FAULT_TENSOR_WAIT 1u
 /* The same for the next tensor-core training launch. */
 #define RISLTC_FAULT_TRAIN_TENSOR_WAIT 2u
+/* The next device allocation of the context finds no memory at its first
+   attempt, and with the second bit also after the uniform-light scratch has
+   been given back for it. */
+#define RISLTC_FAULT_ALLOCATION 4u
+#define RISLTC_FAULT_ALLOCATION_RETRY 8u
 EXTERN_C int risltc_ctx_inject_fault(risltc_ctx_t* ctx, uint32_t faults);
 EXTERN_C const char* risltc_status_string(int status);
 

@@ -97,11 +97,14 @@ class Context:
     def check(self):
         check(self._lib.risltc_ctx_check(self._h), "risltc_ctx_check")
 
-    def inject_fault(self, tensor_wait=False, train_tensor_wait=False):
+    def inject_fault(self, tensor_wait=False, train_tensor_wait=False, allocation=False, allocation_retry=False):
         """risltc_ctx_inject_fault: host-made faults for tests of the failure
         paths (see include/risltc.h): the next logits launch (tensor_wait) or
-        tensor-core training launch (train_tensor_wait) issues no products."""
-        faults = (1 if tensor_wait else 0) | (2 if train_tensor_wait else 0)
+        tensor-core training launch (train_tensor_wait) issues no products; the
+        next device allocation finds no memory (allocation), also when it is
+        tried again (allocation_retry)."""
+        faults = ((1 if tensor_wait else 0) | (2 if train_tensor_wait else 0) | (4 if allocation else 0)
+                  | (8 if allocation_retry else 0))
         check(self._lib.risltc_ctx_inject_fault(self._h, faults), "risltc_ctx_inject_fault")
 
     def profile(self, enable=True):

@@ -31,9 +31,10 @@ struct risltc_ctx_s {
 	cudaStream_t stream;
 	int sm_count;
 	uint32_t* d_error;  // the error word, then the fetch cursor of risltc_trace_shadow
-	// The counters of risltc_shade calls' launches (allocated with the context:
-	// a captured call's graph refers to them, and risltc_ctx_ray_count reads the
-	// last call's).
+	// The counters of risltc_shade calls' launches, of default calls and of
+	// uniform-light ones (allocated with the context: a captured default call's
+	// graph refers to the first set, and risltc_ctx_ray_count reads the last
+	// call's).
 	risltc::LaunchCounters* d_counters;
 	// Staging for risltc_shade_host, grown on demand.
 	float* d_gbuffer;
@@ -68,9 +69,11 @@ struct risltc_ctx_s {
 	risltc::LaunchCounters* d_batch_counters;
 	size_t batch_counter_capacity;
 	// The scratch of uniform-light calls with queued shadow rays
-	// (uniform_scratch).
+	// (uniform_scratch), and the smallest size that found no memory, or was
+	// given up for another allocation (0: none).
 	void* d_uniform;
 	size_t uniform_pixel_frames;
+	size_t uniform_refused;
 	// risltc_shade_batch: items run on these streams, forked from and joined
 	// back to the context's stream.
 	cudaStream_t batch_streams[RISLTC_BATCH_STREAMS];
@@ -87,8 +90,7 @@ struct risltc_ctx_s {
 	// Kernels of this library launched through the context (risltc_ctx_launch_count).
 	uint64_t kernel_launches;
 	// Where the last risltc_shade call queued its shadow rays, whose number
-	// risltc_ctx_ray_count reports: 0 nowhere, 1 the queue of d_counters, 2 that
-	// of d_uniform.
+	// risltc_ctx_ray_count reports: 0 nowhere, k that of d_counters[k - 1].
 	int rays_queued;
 	int events_created;
 };
@@ -142,6 +144,38 @@ int cuda_status(cudaError_t e) {
 	if (e == cudaErrorMemoryAllocation) return RISLTC_ERROR_OUT_OF_MEMORY;
 	if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver) return RISLTC_ERROR_NO_DEVICE;
 	return RISLTC_ERROR_CUDA;
+}
+
+// Device memory for the context's and its scenes' and models' buffers.  The
+// uniform-light scratch only makes calls faster: where there is no memory left
+// it is given back, and the allocation tried once more.  (Not while the stream
+// is being captured, when nothing may wait for it.)
+cudaError_t device_alloc(risltc_ctx_t* ctx, void** p, size_t bytes) {
+	const uint32_t faults = ctx->inject;
+	ctx->inject &= ~(uint32_t) (RISLTC_FAULT_ALLOCATION | RISLTC_FAULT_ALLOCATION_RETRY);
+	cudaError_t e = (faults & RISLTC_FAULT_ALLOCATION) ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+	if (e != cudaErrorMemoryAllocation) return e;
+	*p = nullptr;
+	cudaGetLastError();
+	cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+	const bool capturing = cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone;
+	if (capturing) cudaGetLastError();
+	if (ctx->d_uniform && !capturing) {
+		cudaStreamSynchronize(ctx->stream);
+		cudaFree(ctx->d_uniform);
+		ctx->d_uniform = nullptr;
+		ctx->uniform_refused = ctx->uniform_pixel_frames;
+		ctx->uniform_pixel_frames = 0;
+		e = (faults & RISLTC_FAULT_ALLOCATION_RETRY) ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+		if (e == cudaErrorMemoryAllocation) {
+			*p = nullptr;
+			cudaGetLastError();
+		}
+	}
+	return e;
+}
+template <class T> cudaError_t device_alloc(risltc_ctx_t* ctx, T** p, size_t bytes) {
+	return device_alloc(ctx, reinterpret_cast<void**>(p), bytes);
 }
 
 int grid_for(const risltc_ctx_t* ctx, size_t items) {
@@ -238,7 +272,7 @@ int reserve_batch_counters(risltc_ctx_t* ctx, size_t sets) {
 	cudaFree(ctx->d_batch_counters);
 	ctx->d_batch_counters = nullptr;
 	ctx->batch_counter_capacity = 0;
-	const cudaError_t e = cudaMalloc(&ctx->d_batch_counters, sets * sizeof(risltc::LaunchCounters));
+	const cudaError_t e = device_alloc(ctx, &ctx->d_batch_counters, sets * sizeof(risltc::LaunchCounters));
 	if (e != cudaSuccess) return cuda_status(e);
 	ctx->batch_counter_capacity = sets;
 	return RISLTC_OK;
@@ -255,9 +289,9 @@ int reserve_wavefront(risltc_ctx_t* ctx, size_t pixel_frames) {
 	ctx->d_rays = nullptr;
 	ctx->d_hits = nullptr;
 	ctx->wavefront_capacity = 0;
-	e = cudaMalloc(&ctx->d_samples, pixel_frames * sizeof(risltc::SampleRecord));
-	if (e == cudaSuccess) e = cudaMalloc(&ctx->d_rays, 2 * pixel_frames * sizeof(risltc::ShadowRay));
-	if (e == cudaSuccess) e = cudaMalloc(&ctx->d_hits, 2 * pixel_frames);
+	e = device_alloc(ctx, &ctx->d_samples, pixel_frames * sizeof(risltc::SampleRecord));
+	if (e == cudaSuccess) e = device_alloc(ctx, &ctx->d_rays, 2 * pixel_frames * sizeof(risltc::ShadowRay));
+	if (e == cudaSuccess) e = device_alloc(ctx, &ctx->d_hits, 2 * pixel_frames);
 	if (e != cudaSuccess) return cuda_status(e);
 	ctx->wavefront_capacity = pixel_frames;
 	return RISLTC_OK;
@@ -280,7 +314,7 @@ EXTERN_C int risltc_ctx_create(risltc_ctx_t** out, int device, void* stream) {
 	cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device);
 	if ((e = cudaMalloc(&ctx->d_error, 2 * sizeof(uint32_t))) != cudaSuccess ||
 	    (e = cudaMemsetAsync(ctx->d_error, 0, 2 * sizeof(uint32_t), ctx->stream)) != cudaSuccess ||
-	    (e = cudaMalloc(&ctx->d_counters, sizeof(risltc::LaunchCounters))) != cudaSuccess) {
+	    (e = cudaMalloc(&ctx->d_counters, 2 * sizeof(risltc::LaunchCounters))) != cudaSuccess) {
 		cudaFree(ctx->d_error);
 		free(ctx);
 		return cuda_status(e);
@@ -375,7 +409,7 @@ EXTERN_C int risltc_scene_create(risltc_ctx_t* ctx, const float* lights_std140, 
 	cudaError_t e = cudaSuccess;
 	auto upload = [&](void** dst, const void* src, size_t bytes) {
 		if (e != cudaSuccess || bytes == 0) return;
-		e = cudaMalloc(dst, bytes);
+		e = device_alloc(ctx, dst, bytes);
 		if (e == cudaSuccess) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
 	};
 	{
@@ -513,7 +547,7 @@ EXTERN_C int risltc_scene_set_clusters(risltc_scene_t* scene, const uint32_t* of
 	scene->clusters = risltc::ClusterView{};
 	auto upload = [&](void** dst, const void* src, size_t bytes) {
 		if (e != cudaSuccess) return;
-		e = cudaMalloc(dst, bytes);
+		e = device_alloc(scene->ctx, dst, bytes);
 		if (e == cudaSuccess) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
 	};
 	upload(&scene->d_cluster_offsets, offsets, sizeof(uint32_t) * (cluster_count + 1));
@@ -617,7 +651,7 @@ int reserve_logits(risltc_ctx_t* ctx, size_t need) {
 	cudaFree(ctx->d_logits);
 	ctx->d_logits = nullptr;
 	ctx->logit_capacity = 0;
-	cudaError_t e = cudaMalloc(&ctx->d_logits, need * sizeof(__nv_bfloat16));
+	cudaError_t e = device_alloc(ctx, &ctx->d_logits, need * sizeof(__nv_bfloat16));
 	if (e != cudaSuccess) return cuda_status(e);
 	ctx->logit_capacity = need;
 	return RISLTC_OK;
@@ -768,7 +802,7 @@ int reserve_candidates(risltc_ctx_t* ctx, size_t need) {
 	cudaFree(ctx->d_candidates);
 	ctx->d_candidates = nullptr;
 	ctx->candidate_capacity = 0;
-	cudaError_t e = cudaMalloc(&ctx->d_candidates, need * sizeof(risltc::ProposalCandidate));
+	cudaError_t e = device_alloc(ctx, &ctx->d_candidates, need * sizeof(risltc::ProposalCandidate));
 	if (e != cudaSuccess) return cuda_status(e);
 	ctx->candidate_capacity = need;
 	return RISLTC_OK;
@@ -786,7 +820,7 @@ int reserve_phat(risltc_ctx_t* ctx, int regions) {
 	cudaFree(ctx->d_phat);
 	ctx->d_phat = nullptr;
 	ctx->phat_regions = 0;
-	cudaError_t e = cudaMalloc(&ctx->d_phat, sizeof(float) * phat_region_floats(ctx) * regions);
+	cudaError_t e = device_alloc(ctx, &ctx->d_phat, sizeof(float) * phat_region_floats(ctx) * regions);
 	if (e != cudaSuccess) return cuda_status(e);
 	ctx->phat_regions = regions;
 	return RISLTC_OK;
@@ -799,7 +833,7 @@ int reserve_records(risltc_ctx_t* ctx, size_t need) {
 	cudaFree(ctx->d_records);
 	ctx->d_records = nullptr;
 	ctx->record_capacity = 0;
-	cudaError_t e = cudaMalloc(&ctx->d_records, need * sizeof(risltc::ReservoirRecord));
+	cudaError_t e = device_alloc(ctx, &ctx->d_records, need * sizeof(risltc::ReservoirRecord));
 	if (e != cudaSuccess) return cuda_status(e);
 	ctx->record_capacity = need;
 	return RISLTC_OK;
@@ -927,7 +961,7 @@ int shade_one(risltc_ctx_t* ctx, cudaStream_t stream, const Scratch& sc, const r
 					cudaFree(mm->d_shaded);
 					mm->d_shaded = nullptr;
 					mm->shaded_capacity = 0;
-					if ((e = cudaMalloc(&mm->d_shaded, pixels * sizeof(float))) != cudaSuccess) return cuda_status(e);
+					if ((e = device_alloc(ctx, &mm->d_shaded, pixels * sizeof(float))) != cudaSuccess) return cuda_status(e);
 					mm->shaded_capacity = pixels;
 				}
 				r.train_shaded = mm->d_shaded;
@@ -972,8 +1006,9 @@ int check_shade_call(const risltc_ctx_t* ctx, const risltc_scene_t* scene, const
 // The scratch of may_queue_uniform's route into sc, an allocation of its own:
 // such a call must not move the scratch that a captured frame of the default
 // configuration refers to.  False where the route is not to be taken: no
-// memory, or the stream is being captured into a graph (which then needs no
-// scratch that a later, larger call would move).
+// memory (not tried again at a size that found none), or the stream is being
+// captured into a graph (which then needs no scratch that a later, larger call
+// would move, or that is given back).
 bool uniform_scratch(risltc_ctx_t* ctx, size_t pixel_frames, Scratch& sc) {
 	cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
 	if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
@@ -981,22 +1016,32 @@ bool uniform_scratch(risltc_ctx_t* ctx, size_t pixel_frames, Scratch& sc) {
 		return false;
 	}
 	if (pixel_frames > ctx->uniform_pixel_frames) {
-		cudaStreamSynchronize(ctx->stream);
-		cudaFree(ctx->d_uniform);
-		ctx->d_uniform = nullptr;
-		ctx->uniform_pixel_frames = 0;
-		if (cudaMalloc(&ctx->d_uniform, 256 + pixel_frames * (sizeof(risltc::SampleRecord) + 2 * sizeof(risltc::ShadowRay) +
-		                                                      sizeof(risltc::ReservoirRecord) + 2)) != cudaSuccess) {
-			cudaGetLastError();
-			ctx->d_uniform = nullptr;
+		if (ctx->uniform_refused && pixel_frames >= ctx->uniform_refused) return false;
+		auto bytes = [](size_t pf) {
+			return pf * (sizeof(risltc::SampleRecord) + 2 * sizeof(risltc::ShadowRay) + sizeof(risltc::ReservoirRecord) + 2);
+		};
+		// The larger block first: where there is none the smaller one is still
+		// there, or, having been given back in the attempt, is taken again.
+		const size_t before = ctx->uniform_pixel_frames;
+		void* block = nullptr;
+		if (device_alloc(ctx, &block, bytes(pixel_frames)) != cudaSuccess) {
+			if (before && !ctx->d_uniform && device_alloc(ctx, &ctx->d_uniform, bytes(before)) == cudaSuccess)
+				ctx->uniform_pixel_frames = before;
+			ctx->uniform_refused = ctx->d_uniform || !before ? pixel_frames : before;
 			return false;
 		}
+		if (ctx->d_uniform) {
+			cudaStreamSynchronize(ctx->stream);
+			cudaFree(ctx->d_uniform);
+		}
+		ctx->d_uniform = block;
 		ctx->uniform_pixel_frames = pixel_frames;
+		ctx->uniform_refused = 0;
 	}
-	// 256 bytes for the counters, then the arrays by falling alignment.
+	// The arrays by falling alignment.
 	const size_t pf = ctx->uniform_pixel_frames;
-	sc.counters = static_cast<risltc::LaunchCounters*>(ctx->d_uniform);
-	sc.samples = reinterpret_cast<risltc::SampleRecord*>(static_cast<char*>(ctx->d_uniform) + 256);
+	sc.counters = ctx->d_counters + 1;
+	sc.samples = static_cast<risltc::SampleRecord*>(ctx->d_uniform);
 	sc.rays = reinterpret_cast<risltc::ShadowRay*>(sc.samples + pf);
 	sc.records = reinterpret_cast<risltc::ReservoirRecord*>(sc.rays + 2 * pf);
 	sc.hits = reinterpret_cast<uint8_t*>(sc.records + pf);
@@ -1362,9 +1407,9 @@ static int ensure_staging(risltc_ctx_t* ctx, size_t pixels) {
 	ctx->d_primitive = nullptr;
 	ctx->d_rgb = nullptr;
 	ctx->pixel_capacity = 0;
-	cudaError_t e = cudaMalloc(&ctx->d_gbuffer, pixels * RISLTC_GBUFFER_PLANES * sizeof(float));
-	if (e == cudaSuccess) e = cudaMalloc(&ctx->d_primitive, pixels * sizeof(uint32_t));
-	if (e == cudaSuccess) e = cudaMalloc(&ctx->d_rgb, pixels * 3 * sizeof(float));
+	cudaError_t e = device_alloc(ctx, &ctx->d_gbuffer, pixels * RISLTC_GBUFFER_PLANES * sizeof(float));
+	if (e == cudaSuccess) e = device_alloc(ctx, &ctx->d_primitive, pixels * sizeof(uint32_t));
+	if (e == cudaSuccess) e = device_alloc(ctx, &ctx->d_rgb, pixels * 3 * sizeof(float));
 	if (e == cudaSuccess && !ctx->h_error) e = cudaMallocHost((void**) &ctx->h_error, sizeof(uint32_t));
 	if (e != cudaSuccess) return cuda_status(e);
 	ctx->pixel_capacity = pixels;
@@ -1427,10 +1472,9 @@ EXTERN_C int risltc_trace_shadow(risltc_ctx_t* ctx, const risltc_scene_t* scene,
 EXTERN_C int risltc_ctx_ray_count(risltc_ctx_t* ctx, uint32_t* rays) {
 	if (!ctx || !rays) return RISLTC_ERROR_INVALID_ARGUMENT;
 	*rays = 0;
-	const auto* counters = ctx->rays_queued == 2 ? static_cast<const risltc::LaunchCounters*>(ctx->d_uniform) : ctx->d_counters;
-	if (!ctx->rays_queued || !counters) return RISLTC_OK;
+	if (!ctx->rays_queued) return RISLTC_OK;
 	cudaSetDevice(ctx->device);
-	cudaError_t e = cudaMemcpyAsync(rays, &counters->rays, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream);
+	cudaError_t e = cudaMemcpyAsync(rays, &ctx->d_counters[ctx->rays_queued - 1].rays, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream);
 	if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
 	return cuda_status(e);
 }
@@ -1465,7 +1509,8 @@ EXTERN_C int risltc_ctx_profile(risltc_ctx_t* ctx, int enable, float* phase_ms, 
 }
 
 EXTERN_C int risltc_ctx_inject_fault(risltc_ctx_t* ctx, uint32_t faults) {
-	if (!ctx || (faults & ~(uint32_t) (RISLTC_FAULT_TENSOR_WAIT | RISLTC_FAULT_TRAIN_TENSOR_WAIT)))
+	if (!ctx || (faults & ~(uint32_t) (RISLTC_FAULT_TENSOR_WAIT | RISLTC_FAULT_TRAIN_TENSOR_WAIT | RISLTC_FAULT_ALLOCATION |
+	                                          RISLTC_FAULT_ALLOCATION_RETRY)))
 		return RISLTC_ERROR_INVALID_ARGUMENT;
 	ctx->inject |= faults;
 	return RISLTC_OK;
@@ -1527,13 +1572,13 @@ EXTERN_C int risltc_model_create(risltc_ctx_t* ctx, uint32_t cluster_count, uint
 	m->parameter_count = (int) risltc_model_parameter_count(cluster_count);
 	m->inv_half_extent = 1.0f;
 	cudaSetDevice(ctx->device);
-	cudaError_t e = cudaMalloc(&m->d_params, sizeof(float) * m->parameter_count);
+	cudaError_t e = device_alloc(ctx, &m->d_params, sizeof(float) * m->parameter_count);
 	// The operand-layout weights; W3's padding rows stay zero.
 	const size_t weight_bytes = sizeof(__nv_bfloat16) * (size_t) risltc::mlp_weight_elements((int) cluster_count);
-	if (e == cudaSuccess) e = cudaMalloc(&m->d_weights, weight_bytes);
+	if (e == cudaSuccess) e = device_alloc(ctx, &m->d_weights, weight_bytes);
 	if (e == cudaSuccess) e = cudaMemset(m->d_weights, 0, weight_bytes);
 	for (float** buf : {&m->d_grad, &m->d_adam_m, &m->d_adam_v}) {
-		if (e == cudaSuccess) e = cudaMalloc(buf, sizeof(float) * m->parameter_count);
+		if (e == cudaSuccess) e = device_alloc(ctx, buf, sizeof(float) * m->parameter_count);
 		if (e == cudaSuccess) e = cudaMemset(*buf, 0, sizeof(float) * m->parameter_count);
 	}
 	m->learning_rate = 1e-3f;
