@@ -600,7 +600,9 @@ EXTERN_C int risltc_shade_noalloc(const risltc_scene_t* scene, const risltc_gbuf
 
 /* Any-hit shadow queries through the scene BVH: rays are 8 floats
    {origin xyz, t_min, direction xyz, t_max} in device memory; hits gets
-   1 (occluded) or 0 per ray. */
+   1 (occluded) or 0 per ray.  Beyond one wave of rays the context's stream
+   orders its calls (they share a cursor); a call captured into a graph has no
+   such state, and its graph may be replayed beside them on any stream. */
 EXTERN_C int risltc_trace_shadow(risltc_ctx_t* ctx, const risltc_scene_t* scene, const float* rays, uint32_t ray_count,
                                  uint32_t* hits);
 

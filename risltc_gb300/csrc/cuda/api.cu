@@ -23,7 +23,7 @@ namespace risltc {
 cudaError_t launch_proposal(const ProposalParams& p, cudaStream_t stream, int grid);
 cudaError_t launch_shade(const ShadeParams& p, cudaStream_t stream, int grid, cudaEvent_t* events, bool fast);
 cudaError_t launch_trace_exact(const SceneView& s, const float4* rays, uint32_t count, uint32_t* hits, uint32_t* error,
-                               uint32_t* cursor, cudaStream_t stream, int grid, int resident);
+                               uint32_t* cursor, cudaStream_t stream, int resident);
 }  // namespace risltc
 
 struct risltc_ctx_s {
@@ -1462,9 +1462,19 @@ EXTERN_C int risltc_trace_shadow(risltc_ctx_t* ctx, const risltc_scene_t* scene,
 	if (!ctx || !scene || (ray_count && (!rays || !hits))) return RISLTC_ERROR_INVALID_ARGUMENT;
 	if (ray_count == 0) return RISLTC_OK;
 	cudaSetDevice(ctx->device);
-	const int blocks = (int) (((size_t) ray_count + 127) / 128);
-	cudaError_t e = risltc::launch_trace_exact(scene->view, (const float4*) rays, ray_count, hits, ctx->d_error,
-	                                           ctx->d_error + 1, ctx->stream, blocks, ctx->sm_count * kTraceBlocksPerSm);
+	// A captured call takes no cursor of the context's: its graph may run beside
+	// the context's other calls, on any stream.
+	const int resident = ctx->sm_count * kTraceBlocksPerSm;
+	uint32_t* cursor = nullptr;
+	if ((uint64_t) ray_count > (uint64_t) resident * 128) {
+		cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+		if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess)
+			cudaGetLastError();
+		else if (capture == cudaStreamCaptureStatusNone)
+			cursor = ctx->d_error + 1;
+	}
+	cudaError_t e = risltc::launch_trace_exact(scene->view, (const float4*) rays, ray_count, hits, ctx->d_error, cursor,
+	                                           ctx->stream, resident);
 	if (e == cudaSuccess) ctx->kernel_launches += 1;
 	return cuda_status(e);
 }

@@ -65,19 +65,24 @@ cudaError_t launch_batch_estimator(const RisBatch& b, cudaStream_t stream, int p
 	ris_resolve_batch_kernel<ExactNumerics><<<pixel_grid, 128, 0, stream>>>(b);
 	return cudaGetLastError();
 }
-// One thread per ray while all of them are resident at once (grid blocks of
-// 128), the persistent queue beyond that, whose cursor is zeroed first: 2M rays
-// against 200k occluders took 831 us with a thread per ray, 667 with the queue
-// when it was brought in and 576 with the present traversal.
+// One thread per ray while all of them are resident at once (blocks of 128),
+// the persistent queue beyond that, whose cursor (if any) is zeroed first: 2M
+// rays against 200k occluders took 831 us with a thread per ray, 667 with the
+// queue when it was brought in and 576 with the present traversal.
 cudaError_t launch_trace_exact(const SceneView& s, const float4* rays, uint32_t count, uint32_t* hits, uint32_t* error,
-                               uint32_t* cursor, cudaStream_t stream, int grid, int resident) {
+                               uint32_t* cursor, cudaStream_t stream, int resident) {
+	const int grid = (int) (((size_t) count + 127) / 128);
 	if (grid <= resident) {
 		trace_shadow_kernel<ExactNumerics><<<grid, 128, 0, stream>>>(s, rays, count, hits, error);
 		return cudaGetLastError();
 	}
+	if (!cursor) {
+		trace_shadow_queue_kernel<ExactNumerics, false><<<resident, 128, 0, stream>>>(s, rays, count, hits, cursor, error);
+		return cudaGetLastError();
+	}
 	const cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(uint32_t), stream);
 	if (e != cudaSuccess) return e;
-	trace_shadow_queue_kernel<ExactNumerics><<<resident, 128, 0, stream>>>(s, rays, count, hits, cursor, error);
+	trace_shadow_queue_kernel<ExactNumerics, true><<<resident, 128, 0, stream>>>(s, rays, count, hits, cursor, error);
 	return cudaGetLastError();
 }
 }  // namespace risltc

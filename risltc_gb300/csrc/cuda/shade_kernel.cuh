@@ -568,11 +568,12 @@ template <class C, class P> __global__ void __launch_bounds__(kShadeThreads) sha
 	}
 }
 
-// Batch of independent any-hit queries (risltc_trace_shadow).
+// Batch of independent any-hit queries (risltc_trace_shadow), a thread per ray.
 template <class P>
 __global__ void __launch_bounds__(128) trace_shadow_kernel(SceneView s, const float4* rays, uint32_t count,
                                                           uint32_t* hits, uint32_t* error) {
-	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i < count) {
 		float4 a = rays[2 * (size_t) i], b = rays[2 * (size_t) i + 1];
 		hits[i] = any_hit<P>(s, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), a.w, b.w, error) ? 1u : 0u;
 	}
