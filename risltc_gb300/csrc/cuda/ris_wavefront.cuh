@@ -459,6 +459,11 @@ __global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_ker
 	trace_queue<P, true>(s, ShadowQueue{rays, hits}, count, cursor, error);
 }
 
+// Whether a 32-bit cursor can deal out `rays` to `threads` threads: after the
+// last ray each warp may add up to 32 once more, and a cursor that wrapped there
+// would deal the first rays out again, and again after them.
+constexpr bool cursor_holds(uint32_t rays, uint32_t threads) { return rays <= 0xffffffffu - threads; }
+
 // A caller's rays (risltc_trace_shadow).
 struct CallerQueue {
 	const float4* rays;

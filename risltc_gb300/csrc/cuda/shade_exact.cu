@@ -66,8 +66,8 @@ cudaError_t launch_batch_estimator(const RisBatch& b, cudaStream_t stream, int p
 	return cudaGetLastError();
 }
 // One thread per ray while all of them are resident at once (blocks of 128),
-// the persistent queue beyond that, whose cursor (if any) is zeroed first: 2M
-// rays against 200k occluders took 831 us with a thread per ray, 667 with the
+// the persistent queue beyond that, whose cursor (if any that holds the count)
+// is zeroed first: 2M rays against 200k occluders took 831 us with a thread per ray, 667 with the
 // queue when it was brought in and 576 with the present traversal.
 cudaError_t launch_trace_exact(const SceneView& s, const float4* rays, uint32_t count, uint32_t* hits, uint32_t* error,
                                uint32_t* cursor, cudaStream_t stream, int resident) {
@@ -76,7 +76,7 @@ cudaError_t launch_trace_exact(const SceneView& s, const float4* rays, uint32_t 
 		trace_shadow_kernel<ExactNumerics><<<grid, 128, 0, stream>>>(s, rays, count, hits, error);
 		return cudaGetLastError();
 	}
-	if (!cursor) {
+	if (!cursor || !cursor_holds(count, (uint32_t) resident * 128)) {
 		trace_shadow_queue_kernel<ExactNumerics, false><<<resident, 128, 0, stream>>>(s, rays, count, hits, cursor, error);
 		return cudaGetLastError();
 	}
