@@ -530,9 +530,10 @@ typedef struct risltc_batch_item_s {
  * and one sample per technique, uniform candidates, shadows on a scene with
  * occluders) with the same numerics and a binned tile shape, the batch runs
  * as one launch per phase for all items (candidate, sample, trace and
- * resolve kernels over the items' concatenated work, in groups of 8 items) on the context's stream; otherwise each item runs its own
- * kernels on one of RISLTC_BATCH_STREAMS streams forked from the context's
- * stream and joined back to it.  Either way small frames fill the GPU
+ * resolve kernels over the items' concatenated work); more than 8 items run as
+ * groups of 8 beside each other; otherwise each item runs its own kernels.
+ * Groups and items run on RISLTC_BATCH_STREAMS streams forked from the
+ * context's stream and joined back to it, a single group on that stream.  Either way small frames fill the GPU
  * together and the results equal the items' risltc_shade calls bit for bit.
  * All items are validated before any work; noise->random_seed of each item
  * advances by its frame_count.  The first call grows the scratch (and creates
