@@ -839,6 +839,12 @@ int reserve_records(risltc_ctx_t* ctx, size_t need) {
 	return RISLTC_OK;
 }
 
+// Whether a queue for the rays of so many pixel-frames is dealt out by shares and
+// without background (kSharesPerLane).
+bool is_large_queue(const risltc_ctx_t* ctx, size_t pixel_frames) {
+	return 2 * pixel_frames >= (size_t) ctx->sm_count * RISLTC_TRACE_MIN_BLOCKS * 128 * risltc::kSharesPerLane;
+}
+
 // The parameters of the candidate/estimator kernels of one frame set of the
 // default configuration (LTC-CP, reservoir, one light sample) with its
 // share of the scratch: the reservoir records, p_hat slots and, with the ray
@@ -872,6 +878,7 @@ risltc::RisParams ris_params(const risltc_ctx_t* ctx, const Scratch& sc, const r
 		r.samples = sc.samples;
 		r.rays = sc.rays;
 		r.hits = sc.hits;
+		r.compact = !r.uniform_light && is_large_queue(ctx, (size_t) r.width * r.height * frame_count) ? 1 : 0;
 	}
 	r.out_rgb = out_rgb;
 	r.accum = accum;
@@ -1334,6 +1341,7 @@ int shade_batch_fused(risltc_ctx_t* ctx, const risltc_batch_item_t* items, uint3
 		b.tile_begin[gn] = tiles;
 		b.pixel_begin[gn] = pixels;
 		b.ray_begin[gn] = 2 * pfs;
+		for (uint32_t k = 0; k != gn; ++k) b.item[k].compact = is_large_queue(ctx, pfs) ? 1 : 0;
 		cudaError_t e = cudaMemsetAsync(counters, 0, kGroupCounters * sizeof(risltc::LaunchCounters), stream);
 		if (e == cudaSuccess)
 			e = fast ? risltc::launch_candidates_batch_fast(b, stream, ctx->sm_count * 16, (int) tile)
@@ -1478,9 +1486,6 @@ EXTERN_C int risltc_shade_host(risltc_ctx_t* ctx, const risltc_scene_t* scene, u
 	return error_status(ctx, *ctx->h_error);
 }
 
-// Blocks of the query kernels that fit an SM.
-static constexpr int kTraceBlocksPerSm = 12;
-
 EXTERN_C int risltc_trace_shadow(risltc_ctx_t* ctx, const risltc_scene_t* scene, const float* rays, uint32_t ray_count,
                                  uint32_t* hits) {
 	if (!ctx || !scene || (ray_count && (!rays || !hits))) return RISLTC_ERROR_INVALID_ARGUMENT;
@@ -1488,7 +1493,7 @@ EXTERN_C int risltc_trace_shadow(risltc_ctx_t* ctx, const risltc_scene_t* scene,
 	cudaSetDevice(ctx->device);
 	// A captured call takes no cursor of the context's: its graph may run beside
 	// the context's other calls, on any stream.
-	const int resident = ctx->sm_count * kTraceBlocksPerSm;
+	const int resident = ctx->sm_count * RISLTC_TRACE_MIN_BLOCKS;
 	uint32_t* cursor = nullptr;
 	if ((uint64_t) ray_count > (uint64_t) resident * 128) {
 		cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;

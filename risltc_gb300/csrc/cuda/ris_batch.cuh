@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kSampleThreads, RISLTC_SAMPLE_MIN_BLOCKS) ris_
 	const uint32_t chunks = b.pixel_begin[b.count] / 32;
 	for (uint32_t c = next_warp_tile(&b.counters->sample); c < chunks; c = next_warp_tile(&b.counters->sample)) {
 		const uint32_t u = c * 32 + threadIdx.x % 32, k = batch_item(b.pixel_begin, b.count, c * 32);
-		sample_pixel<P, false>(b.item[k], u - b.pixel_begin[k], poly[threadIdx.x]);
+		sample_pixel<P, false>(b.item[k], u - b.pixel_begin[k], poly[threadIdx.x], has_numbers(b.item[k]));
 	}
 }
 
@@ -147,6 +147,61 @@ __global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_bat
 			}
 		}
 	}
+}
+
+// The same for many places, claimed by shares, of the items' covered pixels.
+struct BatchRays {
+	const RisBatch& b;
+	const uint32_t* begin;  // prefix sums of the items' rays
+	int shift;
+	uint2& claimed;
+	SceneView s;            // of the lane's ray: the fields that the traversal reads,
+	uint8_t* hit;           // its outcome's place
+	const ShadowRay* rays;  // and its own
+
+	RL_DEV bool deal(uint32_t idle, bool& drained) {
+		uint32_t g;
+		if (!deal_places(idle, drained, claimed, begin[b.count], shift, g, &b.counters->fetch)) return false;
+		const uint32_t k = batch_item(begin, b.count, g);
+		const RisParams& pr = b.item[k];
+		s.pairs = pr.scene.pairs;
+		s.triangles = pr.scene.triangles;
+		s.triangle_count = pr.scene.triangle_count;
+		const uint32_t n = begin[k + 1] - begin[k], pixels = pr.width * pr.height;
+		g -= begin[k];
+		// (n is 2 * covered * frames.)
+		if (n != b.ray_begin[k + 1] - b.ray_begin[k]) g = queue_place(g, n / (2u * pr.frame_count), pixels);
+		hit = pr.hits + g;
+		rays = pr.rays + g;
+		return true;
+	}
+	RL_DEV const SceneView& scene() const { return s; }
+	RL_DEV void ray(f3& o, f3& d, float& t_min, float& t_max) const {
+		const float4 a = __ldg(&rays->origin), r = __ldg(&rays->dir_tmax);
+		o = mk3(a.x, a.y, a.z);
+		d = mk3(r.x, r.y, r.z);
+		t_min = 1.0e-3f;
+		t_max = r.w;
+	}
+	RL_DEV void outcome(bool occluded) const { *hit = occluded ? 1 : 0; }
+};
+template <class P>
+__global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS)
+shadow_trace_batch_shares_kernel(const __grid_constant__ RisBatch b, int shift) {
+	__shared__ uint2 claimed[4];
+	__shared__ uint32_t begin[kBatchItems + 1];
+	claimed[threadIdx.x / 32] = make_uint2(0u, 0u);
+	if (threadIdx.x <= b.count) {
+		uint32_t sum = 0;
+		for (uint32_t k = 0; k != threadIdx.x; ++k) {
+			const RisParams& pr = b.item[k];
+			sum += 2u * queue_covered(pr.counters, pr.width * pr.height) * pr.frame_count;
+		}
+		begin[threadIdx.x] = sum;
+	}
+	__syncthreads();
+	BatchRays source{b, begin, shift, claimed[threadIdx.x / 32], SceneView{}, nullptr, nullptr};
+	trace_dealt<P>(source, b.item[0].error);
 }
 
 template <class P> __global__ void __launch_bounds__(128) ris_resolve_batch_kernel(const __grid_constant__ RisBatch b) {

@@ -302,7 +302,7 @@ RL_DEV void binned_candidate_pair(const float4* f, const float4* record, float& 
 		f3x2 next = first;
 		if (j + 1 != n) {
 			v = mul_point2<P>(t, q);
-					q = __ldg(record + kRecordVertex + min(j + 2, (uint32_t) kMaxLightVertices - 1));
+			q = __ldg(record + kRecordVertex + min(j + 2, (uint32_t) kMaxLightVertices - 1));
 			above_s |= (v.z.x > 0.0f ? 1u : 0u) << (j + 1);
 			above_c |= (v.z.y > 0.0f ? 1u : 0u) << (j + 1);
 			next = normalize2<P>(v);
@@ -520,6 +520,9 @@ RL_DEV void binned_tile(const RisParams& pr, WarpTile<BinnedSuper<P>::value, kPi
 		store_frame(tile.frame[lane], diffuse_albedo, ltc.albedo, ltc.world_to_shading,
 		            mul(ltc.shading_to_cosine, ltc.world_to_shading));
 	}
+	// Background is noted by one of its lanes, and nothing waits for that.
+	if (pr.compact && own && i < np && !valid && lane == (uint32_t) __ffs(__activemask()) - 1u)
+		atomicOr(&pr.counters->background, 1u);
 	if (lane == 0) tile.deferred_count = 0;
 	__syncwarp();
 	// The noise state at the start of frame f (get_noise_accessor with the

@@ -74,7 +74,15 @@ struct LaunchCounters {
 	uint32_t sample;  // the sample kernel's next 32 pixels
 	uint32_t rays;    // shadow rays to trace (risltc_ctx_ray_count)
 	uint32_t fetch;   // the trace kernel's next queue entry
+	// Whether some pixel is background, set by the candidate kernel, and then the
+	// number of the others (queue_place): a line apart from the cursors, which
+	// every warp's atomics keep busy.
+	alignas(128) uint32_t background;
+	uint32_t covered;
 };
+// What is zeroed before the launches of a call: all of a set only where the
+// second line is used (RisParams::compact).
+constexpr size_t kPlainCounterBytes = 4 * sizeof(uint32_t);
 
 struct RisParams {
 	SceneView scene;
@@ -100,6 +108,7 @@ struct RisParams {
 	// candidate kernel.
 	float* p_hat_scratch;
 	LaunchCounters* counters;  // null where no kernel that needs them runs
+	uint32_t compact;          // with background, number the covered pixels (queue_covered)
 	// Candidates drawn by a proposal ([frame][pixel][candidate]); null: each
 	// candidate is drawn uniformly from the pixel's noise as in the reference.
 	const ProposalCandidate* candidates;
@@ -393,7 +402,7 @@ cudaError_t launch_ris_resolve(const RisParams& p, cudaStream_t stream, int grid
 // kernel together).
 inline cudaError_t launch_ris(const RisParams& p, cudaStream_t stream, int grid, int trace_grid, cudaEvent_t* events,
                               bool fast, int tile, int grid_cap) {
-	cudaError_t e = p.counters ? cudaMemsetAsync(p.counters, 0, sizeof(LaunchCounters), stream) : cudaSuccess;
+	cudaError_t e = p.counters ? cudaMemsetAsync(p.counters, 0, p.compact ? sizeof(LaunchCounters) : kPlainCounterBytes, stream) : cudaSuccess;
 	if (e != cudaSuccess) return e;
 	if (events) cudaEventRecord(events[0], stream);
 	if (!p.uniform_light)

@@ -6,19 +6,23 @@
 //     for the chosen light up to the visibility test.  For each of its (at
 //     most two) samples it stores the MIS-weighted contribution for both
 //     outcomes of the shadow ray and puts the ray at the sample's own place
-//     in the queue.  Nearly every sample has one; where there is none the
-//     place holds an empty interval.  In this order a warp traces both rays
+//     in the queue.  Nearly every sample of a surface has one; where there is
+//     none the place holds an empty interval.  In large calls background has
+//     no places (queue_covered).  In this order a warp traces both rays
 //     of 16 neighbouring pixels: grouped by light (a counting sort, 0.68 ms
 //     of its own) they took 4.39 ms per 4-frame 1080p launch with 16,384
 //     lights, appended technique by technique 4.36, in this order 4.10 (3.36
 //     with the traversal's present form).
-//   shadow_trace_kernel: one any-hit query per queued ray, with a small
-//     register footprint and no divergence from the shading code around it.
+//   shadow_trace_kernel, and shadow_trace_shares_kernel for large calls: one
+//     any-hit query per queued ray, with a small register footprint and no
+//     divergence from the shading code around it.
 //   ris_resolve_kernel: per pixel, picks each sample's contribution by its
 //     ray's outcome and finishes the frame and the accumulation exactly as
 //     ris_shade_kernel does.
 // The contributions are the same operations on the same values, added in
 // the same order, so the pixels are bit-identical to ris_shade_kernel's.
+// ris_estimate_kernel: the sample and resolve phases in one where no shadow ray is
+// traced.
 // Used for one sample per technique (SAMPLE_COUNT == 1, the reference's
 // default) with shadows on: after the candidate kernel, or (uniform_light)
 // with one uniformly drawn light per pixel-frame, the reference's ground-truth
@@ -43,7 +47,8 @@ struct SampleRecord {
 	float c[2][2][3];  // [technique][unoccluded, occluded][rgb]
 	float W;           // the reservoir's unbiased contribution weight
 	uint32_t flags;
-	uint32_t pad[2];
+	uint32_t number;   // the pixel's in the queue
+	uint32_t pad;
 };
 static_assert(sizeof(SampleRecord) == 64, "SampleRecord layout");
 
@@ -53,11 +58,26 @@ struct ShadowRay {
 	float4 origin;
 	float4 dir_tmax;
 };
-// No ray at a place of the queue: t_max below t_min, so that the query ends at
+// No ray at a covered pixel's place: t_max below t_min, so that the query ends at
 // the root's box.
 RL_DEV void store_no_ray(ShadowRay* ray) {
 	ray->origin = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 	ray->dir_tmax = make_float4(0.0f, 0.0f, 1.0f, -1.0f);
+}
+
+// The queue's places are [frame][number][technique], with room for `pixels`
+// numbers in a frame.  A pixel's number is its index, and with background in the
+// G-buffer (noted by the candidate kernel) the covered pixels, those that are no
+// background, are numbered as the sample kernel's warps come to them, so that
+// background costs nothing.  (Numbered in every call, full frames took 0.3 to
+// 0.8% longer.)  Whether they are, and the pixels that have places:
+RL_DEV bool has_numbers(const RisParams& pr) { return pr.compact && pr.counters->background != 0; }
+RL_DEV uint32_t queue_covered(const LaunchCounters* counters, uint32_t pixels) {
+	return counters->background != 0 ? counters->covered : pixels;
+}
+// The place of ray g of the call:
+RL_DEV uint32_t queue_place(uint32_t g, uint32_t covered, uint32_t pixels) {
+	return covered == pixels ? g : g + g / (2u * covered) * (2u * (pixels - covered));
 }
 
 // Technique j's two contributions (unoccluded, occluded) into floats
@@ -212,7 +232,8 @@ constexpr int kSampleThreads = 128;
 // i may be past the frame (the thread then does nothing).
 // kUniform: RisParams::uniform_light (a variant of its own: its few
 // instructions cost the other 2%).
-template <class P, bool kUniform> RL_DEV void sample_pixel(const RisParams& pr, uint32_t i, PsaPolygon& poly) {
+template <class P, bool kUniform>
+RL_DEV void sample_pixel(const RisParams& pr, uint32_t i, PsaPolygon& poly, bool numbered) {
 	const uint32_t np = pr.width * pr.height;
 	ShadeParams sp;  // the fields psa_prepare_both and psa_mis_emit read
 	sp.scene = pr.scene;
@@ -226,13 +247,22 @@ template <class P, bool kUniform> RL_DEV void sample_pixel(const RisParams& pr, 
 	sp.error = pr.error;
 	{
 		const bool active = i < np && !(pr.primitive && pr.primitive[i] == 0xffffffffu);
+		uint32_t number = i;
+		if (numbered) {
+			const uint32_t covered = __ballot_sync(0xffffffffu, active);
+			if (threadIdx.x % 32 == 0 && covered) number = atomicAdd(&pr.counters->covered, (uint32_t) __popc(covered));
+		}
 		ShadingData sd;
 		Ltc ltc;
 		if (active) {
 			load_pixel<P>(pr, i, sd, ltc);
 		}
+		if (numbered)
+			number = __shfl_sync(0xffffffffu, number, 0) +
+			         (uint32_t) __popc(__ballot_sync(0xffffffffu, active) & ((1u << threadIdx.x % 32) - 1u));
 		for (uint32_t f = 0; f != pr.frame_count; ++f) {
 			const size_t pf = (size_t) f * np + i;
+			ShadowRay* const rays = pr.rays + 2 * ((size_t) f * np + number);
 			uint32_t modes = 0;
 			if (active) {
 				ReservoirRecord r;
@@ -254,20 +284,22 @@ template <class P, bool kUniform> RL_DEV void sample_pixel(const RisParams& pr, 
 					SampleRecord* const dst = pr.samples + pf;
 					modes = psa_mis_emit<P, true>(
 					    sp, peters, sd, ltc, l, light_record(pr.scene, r.light_index), seed,
-					    [dst](int j, f3 c0, f3 c1) { store_contributions(dst, j, c0, c1); }, pr.rays + 2 * pf, poly);
+					    [dst](int j, f3 c0, f3 c1) { store_contributions(dst, j, c0, c1); }, rays, poly);
 					float W = P::div(r.w_sum, (float) pr.candidate_count * r.p_hat);
 					if (r.p_hat == 0.0f) W = 0.0f;
 					if (kUniform) W = (float) pr.scene.light_count;
 					*reinterpret_cast<float2*>(reinterpret_cast<float*>(pr.samples + pf) + 12) =
 					    make_float2(W, __uint_as_float(modes));
+					if (numbered) pr.samples[pf].number = number;
 				} else {
 					const f3 zero[2][2] = {{splat(0.0f), splat(0.0f)}, {splat(0.0f), splat(0.0f)}};
 					store_sample(pr.samples + pf, zero, 0.0f, kSampleNoLight);
 				}
 			}
 			const bool t0 = (modes & 3u) == kSampleTraced, t1 = ((modes >> 2) & 3u) == kSampleTraced;
-			if (i < np && !t0) store_no_ray(pr.rays + 2 * pf);
-			if (i < np && !t1) store_no_ray(pr.rays + 2 * pf + 1);
+			const bool place = numbered ? active : i < np;
+			if (place && !t0) store_no_ray(rays);
+			if (place && !t1) store_no_ray(rays + 1);
 			const uint32_t count = __popc(__ballot_sync(0xffffffffu, t0)) + __popc(__ballot_sync(0xffffffffu, t1));
 			if (threadIdx.x % 32 == 0 && count) atomicAdd(&pr.counters->rays, count);
 		}
@@ -281,8 +313,9 @@ __global__ void __launch_bounds__(kSampleThreads, RISLTC_SAMPLE_MIN_BLOCKS) ris_
 	__shared__ PsaPolygon poly[kSampleThreads];
 	const uint32_t np = pr.width * pr.height;
 	const uint32_t chunks = (np + 31) / 32;
+	const bool numbered = !kUniform && has_numbers(pr);
 	for (uint32_t c = next_warp_tile(&pr.counters->sample); c < chunks; c = next_warp_tile(&pr.counters->sample))
-		sample_pixel<P, kUniform>(pr, c * 32 + threadIdx.x % 32, poly[threadIdx.x]);
+		sample_pixel<P, kUniform>(pr, c * 32 + threadIdx.x % 32, poly[threadIdx.x], numbered);
 }
 
 // The whole estimator of pixel i (all frames of the call) where no shadow ray is
@@ -375,17 +408,16 @@ __global__ void __launch_bounds__(kSampleThreads, RISLTC_SAMPLE_MIN_BLOCKS) ris_
 #ifndef RISLTC_TRACE_REFILL
 #define RISLTC_TRACE_REFILL 12
 #endif
-// Persistent any-hit tracing of a queue of n rays (*cursor is the fetch cursor,
-// zero at launch).  Each lane holds one ray and advances it by one unit of
+// Persistent any-hit tracing of a queue of n rays.  Each lane holds one ray and advances it by one unit of
 // work (a triangle test or an inner node) per iteration; whenever
 // RISLTC_TRACE_REFILL or more lanes of a warp are idle they fetch the next
 // rays together, so lanes do not wait for the warp's longest ray.  Queue
-// supplies ray k (its origin, direction and interval) and takes its outcome.
+// has the fetch cursor (zero at launch), supplies ray k (its origin, direction and interval) and takes its outcome.
 // kShared false: no cursor, each warp takes 32 rays of every gridful of them.
 // (2M and 4M of a caller's rays 612 and 1,140 us, against 574 and 1,070 with
 // the cursor and 700 and 1,332 with a thread per ray.)
 template <class P, bool kShared, class Queue>
-RL_DEV void trace_queue(const SceneView& s, const Queue& queue, uint32_t n, uint32_t* cursor, uint32_t* error) {
+RL_DEV void trace_queue(const SceneView& s, const Queue& queue, uint32_t n, uint32_t* error) {
 	const uint32_t lane = threadIdx.x % 32;
 	const uint32_t stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x - lane;
 	uint32_t taken = 0;
@@ -400,7 +432,7 @@ RL_DEV void trace_queue(const SceneView& s, const Queue& queue, uint32_t n, uint
 			const int leader = __ffs(idle) - 1;
 			uint32_t base = 0;
 			if (kShared) {
-				if ((int) lane == leader) base = atomicAdd(cursor, (uint32_t) __popc(idle));
+				if ((int) lane == leader) base = atomicAdd(queue.cursor, (uint32_t) __popc(idle));
 				base = __shfl_sync(0xffffffffu, base, leader);
 				drained = base + (uint32_t) __popc(idle) >= n;
 			} else {
@@ -443,6 +475,7 @@ RL_DEV void trace_queue(const SceneView& s, const Queue& queue, uint32_t n, uint
 struct ShadowQueue {
 	const ShadowRay* rays;
 	uint8_t* hits;
+	uint32_t* cursor;
 	RL_DEV void ray(uint32_t k, f3& o, f3& d, float& t_min, float& t_max) const {
 		const float4 a = __ldg(&rays[k].origin), b = __ldg(&rays[k].dir_tmax);
 		o = mk3(a.x, a.y, a.z);
@@ -453,11 +486,131 @@ struct ShadowQueue {
 	RL_DEV void outcome(uint32_t k, bool hit) const { hits[k] = hit ? 1 : 0; }
 };
 template <class P>
-__global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) shadow_trace_kernel(SceneView s, const ShadowRay* rays,
-                                                           uint32_t count, uint32_t* cursor, uint8_t* hits, uint32_t* error) {
+__global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS)
+shadow_trace_kernel(SceneView s, const ShadowRay* rays, uint32_t count, uint32_t* cursor, uint8_t* hits, uint32_t* error) {
 	allow_next();
-	trace_queue<P, true>(s, ShadowQueue{rays, hits}, count, cursor, error);
+	trace_queue<P, true>(s, ShadowQueue{rays, hits, cursor}, count, error);
 }
+
+// The same loop over a source of rays that deals them out itself: deal(idle,
+// drained) is called by whole warps with the idle lanes' mask, true for a lane
+// that got a ray, drained when there are no more.  The source gives the lane's
+// ray and its scene and takes its outcome.
+template <class P, class Source> RL_DEV void trace_dealt(Source& source, uint32_t* error) {
+	int32_t stack[kTraceStack];
+	TraceRay r;
+	bool busy = false, drained = false;
+	for (;;) {
+		const uint32_t idle = __ballot_sync(0xffffffffu, !busy);
+		if (drained && idle == 0xffffffffu) break;
+		if (!drained && __popc(idle) >= RISLTC_TRACE_REFILL) {
+			if (source.deal(idle, drained)) {
+				f3 o, d;
+				float t_min, t_max;
+				source.ray(o, d, t_min, t_max);
+				const int st = trace_begin<P>(source.scene(), r, o, d, t_min, t_max, stack);
+				if (st == kTraceContinue)
+					busy = true;
+				else
+					source.outcome(st == kTraceHit);
+			}
+			continue;
+		}
+		if (busy) {
+			const int st = trace_step<P>(source.scene(), r, stack, error);
+			if (st != kTraceContinue) {
+				source.outcome(st == kTraceHit);
+				busy = false;
+			}
+		}
+	}
+}
+
+// Places of a queue that a warp has claimed and not dealt out yet, from claimed.x
+// to claimed.y (in shared memory, a slot per warp: two registers made the batch
+// kernel spill).  A claim takes what the idle lanes want or, while more remain,
+// a share of the remaining places, 2^-shift: a cursor answers one claim after
+// another, 0.7 ns each, and places without a ray are done faster than that.
+RL_DEV bool deal_places(uint32_t idle, bool& drained, uint2& claimed, uint32_t count, int shift, uint32_t& place, uint32_t* cursor) {
+	const uint32_t lane = threadIdx.x % 32, n = (uint32_t) __popc(idle);
+	const uint32_t rank = (uint32_t) __popc(idle & ((1u << lane) - 1u));
+	uint32_t next = claimed.x, end = claimed.y;
+	const uint32_t left = end - next;
+	uint32_t at = next + rank;
+	next += n;
+	if (left < n) {
+		const uint32_t size = max(n - left, (count - min(end, count)) >> shift);
+		uint32_t base = 0;
+		if (lane == 0) base = atomicAdd(cursor, size);
+		base = __shfl_sync(0xffffffffu, base, 0);
+		if (rank >= left) at = base + rank - left;
+		next = base + n - left;
+		end = base + size;
+	}
+	__syncwarp();
+	if (lane == 0) claimed = make_uint2(next, end);
+	__syncwarp();
+	drained = next >= count;
+	place = at;
+	return (idle >> lane & 1u) && at < count;
+}
+
+// The rays of a call with many places, claimed by shares.
+struct FrameRays {
+	const SceneView& s;
+	const ShadowRay* rays;
+	uint8_t* hits;
+	uint32_t* cursor;
+	uint32_t covered, pixels, frames;
+	int shift;
+	uint2& claimed;
+	uint32_t place;  // the lane's
+
+	RL_DEV bool deal(uint32_t idle, bool& drained) {
+		uint32_t g;
+		if (!deal_places(idle, drained, claimed, 2u * covered * frames, shift, g, cursor)) return false;
+		place = queue_place(g, covered, pixels);
+		return true;
+	}
+	RL_DEV const SceneView& scene() const { return s; }
+	RL_DEV void ray(f3& o, f3& d, float& t_min, float& t_max) const {
+		const float4 a = __ldg(&rays[place].origin), b = __ldg(&rays[place].dir_tmax);
+		o = mk3(a.x, a.y, a.z);
+		d = mk3(b.x, b.y, b.z);
+		t_min = 1.0e-3f;
+		t_max = b.w;
+	}
+	RL_DEV void outcome(bool hit) const { hits[place] = hit ? 1 : 0; }
+};
+template <class P>
+__global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS)
+shadow_trace_shares_kernel(SceneView s, const ShadowRay* rays, uint32_t pixels, uint32_t frames, int shift,
+                           LaunchCounters* counters, uint8_t* hits, uint32_t* error) {
+	__shared__ uint2 claimed[4];
+	claimed[threadIdx.x / 32] = make_uint2(0u, 0u);
+	__syncwarp();
+	allow_next();
+	FrameRays source{s, rays, hits, &counters->fetch, queue_covered(counters, pixels), pixels, frames, shift,
+	                 claimed[threadIdx.x / 32], 0u};
+	trace_dealt<P>(source, error);
+}
+// The shift: at least 15 (for the 7,296 warps of a full grid a claim is at most
+// two ninths of a warp's even share of what remains), and no claim of more than
+// 256 places, which warps that come to them last would be left alone with.
+inline int claim_shift(uint32_t count) {
+	int shift = 15;
+	while ((count >> shift) > 256u) ++shift;
+	return shift;
+}
+// Places per lane of a full grid from which queues with background are numbered
+// and claims made by shares.  Above: 4-frame 1080p calls with 16,384 lights take
+// 14.60 ms without background (14.61 with single claims and every pixel's places
+// kept), 1.48 with 95% of it above a horizon (2.15; 2.09 when the rays were
+// compacted and grouped by light, which all else paid for), 0.36 with nothing
+// else (0.78; 0.42); one frame with 1,024 lights 3.78, 0.53 and 0.18 ms (3.78,
+// 0.60, 0.26; 5.36, 0.64, 0.19).  Below, calls of 3 frames of 961x541 with any
+// background but all lose 1% or less to the empty places.
+constexpr uint32_t kSharesPerLane = 16;
 
 // Whether a 32-bit cursor can deal out `rays` to `threads` threads: after the
 // last ray each warp may add up to 32 once more, and a cursor that wrapped there
@@ -468,6 +621,7 @@ constexpr bool cursor_holds(uint32_t rays, uint32_t threads) { return rays <= 0x
 struct CallerQueue {
 	const float4* rays;
 	uint32_t* hits;
+	uint32_t* cursor;
 	RL_DEV void ray(uint32_t k, f3& o, f3& d, float& t_min, float& t_max) const {
 		const float4 a = rays[2 * (size_t) k], b = rays[2 * (size_t) k + 1];
 		o = mk3(a.x, a.y, a.z);
@@ -480,7 +634,7 @@ struct CallerQueue {
 template <class P, bool kShared>
 __global__ void __launch_bounds__(128, RISLTC_TRACE_MIN_BLOCKS) trace_shadow_queue_kernel(SceneView s, const float4* rays, uint32_t count,
                                                                  uint32_t* hits, uint32_t* cursor, uint32_t* error) {
-	trace_queue<P, kShared>(s, CallerQueue{rays, hits}, count, cursor, error);
+	trace_queue<P, kShared>(s, CallerQueue{rays, hits, cursor}, count, error);
 }
 
 // The resolve phase of pixel i (all frames of the call); i may be past the
@@ -499,6 +653,7 @@ template <class P> RL_DEV void resolve_pixel(const RisParams& pr, uint32_t i) {
 			}
 			return;
 		}
+		const bool numbered = has_numbers(pr);
 		f3 sum = splat(0.0f);
 		double acc[3] = {0.0, 0.0, 0.0};
 		for (uint32_t f = 0; f != pr.frame_count; ++f) {
@@ -515,7 +670,7 @@ template <class P> RL_DEV void resolve_pixel(const RisParams& pr, uint32_t i) {
 				for (int j = 0; j != 2; ++j) {
 					const uint32_t mode = (flags >> (2 * j)) & 3u;
 					if (mode == kSampleSkip) continue;
-					const bool occluded = mode == kSampleTraced && pr.hits[2 * pf + j] != 0;
+					const bool occluded = mode == kSampleTraced && pr.hits[2 * ((size_t) f * np + (numbered ? __float_as_uint(q3.z) : i)) + j] != 0;
 					result = add(result, occluded ? c[j][1] : c[j][0]);
 				}
 				const f3 color = scale(result, P::rcp(1.0f));

@@ -45,8 +45,13 @@ cudaError_t launch_shadow_trace(const RisParams& p, cudaStream_t stream, int gri
 	const uint32_t count = 2u * p.width * p.height * p.frame_count;
 	// Never early: its blocks would gather on the SMs that drain first (a 349x168
 	// frame took 157 instead of 144 us).
-	shadow_trace_kernel<ExactNumerics>
-	    <<<grid, 128, 0, stream>>>(p.scene, p.rays, count, &p.counters->fetch, p.hits, p.error);
+	if (p.compact)
+		shadow_trace_shares_kernel<ExactNumerics>
+		    <<<grid, 128, 0, stream>>>(p.scene, p.rays, p.width * p.height, p.frame_count, claim_shift(count), p.counters,
+		                               p.hits, p.error);
+	else
+		shadow_trace_kernel<ExactNumerics>
+		    <<<grid, 128, 0, stream>>>(p.scene, p.rays, count, &p.counters->fetch, p.hits, p.error);
 	return cudaGetLastError();
 }
 cudaError_t launch_ris_resolve(const RisParams& p, cudaStream_t stream, int grid) {
@@ -60,7 +65,10 @@ cudaError_t launch_batch_estimator(const RisBatch& b, cudaStream_t stream, int p
 	ris_sample_batch_kernel<ExactNumerics><<<pixel_grid, kSampleThreads, 0, stream>>>(b);
 	cudaError_t e = cudaGetLastError();
 	if (e != cudaSuccess) return e;
-	shadow_trace_batch_kernel<ExactNumerics><<<ray_grid, 128, 0, stream>>>(b);
+	if (b.item[0].compact)
+		shadow_trace_batch_shares_kernel<ExactNumerics><<<ray_grid, 128, 0, stream>>>(b, claim_shift(b.ray_begin[b.count]));
+	else
+		shadow_trace_batch_kernel<ExactNumerics><<<ray_grid, 128, 0, stream>>>(b);
 	if ((e = cudaGetLastError()) != cudaSuccess) return e;
 	ris_resolve_batch_kernel<ExactNumerics><<<pixel_grid, 128, 0, stream>>>(b);
 	return cudaGetLastError();
