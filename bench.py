@@ -490,7 +490,8 @@ def kernel_table(prof, samples_per_step, info, fp32_peak, peaks):
     CPU leg, achieved FP32 work against the FP32 peak; the traversal's
     node and triangle bytes (served from L1/L2) against its time."""
     calls = max(prof["calls"], 1)
-    # One launch of each kernel per step (all spp frames in one call).
+    # One launch of each kernel per step (all spp frames in one call); the trace
+    # is shadow_trace_shares_kernel's in large calls.
     kernels = {"ris_candidates_binned_kernel": {"ms_per_launch": prof["candidates"] / calls},
                "ris_sample_kernel": {"ms_per_launch": prof["shade"] / calls},
                "shadow_trace_kernel": {"ms_per_launch": prof["shadow_trace"] / calls},

@@ -10,8 +10,8 @@
 //
 // Weights are BF16 for inference (each layer stored [out][in]), biases FP32.
 // The forward pass runs on the tcgen05 tensor cores (mlp_tc.cuh); online
-// training runs there too for up to 256 clusters (mlp_train_tc.cuh), and in
-// FP32 on the CUDA cores (below) for larger models or on request.
+// training runs there too (mlp_train_tc.cuh up to 256 clusters,
+// mlp_train_tc_wide.cuh above), and in FP32 on the CUDA cores (below) on request.
 #pragma once
 #include <cuda_bf16.h>
 #include "proposal.cuh"
